@@ -117,6 +117,9 @@ def c_solve_structs(mats, Ct, rho_t, h, dt, coeffs, src_idx, src_w, rec_off, rec
         if on_device:
             # indices below 2^14 (the flag bits are set by the solver): int16 holds them
             lab_t = mats.to(device=dev, dtype=torch.int16).contiguous()
+            # the solver copies the labels on a stream of its own: whatever
+            # still writes them on the caller's stream must be finished
+            torch.cuda.current_stream(dev).synchronize()
         else:
             lab_t = torch.from_numpy(np.ascontiguousarray(mats.astype(np.uint16).view(np.int16))).to(dev)
         dvol_t = (torch.from_numpy(np.ascontiguousarray(damp_volume, np.float32)).to(dev)
