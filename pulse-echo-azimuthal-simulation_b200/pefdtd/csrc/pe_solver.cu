@@ -373,21 +373,33 @@ bool same_state(const PeState &a, const PeState &b)
     return true;
 }
 
-// Planes per z-march: the split of nz into chunks that minimises
-// waves x (planes per chunk + per-chunk start-up planes), where a wave is
-// one block on every SM slot the occupancy allows.
+// Planes per z-march: the split of nz into chunks that minimises the modelled
+// time of a launch, in planes marched at the full-SM rate: (planes per chunk +
+// start-up planes) x waves, a wave being one block on every slot. Kernels with
+// one block per SM run their waves in step, so waves count whole. With two per
+// SM, a launch that leaves every SM at most one block runs its planes in 0.7
+// of the time (measured 1.75 us a plane alone and 2.65 with two blocks per SM
+// for the stress kernel, 1.55 and 1.95 for the velocity kernel); one that fits
+// one wave waits for its slowest, guarded, blocks (1.15); beyond that the
+// blocks drift apart and the tail costs about half a wave, not a whole one.
+// Against whole waves throughout (which preferred one full wave): velocity
+// kernel on 96x160x160 56 -> 51 us (20 -> 8 planes), on 20x24x28 14.5 -> 12.5
+// us (4 -> 2 planes). A shorter march must be worth 2 %: longer ones re-read
+// less of the z halo.
 int pick_zchunk(int nz, long long tiles, int slots, int startup)
 {
+    int nsm = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     int best_zc = nz;
     double best = 1e300;
     for (int nch = 1; nch <= nz; ++nch) {
         const int zc = (nz + nch - 1) / nch;
-        const int real = (nz + zc - 1) / zc;
-        if (zc < 4 && nch > 1) break;
-        const long long blocks = tiles * real;
-        const long long waves = (blocks + slots - 1) / slots;
-        const double cost = (double)waves * (zc + startup);
-        if (cost < best - 1e-9) {
+        const long long blocks = tiles * ((nz + zc - 1) / zc);
+        double waves = (double)((blocks + slots - 1) / slots);
+        if (slots > nsm) waves = blocks <= nsm ? 0.7 : (blocks <= slots ? 1.15 : (double)blocks / slots + 0.5);
+        const double cost = waves * (zc + startup);
+        if (cost < 0.98 * best) {
             best = cost;
             best_zc = zc;
         }
@@ -499,7 +511,7 @@ int configure_kernels(PeSolver *S)
             const int sps = occupancy_slots(pe::k_stress_pair<4, true>, pe::PS_N, ps);
             const int spv = occupancy_slots(pe::k_velocity_pair<4>, pe::PV_N, pv);
             S->zc_ps = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tps, sps, 3);
-            S->zc_pv = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tpv, spv, 2);
+            S->zc_pv = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tpv, spv, 1);
         }
     }
     return PE_OK;
