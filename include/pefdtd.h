@@ -72,9 +72,12 @@ typedef struct PeConfig {
 } PeConfig;
 
 /* Kernel family; all are bit-identical. TILED picks the fastest tiled kernels
- * the grid allows: in FP32 on grids whose rows are 16-byte multiples the
- * pair-column kernels (each thread updates two x-adjacent cells), else the
- * one-column tiled kernels. COLUMN forces the one-column tiled kernels and
+ * the grid allows: in FP32 the pair-column kernels (each thread updates two
+ * x-adjacent cells), on grids whose rows are not 16-byte multiples through
+ * solver-owned row-padded copies of the state, made at the start and copied
+ * back at the end of every run of 8 and more steps (38 B per padded cell of
+ * device memory, 42 with a damping volume); else the one-column tiled
+ * kernels. COLUMN forces the one-column tiled kernels and
  * SIMPLE the untiled ones (every tap read through the L1 cache); both are
  * kept as independent cross-checks of TILED. */
 enum PeKernelVariant { PE_KERNEL_TILED = 0, PE_KERNEL_SIMPLE = 1, PE_KERNEL_COLUMN = 2, PE_KERNEL_DENSE = 3 };
@@ -154,7 +157,8 @@ int pe_solver_run(PeSolver *s, const PeState *state, void *traces_dev, int64_t s
  * which case the traces of the affected run are invalid. Clears the status. */
 int pe_solver_status(PeSolver *s);
 
-/* Kernel launches issued by the last pe_solver_run (diagnostics). */
+/* Kernel launches issued by the last pe_solver_run (diagnostics; the copies
+ * into and out of row-padded fields are not counted). */
 int64_t pe_solver_launch_count(const PeSolver *s);
 
 /* Diagnostics for roofline reporting: advance `state` by n_steps from step 0
@@ -233,7 +237,8 @@ int pe_solver_adjoint_segment(PeSolver *s, const PeState *state, const PeAdjoint
  * and traces); all share one dtype and the tiled kernels. Each step is one
  * stress and one velocity launch covering every solve with nx a multiple of
  * 4 (state buffers 16-byte aligned), plus one launch pair per solve whose
- * rows are not whole 16-byte units (the cp.async kernels); when the batched
+ * rows are not whole 16-byte units (in persistent mode, in runs of 8 and
+ * more steps, those share the launch too); when the batched
  * kernels' shared memory cannot hold the largest table (FP64), every solve
  * runs its own pair. Chunks of steps replay as CUDA graphs. */
 typedef struct PeBatch PeBatch;

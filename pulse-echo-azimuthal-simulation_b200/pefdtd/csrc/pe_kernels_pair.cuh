@@ -1,5 +1,6 @@
-// Pair-column FP32 step kernels (the default FP32 path on grids whose rows
-// are 16-byte multiples).
+// Pair-column FP32 step kernels (the default FP32 path: on grids whose rows
+// are 16-byte multiples in place, on others in a row-padded copy of the state,
+// see k_repitch).
 //
 // Arithmetic, term order and explicit FMA placement are those of the
 // one-column kernels (pe_kernels_tma.cuh, pe_kernels.cuh), so the results are
@@ -435,7 +436,9 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
     const long long sy = A.sy, sz = A.sz;
     const int S0 = bx * PS_OX - 2, S0y = by * PS_OY - 1;   // first strain column / row (S0 even)
     const int gx0 = S0 + 2 * l, gy = S0y + r;
-    const bool pair_ok = TIN || (gx0 >= 0 && gx0 < nx && gy >= 0 && gy < ny);   // nx even: both columns
+    // odd nx (padded rows): the pair at nx - 1 holds a pad column, whose
+    // fields stay zero and which is never updated
+    const bool pair_ok = TIN || (gx0 >= 0 && gx0 < nx && gy >= 0 && gy < ny);
     const int col = pair_ok ? (int)(gy * sy + gx0) : 0;
     const long long n = *A.step + A.k;
     const float wn = A.n_src ? A.wavelet[n] : 0.f;
@@ -792,6 +795,29 @@ __device__ __forceinline__ float div_face_rcp(float a, float b, bool own, float 
     return (float)((double)a / (double)b);
 }
 
+// Rows of spitch elements to rows of dpitch, nx of each, for up to nine
+// fields at once. A state whose rows are not 16-byte multiples cannot be read
+// by TMA boxes or 64-bit pairs; a run of several steps therefore copies it
+// once into solver-owned fields whose rows are padded to four cells, steps
+// those with the pair kernels, and copies it back. Each copy moves 72 B per
+// cell, about one step's traffic. 100 steps of 136x338x338: 120.8 ms with the
+// cp.async kernels, 73.8 ms padded, both copies included.
+struct FieldSet {
+    float *f[9];
+};
+__global__ void __launch_bounds__(256) k_repitch(const FieldSet src, const FieldSet dst, int nx, long long spitch,
+                                                 long long dpitch, long long rows)
+{
+    const float *s = src.f[blockIdx.y];
+    float *d = dst.f[blockIdx.y];
+    for (long long r = (long long)blockIdx.x * 8 + threadIdx.y; r < rows; r += (long long)gridDim.x * 8) {
+        const float *sr = s + r * spitch;
+        float *dr = d + r * dpitch;
+#pragma unroll 4
+        for (int x = threadIdx.x; x < nx; x += 32) dr[x] = sr[x];
+    }
+}
+
 // reciprocal densities RN32(1 / rho), correctly rounded (IEEE division)
 __global__ void k_rho_inv(const float *rho, float *rinv, int n_mat)
 {
@@ -872,7 +898,8 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
     const long long sy = A.sy, sz = A.sz;
     const int x0 = bx * PV_OX, y0 = by * PV_OY;
     const int ix = x0 + 2 * l, iy = y0 + r;
-    const bool out_ok = TIN || (ix < nx && iy < ny);   // nx even: both cells
+    const bool out_ok = TIN || (ix < nx && iy < ny);
+    const bool two = TIN || ix + 1 < nx;   // odd nx (padded rows): the last pair's cell 1 is a pad
     const int col = out_ok ? (int)(iy * sy + ix) : 0;
     const bool has_dvol = A.dvol != nullptr;
     const unsigned bytes = (5u * PV_TSZ + 3u * PV_CSZ + (has_dvol ? (unsigned)PV_CSZ : 0u)) * 4u;
@@ -914,7 +941,7 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
         tl.yb = lim_b(iy, ny);
         tl.yf = lim_f(iy, ny);
     }
-    const bool xin1 = TIN || ix + 1 < nx - 1;   // cell 1 has a +x neighbour (cell 0 always does)
+    const bool xin1 = TIN || ix + 1 < nx - 1;   // cell 1 has a +x neighbour (cell 0 does if cell 1 exists)
     const bool yin = TIN || iy < ny - 1;
     float dyx = 1.0f, dxx[2] = {1.0f, 1.0f};
     if (A.dz && out_ok) {
@@ -988,13 +1015,13 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
             float r0[2], rn[2][3];
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                const bool xin = c == 0 ? true : xin1;
+                const bool xin = c == 0 ? two : xin1;
                 r0[c] = rho_tab[lc[c] & LAB_MAT];
                 rn[c][0] = xin ? rho_tab[lxv[c] & LAB_MAT] : 0.f;
                 rn[c][1] = yin ? rho_tab[lyv[c] & LAB_MAT] : 0.f;
                 rn[c][2] = (z < nz - 1) ? rho_tab[lzv[c] & LAB_MAT] : 0.f;
             }
-            const bool has_nb[2][3] = {{true, yin, z < nz - 1}, {xin1, yin, z < nz - 1}};
+            const bool has_nb[2][3] = {{two, yin, z < nz - 1}, {xin1, yin, z < nz - 1}};
             const float2 r02 = make_float2(r0[0], r0[1]);
             const float2 y2 = make_float2(__ldg(A.rinv + (lc[0] & LAB_MAT)), __ldg(A.rinv + (lc[1] & LAB_MAT)));
             const float2 a2[3] = {ax, ay, az};
@@ -1033,9 +1060,13 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
                 vn[d][1] = v.y;
             }
             const long long idx = (long long)z * sz + col;
-            stg2(A.v[0] + idx, vn[0][0], vn[0][1]);
-            stg2(A.v[1] + idx, vn[1][0], vn[1][1]);
-            stg2(A.v[2] + idx, vn[2][0], vn[2][1]);
+            if (two) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) stg2(A.v[d] + idx, vn[d][0], vn[d][1]);
+            } else {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) A.v[d][idx] = vn[d][0];
+            }
             if (A.rec_kind != 0) {
 #pragma unroll
                 for (int c = 0; c < 2; ++c)
@@ -1091,7 +1122,7 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
 // within a solve, so blocks that run together march the same planes of
 // neighbouring tiles; each resident block walks a contiguous run of items,
 // re-staging the solve's arguments and tables only when the solve changes.
-// All solves of a pair batch have rows of 16-byte multiples.
+// All solves of a pair batch have rows of 16-byte multiples, their own or padded.
 template <int NC, bool TS>
 __global__ void __launch_bounds__(PS_N, 2)
     k_stress_pair_batch(const StepArgs<float> *__restrict__ descs, const TmapsPairStress *__restrict__ maps,

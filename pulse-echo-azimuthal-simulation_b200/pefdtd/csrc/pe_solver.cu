@@ -190,6 +190,15 @@ struct PeSolver {
     int nrep = 0;
     bool pair_capable = false;  // FP32, rows of 16-byte multiples, maps encodable, smem fits
     bool pair = false;          // pair kernels in use for the current state
+    // FP32 grids whose rows are not 16-byte multiples: runs of PAD_MIN_STEPS
+    // steps or more go through row-padded fields and the pair kernels
+    bool padded = false;
+    int px = 0;                 // padded row length
+    void *pfields = nullptr;    // nine padded fields
+    PeState pst{};
+    uint16_t *lab_p = nullptr;
+    float *dvol_p = nullptr;
+    long long *src_idx_p = nullptr, *rec_cell_p = nullptr;   // probe cells in the padded layout
     bool solo = false;          // in a batch: fills the GPU alone, so runs its own launches
     int zc_ps = 0, zc_pv = 0;   // planes per z-march of the pair launches
     pe::TmapsPairStress mps{};
@@ -202,7 +211,8 @@ struct PeSolver {
         if (ev_out) cudaEventDestroy(ev_out);
         if (stream) cudaStreamDestroy(stream);
         void *bufs[] = {lab, c21, rho, dz, dy, dx, dvol, src_idx, src_w, rec_cell,
-                        rec_pos, rec_w, grp_off, rec_val, wavelet, step, status, ent_group, tab36, rinv, grad_rep};
+                        rec_pos, rec_w, grp_off, rec_val, wavelet, step, status, ent_group, tab36, rinv, grad_rep,
+                        pfields, lab_p, dvol_p, src_idx_p, rec_cell_p};
         for (void *b : bufs)
             if (b) dev_free(b);
     }
@@ -210,35 +220,39 @@ struct PeSolver {
 
 namespace {
 
+// whether st is the solver's own row-padded state
+bool is_padded_state(const PeSolver *S, const PeState *st) { return S->padded && st->v[0] == S->pst.v[0]; }
+
 template <typename T>
 pe::StepArgs<T> make_args(const PeSolver *S, const PeState *st, int k)
 {
+    const bool pad = is_padded_state(S, st);
     pe::StepArgs<T> A{};
     for (int i = 0; i < 3; ++i) A.v[i] = (T *)st->v[i];
     for (int i = 0; i < 6; ++i) A.s[i] = (T *)st->s[i];
-    A.lab = S->lab;
+    A.lab = pad ? S->lab_p : S->lab;
     A.c21 = (const T *)S->c21;
     A.rho = (const T *)S->rho;
     A.rinv = S->rinv;
     A.dz = S->dz;
     A.dy = S->dy;
     A.dx = S->dx;
-    A.dvol = S->dvol;
+    A.dvol = pad ? S->dvol_p : S->dvol;
     A.nz = S->cfg.nz;
     A.ny = S->cfg.ny;
     A.nx = S->cfg.nx;
-    A.sy = S->cfg.nx;
-    A.sz = (long long)S->cfg.nx * S->cfg.ny;
+    A.sy = pad ? S->px : S->cfg.nx;
+    A.sz = A.sy * S->cfg.ny;
     for (int j = 0; j < 4; ++j) A.c[j] = j < S->cfg.n_coeffs ? (T)S->cfg.coeffs[j] : T(0);
     A.nc = S->cfg.n_coeffs;
     A.inv_h = (T)(1.0 / S->cfg.h);
     A.dt = (T)S->cfg.dt;
     A.dt_h = (T)(S->cfg.dt / S->cfg.h);
-    A.src_idx = S->src_idx;
+    A.src_idx = pad ? S->src_idx_p : S->src_idx;
     A.src_w = (const T *)S->src_w;
     A.n_src = S->n_src;
     A.wavelet = (const T *)S->wavelet;
-    A.rec_cell = S->rec_cell;
+    A.rec_cell = pad ? S->rec_cell_p : S->rec_cell;
     A.rec_pos = S->rec_pos;
     A.n_rec = S->n_rec;
     A.rec_val = (T *)S->rec_val;
@@ -439,13 +453,14 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
-// 3-D map (x fastest) of one (nz, ny, nx) field with a (bw, bh, 1) box;
-// out-of-grid box elements read as zero
+// 3-D map (x fastest) of one (nz, ny, nx) field, rows `pitch` elements apart
+// (0 = nx), with a (bw, bh, 1) box; out-of-grid box elements read as zero
 int encode_box(CUtensorMap *m, const void *base, CUtensorMapDataType dt, int es, const PeConfig &c,
-               int bw, int bh)
+               int bw, int bh, int pitch = 0)
 {
+    const cuuint64_t row = (cuuint64_t)(pitch ? pitch : c.nx) * es;
     const cuuint64_t dims[3] = {(cuuint64_t)c.nx, (cuuint64_t)c.ny, (cuuint64_t)c.nz};
-    const cuuint64_t strides[2] = {(cuuint64_t)c.nx * es, (cuuint64_t)c.nx * c.ny * es};
+    const cuuint64_t strides[2] = {row, row * c.ny};
     const cuuint32_t box[3] = {(cuuint32_t)bw, (cuuint32_t)bh, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = encode_fn()(m, dt, 3, const_cast<void *>(base), dims, strides, box, estr,
@@ -495,9 +510,12 @@ int configure_kernels(PeSolver *S)
     S->zc_v = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tv, sv, 3);
     if constexpr (std::is_same<T, float>::value) {
         const size_t ps = pe::stress_pair_smem(c.n_mat), pv = pe::velocity_pair_smem(c.n_mat);
-        S->pair_capable = S->variant == PE_KERNEL_TILED && c.nx % 4 == 0 && ps <= (size_t)optin &&
-                          pv <= (size_t)optin && encode_fn() != nullptr;
-        if (S->pair_capable) {
+        const bool pair_ok = S->variant == PE_KERNEL_TILED && ps <= (size_t)optin && pv <= (size_t)optin &&
+                             encode_fn() != nullptr;
+        S->pair_capable = pair_ok && c.nx % 4 == 0;
+        S->padded = pair_ok && c.nx % 4 != 0;
+        S->px = (c.nx + 3) / 4 * 4;
+        if (pair_ok) {
             // the attribute belongs to the kernel, not to this solve: allow the
             // device maximum so that solves with other table sizes can coexist
             PE_CUDA(cudaFuncSetAttribute(pe::k_stress_pair<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
@@ -522,37 +540,41 @@ int configure_kernels(PeSolver *S)
 // to the cp.async kernels when a buffer is not 16-byte aligned.
 int ensure_maps(PeSolver *S, const PeState *st)
 {
-    if (!S->tma_capable && !S->pair_capable) {
+    const bool pad = is_padded_state(S, st);
+    const float *const dvol = pad ? S->dvol_p : S->dvol;
+    const int pitch = pad ? S->px : 0;
+    if (!S->tma_capable && !S->pair_capable && !pad) {
         S->tma = false;
         S->pair = false;
+        S->maps_ok = false;   // a later padded run sets them again
         return PE_OK;
     }
     if (S->maps_ok && same_state(S->mstate, *st)) return PE_OK;
     const PeConfig &c = S->cfg;
     const int es = S->esize;
-    bool aligned = !S->dvol || ((uintptr_t)S->dvol % 16) == 0;
+    bool aligned = !dvol || ((uintptr_t)dvol % 16) == 0;
     for (int i = 0; i < 3; ++i) aligned = aligned && ((uintptr_t)st->v[i] % 16) == 0;
     for (int i = 0; i < 6; ++i) aligned = aligned && ((uintptr_t)st->s[i] % 16) == 0;
     S->mstate = *st;
     S->maps_ok = true;
     S->tma = aligned && S->tma_capable;
-    S->pair = aligned && S->pair_capable;
+    S->pair = aligned && (S->pair_capable || pad);
     if (!aligned) return PE_OK;
     const CUtensorMapDataType dt = es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     int rc;
     if (S->pair) {
         for (int f = 0; f < 3; ++f)
-            if ((rc = encode_box(&S->mps.vt[f], st->v[f], dt, es, c, pe::PS_VW, pe::PS_VH))) return rc;
+            if ((rc = encode_box(&S->mps.vt[f], st->v[f], dt, es, c, pe::PS_VW, pe::PS_VH, pitch))) return rc;
         for (int f = 0; f < 6; ++f)
-            if ((rc = encode_box(&S->mps.sc[f], st->s[f], dt, es, c, pe::PS_SW, pe::PS_SH))) return rc;
+            if ((rc = encode_box(&S->mps.sc[f], st->s[f], dt, es, c, pe::PS_SW, pe::PS_SH, pitch))) return rc;
         const int pvf[5] = {0, 1, 3, 4, 5};
         for (int f = 0; f < 5; ++f)
-            if ((rc = encode_box(&S->mpv.st[f], st->s[pvf[f]], dt, es, c, pe::PV_TW, pe::PV_TH))) return rc;
+            if ((rc = encode_box(&S->mpv.st[f], st->s[pvf[f]], dt, es, c, pe::PV_TW, pe::PV_TH, pitch))) return rc;
         for (int f = 0; f < 3; ++f)
-            if ((rc = encode_box(&S->mpv.vc[f], st->v[f], dt, es, c, pe::PV_OX, pe::PV_OY))) return rc;
-        if (S->dvol) {
-            if ((rc = encode_box(&S->mps.dv, S->dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::PS_SW, pe::PS_SH))) return rc;
-            if ((rc = encode_box(&S->mpv.dv, S->dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::PV_OX, pe::PV_OY))) return rc;
+            if ((rc = encode_box(&S->mpv.vc[f], st->v[f], dt, es, c, pe::PV_OX, pe::PV_OY, pitch))) return rc;
+        if (dvol) {
+            if ((rc = encode_box(&S->mps.dv, dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::PS_SW, pe::PS_SH, pitch))) return rc;
+            if ((rc = encode_box(&S->mpv.dv, dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::PV_OX, pe::PV_OY, pitch))) return rc;
         } else {
             std::memset(&S->mps.dv, 0, sizeof(S->mps.dv));
             std::memset(&S->mpv.dv, 0, sizeof(S->mpv.dv));
@@ -577,6 +599,30 @@ int ensure_maps(PeSolver *S, const PeState *st)
     }
     return PE_OK;
 }
+
+// Runs shorter than this step the caller's state in place: the copies into and
+// out of the padded layout cost about two pair steps and save about 0.4 of a
+// step of the unpadded kernels each.
+constexpr int PAD_MIN_STEPS = 8;
+
+// the first nf fields (v then s) of `from` into `to`; pitches 0 = the caller's
+// unpadded rows
+int repitch(const PeSolver *S, const PeState *from, int spitch, const PeState *to, int dpitch, int nf, cudaStream_t st)
+{
+    pe::FieldSet a{}, b{};
+    for (int i = 0; i < 9; ++i) {
+        a.f[i] = (float *)(i < 3 ? from->v[i] : from->s[i - 3]);
+        b.f[i] = (float *)(i < 3 ? to->v[i] : to->s[i - 3]);
+    }
+    const PeConfig &c = S->cfg;
+    const long long rows = (long long)c.ny * c.nz;
+    const dim3 grid((unsigned)std::min<long long>((rows + 7) / 8, 1 << 16), (unsigned)nf, 1);
+    pe::k_repitch<<<grid, dim3(32, 8, 1), 0, st>>>(a, b, c.nx, spitch ? spitch : c.nx, dpitch ? dpitch : c.nx, rows);
+    PE_CUDA(cudaGetLastError());
+    return PE_OK;
+}
+int pad_in(const PeSolver *S, const PeState *state, cudaStream_t st) { return repitch(S, state, 0, &S->pst, S->px, 9, st); }
+int pad_out(const PeSolver *S, const PeState *state, cudaStream_t st) { return repitch(S, &S->pst, S->px, state, 0, 9, st); }
 
 }  // namespace
 
@@ -740,7 +786,7 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
     if (all_sp) {
         if ((rc = dev_alloc(&S->dz, sizeof(float) * c.nz))) return rc;
         if ((rc = dev_alloc(&S->dy, sizeof(float) * c.ny))) return rc;
-        if ((rc = dev_alloc(&S->dx, sizeof(float) * c.nx))) return rc;
+        if ((rc = dev_alloc(&S->dx, sizeof(float) * (c.nx + 1)))) return rc;   // a pair's cell 1 may be a pad
         PE_CUDA(cudaMemcpyAsync(S->dz, md->sponge_z, sizeof(float) * c.nz, cudaMemcpyHostToDevice, st));
         PE_CUDA(cudaMemcpyAsync(S->dy, md->sponge_y, sizeof(float) * c.ny, cudaMemcpyHostToDevice, st));
         PE_CUDA(cudaMemcpyAsync(S->dx, md->sponge_x, sizeof(float) * c.nx, cudaMemcpyHostToDevice, st));
@@ -752,6 +798,47 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
     // probe
     if ((rc = dev_alloc(&S->src_idx, sizeof(long long) * std::max<size_t>(1, sidx.size())))) return rc;
     if ((rc = dev_alloc(&S->src_w, (size_t)es * std::max<size_t>(1, sidx.size())))) return rc;
+    // padded layout: a label volume, damping volume and probe cells of its own
+    // (the adjoint and short runs use the caller's layout). Without the memory
+    // for it the solve keeps the kernels that need no padding.
+    std::vector<long long> sidx_p, rcell_p;
+    if (S->padded) {
+        const size_t ncp = (size_t)S->px * c.ny * c.nz;
+        rc = dev_alloc(&S->pfields, 9 * sizeof(float) * ncp);
+        if (!rc) rc = dev_alloc(&S->lab_p, sizeof(uint16_t) * ncp);
+        if (!rc && S->dvol) rc = dev_alloc(&S->dvol_p, sizeof(float) * ncp);
+        if (!rc) rc = dev_alloc(&S->src_idx_p, sizeof(long long) * std::max<size_t>(1, sidx.size()));
+        if (!rc) rc = dev_alloc(&S->rec_cell_p, sizeof(long long) * (size_t)std::max<long long>(1, n_rec));
+        if (rc) {
+            cudaGetLastError();
+            dev_free(S->pfields);
+            dev_free(S->lab_p);
+            dev_free(S->dvol_p);
+            S->pfields = nullptr;
+            S->lab_p = nullptr;
+            S->dvol_p = nullptr;
+            S->padded = false;
+        }
+    }
+    if (S->padded) {
+        const size_t ncp = (size_t)S->px * c.ny * c.nz;
+        PE_CUDA(cudaMemsetAsync(S->pfields, 0, 9 * sizeof(float) * ncp, st));
+        PE_CUDA(cudaMemsetAsync(S->lab_p, 0, sizeof(uint16_t) * ncp, st));
+        if (S->dvol_p) {
+            PE_CUDA(cudaMemsetAsync(S->dvol_p, 0, sizeof(float) * ncp, st));
+            PE_CUDA(cudaMemcpy2DAsync(S->dvol_p, sizeof(float) * S->px, S->dvol, sizeof(float) * c.nx,
+                                      sizeof(float) * c.nx, (size_t)c.ny * c.nz, cudaMemcpyDeviceToDevice, st));
+        }
+        for (int i = 0; i < 3; ++i) S->pst.v[i] = (float *)S->pfields + i * ncp;
+        for (int i = 0; i < 6; ++i) S->pst.s[i] = (float *)S->pfields + (3 + i) * ncp;
+        auto to_padded = [&](long long q) { return q / c.nx * S->px + q % c.nx; };
+        for (long long q : sidx) sidx_p.push_back(to_padded(q));
+        for (long long q : rcell_sorted) rcell_p.push_back(to_padded(q));
+        if (!sidx_p.empty())
+            PE_CUDA(cudaMemcpyAsync(S->src_idx_p, sidx_p.data(), sizeof(long long) * sidx_p.size(), cudaMemcpyHostToDevice, st));
+        if (!rcell_p.empty())
+            PE_CUDA(cudaMemcpyAsync(S->rec_cell_p, rcell_p.data(), sizeof(long long) * rcell_p.size(), cudaMemcpyHostToDevice, st));
+    }
     if (!sidx.empty()) {
         PE_CUDA(cudaMemcpyAsync(S->src_idx, sidx.data(), sizeof(long long) * sidx.size(), cudaMemcpyHostToDevice, st));
         PE_CUDA(cudaMemcpyAsync(S->src_w, swb.data(), swb.size(), cudaMemcpyHostToDevice, st));
@@ -770,6 +857,9 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
         PE_CUDA(cudaMemcpyAsync(S->rec_w, pr->rec_w, (size_t)es * n_rec, cudaMemcpyHostToDevice, st));
         pe::k_labels_flag<<<(unsigned)((n_rec + 127) / 128), 128, 0, st>>>(S->lab, S->rec_cell, (int)n_rec, pe::LAB_REC);
     }
+    if (S->padded)   // the flagged labels
+        PE_CUDA(cudaMemcpy2DAsync(S->lab_p, sizeof(uint16_t) * S->px, S->lab, sizeof(uint16_t) * c.nx,
+                                  sizeof(uint16_t) * c.nx, (size_t)c.ny * c.nz, cudaMemcpyDeviceToDevice, st));
     if (S->n_groups > 0)
         PE_CUDA(cudaMemcpyAsync(S->grp_off, roff.data(), sizeof(long long) * (S->n_groups + 1), cudaMemcpyHostToDevice, st));
     {
@@ -815,21 +905,22 @@ int pe_solver_run(PeSolver *S, const PeState *state, void *traces, int64_t b, in
     for (int i = 0; i < 6; ++i)
         if (!state->s[i]) return fail(PE_ERR_INVALID, "state field missing");
     S->launches = 0;
-    {
-        const int rc0 = ensure_maps(S, state);
-        if (rc0) return rc0;
-    }
+    const bool pad = S->padded && e - b >= PAD_MIN_STEPS;
+    const PeState *use = pad ? &S->pst : state;
+    int rc = ensure_maps(S, use);
+    if (rc) return rc;
     if (e == b) return PE_OK;
     cudaStream_t user = (cudaStream_t)stream;
     PE_CUDA(cudaEventRecord(S->ev_in, user));
     PE_CUDA(cudaStreamWaitEvent(S->stream, S->ev_in, 0));
     pe::k_step_set<<<1, 1, 0, S->stream>>>(S->step, b);
     S->launches += 1;
+    if (pad && (rc = pad_in(S, state, S->stream))) return rc;
     int64_t n = b;
     while (n < e) {
         const int len = (int)std::min<int64_t>(S->chunk, e - n);
         if (len == S->chunk) {
-            if (!S->gexec || !same_state(S->gstate, *state) || S->gtraces != traces) {
+            if (!S->gexec || !same_state(S->gstate, *use) || S->gtraces != traces) {
                 if (S->gexec) {
                     cudaGraphExecDestroy(S->gexec);
                     S->gexec = nullptr;
@@ -837,7 +928,7 @@ int pe_solver_run(PeSolver *S, const PeState *state, void *traces, int64_t b, in
                 cudaGraph_t g = nullptr;
                 PE_CUDA(cudaStreamBeginCapture(S->stream, cudaStreamCaptureModeThreadLocal));
                 const long long before = S->launches;
-                int rc = launch_chunk(S, state, traces, len);
+                rc = launch_chunk(S, use, traces, len);
                 cudaError_t ce = cudaStreamEndCapture(S->stream, &g);
                 if (rc) return rc;
                 if (ce != cudaSuccess) return fail(PE_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
@@ -845,17 +936,18 @@ int pe_solver_run(PeSolver *S, const PeState *state, void *traces, int64_t b, in
                 ce = cudaGraphInstantiate(&S->gexec, g, 0);
                 cudaGraphDestroy(g);
                 if (ce != cudaSuccess) return fail(PE_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
-                S->gstate = *state;
+                S->gstate = *use;
                 S->gtraces = traces;
             }
             PE_CUDA(cudaGraphLaunch(S->gexec, S->stream));
             S->launches += 2LL * len + (S->n_groups > 0 ? 1 : 0) + 1;
         } else {
-            int rc = launch_chunk(S, state, traces, len);
+            rc = launch_chunk(S, use, traces, len);
             if (rc) return rc;
         }
         n += len;
     }
+    if (pad && (rc = pad_out(S, state, S->stream))) return rc;
     PE_CUDA(cudaEventRecord(S->ev_out, S->stream));
     PE_CUDA(cudaStreamWaitEvent(user, S->ev_out, 0));
     PE_CUDA(cudaGetLastError());
@@ -961,27 +1053,37 @@ int pe_solver_adjoint_segment(PeSolver *S, const PeState *state, const PeAdjoint
         if (!adj0->ls[i] || !state->s[i]) return fail(PE_ERR_INVALID, "adjoint stress buffers missing");
     if (a < 0 || b <= a) return fail(PE_ERR_INVALID, "need 0 <= step_begin < step_end");
     if (S->n_src > 0 && b > S->nt_wav) return fail(PE_ERR_INVALID, "step_end beyond the wavelet");
-    int rc = ensure_maps(S, state);
+    const bool pad = S->padded && b - a >= PAD_MIN_STEPS;
+    const PeState *use = pad ? &S->pst : state;
+    int rc = ensure_maps(S, use);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    if (pad && (rc = pad_in(S, state, st))) return rc;
     const size_t fb = (size_t)S->esize * (size_t)S->ncell;   // bytes of one field
     char *hist = (char *)v_hist;
     // recompute the segment, keeping v before every step
     for (int64_t n = a; n < b; ++n) {
-        for (int c = 0; c < 3; ++c)
-            PE_CUDA(cudaMemcpyAsync(hist + ((size_t)(n - a) * 3 + c) * fb, state->v[c], fb,
-                                    cudaMemcpyDeviceToDevice, st));
+        if (pad) {
+            PeState h{};
+            for (int c = 0; c < 3; ++c) h.v[c] = hist + ((size_t)(n - a) * 3 + c) * fb;
+            if ((rc = repitch(S, use, S->px, &h, 0, 3, st))) return rc;
+        } else {
+            for (int c = 0; c < 3; ++c)
+                PE_CUDA(cudaMemcpyAsync(hist + ((size_t)(n - a) * 3 + c) * fb, state->v[c], fb,
+                                        cudaMemcpyDeviceToDevice, st));
+        }
         pe::k_step_set<<<1, 1, 0, st>>>(S->step, n);
         if (S->cfg.dtype == PE_F64) {
-            pe::StepArgs<double> A = make_args<double>(S, state, 0);
+            pe::StepArgs<double> A = make_args<double>(S, use, 0);
             launch_stress<double>(S, A, st);
             launch_velocity<double>(S, A, st);
         } else {
-            pe::StepArgs<float> A = make_args<float>(S, state, 0);
+            pe::StepArgs<float> A = make_args<float>(S, use, 0);
             launch_stress<float>(S, A, st);
             launch_velocity<float>(S, A, st);
         }
     }
+    if (pad && (rc = pad_out(S, state, st))) return rc;
     PE_CUDA(cudaGetLastError());
     // then the adjoint steps backwards through it, the gradient sums spread
     // over replicas of the table (allocated zero on the first segment, left
@@ -1033,10 +1135,11 @@ int pe_solver_profile(PeSolver *S, const PeState *state, int n_steps, float *ms_
     for (auto &e : ev) PE_CUDA(cudaEventCreate(&e));
     PE_CUDA(cudaEventRecord(S->ev_in, user));
     PE_CUDA(cudaStreamWaitEvent(S->stream, S->ev_in, 0));
-    {
-        const int rc0 = ensure_maps(S, state);
-        if (rc0) return rc0;
-    }
+    const bool pad = S->padded && n_steps >= PAD_MIN_STEPS;
+    const PeState *use = pad ? &S->pst : state;
+    int rc = ensure_maps(S, use);
+    if (rc) return rc;
+    if (pad && (rc = pad_in(S, state, S->stream))) return rc;
     pe::k_step_set<<<1, 1, 0, S->stream>>>(S->step, 0);
     float tot_s = 0.f, tot_v = 0.f;
     const int saved_chunk = S->chunk;
@@ -1044,12 +1147,12 @@ int pe_solver_profile(PeSolver *S, const PeState *state, int n_steps, float *ms_
         // one step at a time with events around each kernel (no graph)
         PE_CUDA(cudaEventRecord(ev[0], S->stream));
         if (S->cfg.dtype == PE_F64) {
-            pe::StepArgs<double> A = make_args<double>(S, state, 0);
+            pe::StepArgs<double> A = make_args<double>(S, use, 0);
             launch_stress<double>(S, A, S->stream);
             PE_CUDA(cudaEventRecord(ev[1], S->stream));
             launch_velocity<double>(S, A, S->stream);
         } else {
-            pe::StepArgs<float> A = make_args<float>(S, state, 0);
+            pe::StepArgs<float> A = make_args<float>(S, use, 0);
             launch_stress<float>(S, A, S->stream);
             PE_CUDA(cudaEventRecord(ev[1], S->stream));
             launch_velocity<float>(S, A, S->stream);
@@ -1065,6 +1168,7 @@ int pe_solver_profile(PeSolver *S, const PeState *state, int n_steps, float *ms_
     }
     S->chunk = saved_chunk;
     for (auto &e : ev) cudaEventDestroy(e);
+    if (pad && (rc = pad_out(S, state, S->stream))) return rc;
     PE_CUDA(cudaEventRecord(S->ev_out, S->stream));
     PE_CUDA(cudaStreamWaitEvent(user, S->ev_out, 0));
     ms_out[0] = tot_s / n_steps;
@@ -1212,6 +1316,11 @@ struct PeBatch {
     int *nmats = nullptr;
     pe::BatchItem *items_s = nullptr, *items_v = nullptr;
     int n_items_s = 0, n_items_v = 0;
+    // padded solves' items come last in the lists, for the persistent launches:
+    // per-step launches and short runs, which step the callers' states in
+    // place, leave them out (batched(), items_in_use())
+    int n_inplace_s = 0, n_inplace_v = 0;
+    bool pad_on = false;            // this run goes through the padded states
     int grid_s = 1, grid_v = 1;
     size_t smem_s = 0, smem_v = 0;
     int z_chunk = 0, chunk = 200;
@@ -1253,10 +1362,20 @@ struct PeBatch {
 
 namespace {
 
+// Whether padded solves share the batch's launches: in persistent mode, whose
+// phases they fill up. With per-step launches each runs its own pair.
+bool pad_shared(const PeBatch *B) { return B->pad_on && B->persistent; }
+
 // Whether solve S runs inside the batched TMA launches (else its own pair).
 bool batched(const PeBatch *B, const PeSolver *S)
 {
-    return B->pair_batch ? (S->pair_capable && !S->solo) : (B->tma_batch && S->tma_capable);
+    return B->pair_batch ? ((S->pair_capable || (S->padded && pad_shared(B))) && !S->solo)
+                         : (B->tma_batch && S->tma_capable);
+}
+void items_in_use(const PeBatch *B, int *n_s, int *n_v)
+{
+    *n_s = pad_shared(B) ? B->n_items_s : B->n_inplace_s;
+    *n_v = pad_shared(B) ? B->n_items_v : B->n_inplace_v;
 }
 
 // Pair-kernel layout of an FP32 batch: work items, grids and shared memory.
@@ -1272,8 +1391,8 @@ int batch_layout_pair(PeBatch *B, int nsm, int optin, std::vector<pe::BatchItem>
         const PeConfig &c = S->cfg;
         const long long tiles = (long long)((c.nx + pe::PS_OX) / pe::PS_OX) * ((c.ny + pe::PS_OY - 1) / pe::PS_OY);
         const long long blocks = tiles * ((c.nz + S->zc_ps - 1) / std::max(1, S->zc_ps));
-        S->solo = S->pair_capable && S->zc_ps > 0 && blocks >= 2LL * nsm;
-        if (S->pair_capable && !S->solo) {
+        S->solo = (S->pair_capable || S->padded) && S->zc_ps > 0 && blocks >= 2LL * nsm;
+        if ((S->pair_capable || S->padded) && !S->solo) {
             max_mat = std::max(max_mat, S->cfg.n_mat);
             B->pair_nc4 = B->pair_nc4 && S->cfg.n_coeffs == 4;
         }
@@ -1305,17 +1424,23 @@ int batch_layout_pair(PeBatch *B, int nsm, int optin, std::vector<pe::BatchItem>
     PE_CUDA(setattr((const void *)pe::k_pair_batch_persistent<0, true>));
     PE_CUDA(setattr((const void *)pe::k_pair_batch_persistent<0, false>));
     B->smem_p = pe::persistent_pair_smem(B->smem_s, B->smem_v);
-    for (int s = 0; s < (int)B->solves.size(); ++s) {
-        PeSolver *S = B->solves[s];
-        if (!batched(B, S)) continue;
-        const PeConfig &c = S->cfg;
-        const int zc = S->zc_s;
-        const int nzc = (c.nz + zc - 1) / zc;
-        for (int bz = 0; bz < nzc; ++bz) {
-            for (int by = 0; by < (c.ny + pe::PS_OY - 1) / pe::PS_OY; ++by)
-                for (int bx = 0; bx < (c.nx + pe::PS_OX) / pe::PS_OX; ++bx) is.push_back({s, bx, by, bz});
-            for (int by = 0; by < (c.ny + pe::PV_OY - 1) / pe::PV_OY; ++by)
-                for (int bx = 0; bx < (c.nx + pe::PV_OX - 1) / pe::PV_OX; ++bx) iv.push_back({s, bx, by, bz});
+    for (int pass = 0; pass < 2; ++pass) {   // solves stepped in place, then padded ones
+        for (int s = 0; s < (int)B->solves.size(); ++s) {
+            PeSolver *S = B->solves[s];
+            if (S->solo || !(pass ? S->padded : S->pair_capable)) continue;
+            const PeConfig &c = S->cfg;
+            const int zc = S->zc_s;
+            const int nzc = (c.nz + zc - 1) / zc;
+            for (int bz = 0; bz < nzc; ++bz) {
+                for (int by = 0; by < (c.ny + pe::PS_OY - 1) / pe::PS_OY; ++by)
+                    for (int bx = 0; bx < (c.nx + pe::PS_OX) / pe::PS_OX; ++bx) is.push_back({s, bx, by, bz});
+                for (int by = 0; by < (c.ny + pe::PV_OY - 1) / pe::PV_OY; ++by)
+                    for (int bx = 0; bx < (c.nx + pe::PV_OX - 1) / pe::PV_OX; ++bx) iv.push_back({s, bx, by, bz});
+            }
+        }
+        if (!pass) {
+            B->n_inplace_s = (int)is.size();
+            B->n_inplace_v = (int)iv.size();
         }
     }
     int per_v = 1, per_s = 1, per_p = 1;
@@ -1352,7 +1477,7 @@ int batch_layout(PeBatch *B)
     B->pair_batch = false;
     if constexpr (std::is_same<T, float>::value) {
         bool any = false;
-        for (PeSolver *S : B->solves) any = any || S->pair_capable;
+        for (PeSolver *S : B->solves) any = any || S->pair_capable || S->padded;
         if (any) {
             B->pair_batch = true;
             int rc0 = batch_layout_pair(B, nsm, optin, is, iv);
@@ -1399,6 +1524,10 @@ int batch_layout(PeBatch *B)
     }
     B->n_items_s = (int)is.size();
     B->n_items_v = (int)iv.size();
+    if (!B->pair_batch) {
+        B->n_inplace_s = B->n_items_s;
+        B->n_inplace_v = B->n_items_v;
+    }
     if (B->items_s) dev_free(B->items_s);
     if (B->items_v) dev_free(B->items_v);
     B->items_s = B->items_v = nullptr;
@@ -1429,11 +1558,12 @@ int batch_upload(PeBatch *B, const PeState *states, void *const *traces)
     std::vector<const float *> tabs(n, nullptr);
     for (int s = 0; s < n; ++s) {
         PeSolver *S = B->solves[s];
-        int rc = ensure_maps(S, &states[s]);
+        const PeState *use = B->pad_on && S->padded ? &S->pst : &states[s];
+        int rc = ensure_maps(S, use);
         if (rc) return rc;
         if (batched(B, S) && !(B->pair_batch ? S->pair : S->tma))
             return fail(PE_ERR_UNSUPPORTED, "batched solves need 16-byte aligned state buffers");
-        descs[s] = make_args<T>(S, &states[s], 0);
+        descs[s] = make_args<T>(S, use, 0);
         descs[s].step = B->step;
         descs[s].status = B->status;
         descs[s].zc = S->zc_s;
@@ -1480,7 +1610,8 @@ int launch_pair_persistent(PeBatch *B, int len)
     const pe::TmapsPairVelocity *mv = B->pmaps_v;
     const int *nm = B->nmats;
     const pe::BatchItem *is = B->items_s, *iv = B->items_v;
-    const int ns = B->n_items_s, nv = B->n_items_v;
+    int ns, nv;
+    items_in_use(B, &ns, &nv);
     cudaError_t e;
     if (B->pair_nc4 && B->pair_ts)
         e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, true>, d, ms, mv, tabs, nm, is, ns, iv, nv, len, B->bar, B->status);
@@ -1499,17 +1630,19 @@ template <typename T>
 int batch_chunk(PeBatch *B, int len)
 {
     const dim3 block(pe::TB_X, pe::TB_Y, 1);
+    int n_s, n_v;
+    items_in_use(B, &n_s, &n_v);
     if constexpr (std::is_same<T, float>::value) {
-        if (B->pair_batch && B->persistent && B->n_items_s > 0) {
+        if (B->pair_batch && B->persistent && n_s > 0) {
             const int rc = launch_pair_persistent(B, len);
             if (rc) return rc;
         }
     }
     for (int k = 0; k < len; ++k) {
         if constexpr (std::is_same<T, float>::value) {
-            if (B->pair_batch && !B->persistent && B->n_items_s > 0) {
+            if (B->pair_batch && !B->persistent && n_s > 0) {
                 const pe::StepArgs<float> *d = (const pe::StepArgs<float> *)B->descs;
-                const int ns = B->n_items_s, nv = B->n_items_v;
+                const int ns = n_s, nv = n_v;
                 if (B->pair_nc4 && B->pair_ts)
                     pe::k_stress_pair_batch<4, true><<<B->grid_s, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, B->items_s, ns, k);
                 else if (B->pair_nc4)
@@ -1538,7 +1671,7 @@ int batch_chunk(PeBatch *B, int len)
         for (int s = 0; s < (int)B->solves.size(); ++s) {
             PeSolver *S = B->solves[s];
             if (batched(B, S)) continue;
-            pe::StepArgs<T> A = make_args<T>(S, &B->states[s], k);
+            pe::StepArgs<T> A = make_args<T>(S, B->pad_on && S->padded ? &S->pst : &B->states[s], k);
             A.step = B->step;
             A.status = B->status;
             launch_stress<T>(S, A, B->stream);
@@ -1564,12 +1697,20 @@ int batch_chunk(PeBatch *B, int len)
 template <typename T>
 int batch_run_t(PeBatch *B, const PeState *states, void *const *traces, int64_t b, int64_t e, cudaStream_t user)
 {
+    bool pad = false;
+    for (const PeSolver *S : B->solves) pad = pad || (B->pair_batch && S->padded && e - b >= PAD_MIN_STEPS);
+    if (pad != B->pad_on) {   // other states and launches than the ones uploaded
+        B->pad_on = pad;
+        B->uploaded = false;
+    }
     int rc = batch_upload<T>(B, states, traces);
     if (rc) return rc;
     PE_CUDA(cudaEventRecord(B->ev_in, user));
     PE_CUDA(cudaStreamWaitEvent(B->stream, B->ev_in, 0));
     pe::k_step_set<<<1, 1, 0, B->stream>>>(B->step, b);
     B->launches += 1;
+    for (int s = 0; pad && s < (int)B->solves.size(); ++s)
+        if (B->solves[s]->padded && (rc = pad_in(B->solves[s], &states[s], B->stream))) return rc;
     for (int64_t n = b; n < e;) {
         const int len = (int)std::min<int64_t>(B->chunk, e - n);
         if (len == B->chunk) {
@@ -1594,6 +1735,8 @@ int batch_run_t(PeBatch *B, const PeState *states, void *const *traces, int64_t 
         }
         n += len;
     }
+    for (int s = 0; pad && s < (int)B->solves.size(); ++s)
+        if (B->solves[s]->padded && (rc = pad_out(B->solves[s], &states[s], B->stream))) return rc;
     PE_CUDA(cudaEventRecord(B->ev_out, B->stream));
     PE_CUDA(cudaStreamWaitEvent(user, B->ev_out, 0));
     return PE_OK;

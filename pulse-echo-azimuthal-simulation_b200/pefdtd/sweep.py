@@ -270,8 +270,12 @@ def azimuth_setup(cfg, build, co, az, labeller=None):
 
 def setup_bytes(setup, dtype_size=4):
     """Device bytes one solve of this setup holds: nine fields, labels,
-    damping volume, traces."""
-    cells = int(np.prod(setup["spec"]["mats"].shape))
+    damping volume (and, where rows are not 16-byte multiples, the solver's
+    row-padded copies of them), traces."""
+    nz, ny, nx = setup["spec"]["mats"].shape
+    cells = nz * ny * nx
+    if nx % 4 and dtype_size == 4:
+        cells += nz * ny * (-(-nx // 4) * 4)
     return cells * (9 * dtype_size + 2 + 4) + setup["nt"] * dtype_size + (64 << 20)
 
 
