@@ -40,8 +40,8 @@ struct StepArgs {
     T *v[3];
     T *s[6];
     const uint16_t *lab;     // material | flags
-    const T *c21;            // (n_mat, C21_STRIDE)
-    const T *rho;            // (n_mat,)
+    const T *c21;            // (n_mat, C21_STRIDE); per-cell media: 21 planes, cplane apart
+    const T *rho;            // (n_mat,); per-cell media: one plane
     const float *rinv;       // (n_mat,) RN32(1 / rho) (FP32 solves), or null
     const float *dz, *dy, *dx;  // sponge tapers or null
     const float *dvol;          // damping volume or null
@@ -67,7 +67,10 @@ struct StepArgs {
     int k;                      // step within the chunk
     int zc;                     // planes per z-march
     int *status;                // device status word (bounded waits record timeouts)
-    int dense;                  // per-cell media: the table row of cell i is i (untiled kernels)
+    // per-cell media: planes of (nz, ny, cpitch) values, one per constant
+    int dense;
+    int cpitch;
+    long long cplane;
 };
 
 // ---------------------------------------------------------------- helpers
@@ -285,10 +288,16 @@ __global__ void __launch_bounds__(TX *TY) k_stress(const StepArgs<T> A)
 
             const long long idx = z * A.sz + iy * A.sy + ix;
             const uint16_t lab = A.lab[idx];
-            const T *Cr = A.c21 + (A.dense ? idx : (long long)(lab & LAB_MAT)) * C21_STRIDE;
             T Cm[21];
+            if (A.dense) {
+                const T *Cr = A.c21 + ((long long)z * A.ny + iy) * A.cpitch + ix;
 #pragma unroll
-            for (int k = 0; k < 21; ++k) Cm[k] = ldg(Cr + k);
+                for (int k = 0; k < 21; ++k) Cm[k] = ldg(Cr + k * A.cplane);
+            } else {
+                const T *Cr = A.c21 + (long long)(lab & LAB_MAT) * C21_STRIDE;
+#pragma unroll
+                for (int k = 0; k < 21; ++k) Cm[k] = ldg(Cr + k);
+            }
             const T dmp = (T)damp_at(A, z, iy, ix, idx);
             T acc[6];
             acc[0] = row_dot(Cm, 0, q0);
@@ -378,14 +387,15 @@ __global__ void __launch_bounds__(TX *TY) k_velocity(const StepArgs<T> A)
             }
         }
         const uint16_t lab = A.lab[idx];
-        // density of a cell: its table row (the cell itself for per-cell media)
-        auto rho_at = [&](long long q) -> T {
-            return ldg(A.rho + (A.dense ? q : (long long)(A.lab[q] & LAB_MAT)));
+        // density of the cell dz, dy, dx away: its table row (its own value for per-cell media)
+        auto rho_at = [&](int dz, int dy, int dx) -> T {
+            if (A.dense) return ldg(A.rho + ((long long)(iz + dz) * ny + iy + dy) * A.cpitch + ix + dx);
+            return ldg(A.rho + (A.lab[idx + dz * sz + dy * sy + dx] & LAB_MAT));
         };
-        const T r0 = rho_at(idx);
-        const T rvx = (ix < nx - 1) ? T(0.5) * (r0 + rho_at(idx + 1)) : r0;
-        const T rvy = (iy < ny - 1) ? T(0.5) * (r0 + rho_at(idx + sy)) : r0;
-        const T rvz = (iz < nz - 1) ? T(0.5) * (r0 + rho_at(idx + sz)) : r0;
+        const T r0 = rho_at(0, 0, 0);
+        const T rvx = (ix < nx - 1) ? T(0.5) * (r0 + rho_at(0, 0, 1)) : r0;
+        const T rvy = (iy < ny - 1) ? T(0.5) * (r0 + rho_at(0, 1, 0)) : r0;
+        const T rvz = (iz < nz - 1) ? T(0.5) * (r0 + rho_at(1, 0, 0)) : r0;
         const T dmp = (T)damp_at(A, iz, iy, ix, idx);
         T tx = A.dt_h * ax, ty = A.dt_h * ay, tz = A.dt_h * az;
         tx = div_face(tx, rvx); ty = div_face(ty, rvy); tz = div_face(tz, rvz);
@@ -452,6 +462,19 @@ __global__ void k_labels_flag(uint16_t *lab, const long long *cells, int n, uint
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) lab[cells[i]] = lab[cells[i]] | flag;
+}
+
+// per-cell media: rows of 36 to 21 planes of (nz, ny, pitch), `rows` grid rows
+// of nx cells; the pad columns repeat the row's last cell
+template <typename T>
+__global__ void k_c36_to_planes(const T *c36, const T *rho, T *planes, T *rho_p, int nx, int pitch, long long rows)
+{
+    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= rows * pitch) return;
+    const long long r = q / pitch, i = r * nx + min((int)(q % pitch), nx - 1);
+    for (int I = 0; I < 6; ++I)
+        for (int J = I; J < 6; ++J) planes[c21_slot(I, J) * rows * pitch + q] = c36[i * 36 + I * 6 + J];
+    rho_p[q] = rho[i];
 }
 
 template <typename T>

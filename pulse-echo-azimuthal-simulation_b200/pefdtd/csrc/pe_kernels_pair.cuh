@@ -370,6 +370,36 @@ __device__ __forceinline__ void stiff_column(const float *const (&pl)[4], const 
     }
 }
 
+// The same column for per-cell media: the constants of both cells are one
+// 64-bit load from each constant's plane (consecutive lanes, consecutive
+// addresses), so the products run as lane pairs.
+template <int J, bool G>
+__device__ __forceinline__ void stiff_column_cell(const float *const (&pl)[4], const MoveGuards &mg, const float *cell,
+                                                  long long cplane, float2 (&acc)[6])
+{
+    float2 q[4];
+    qpair<0, J, G>(pl, mg, q[0]);
+    qpair<1, J, G>(pl, mg, q[1]);
+    qpair<2, J, G>(pl, mg, q[2]);
+    qpair<3, J, G>(pl, mg, q[3]);
+#pragma unroll
+    for (int I = 0; I < 6; ++I) acc[I] = fmac2(acc[I], ldg2(cell + c21_slot(I, J) * cplane), q[vpos(I)]);
+}
+
+template <bool G>
+__device__ __forceinline__ void stiff_all_cell(const float *const (&pl)[4], const MoveGuards &mg, const float *cell,
+                                               long long cplane, float2 (&acc)[6])
+{
+#pragma unroll
+    for (int I = 0; I < 6; ++I) acc[I] = bc2(0.f);
+    stiff_column_cell<0, G>(pl, mg, cell, cplane, acc);
+    stiff_column_cell<1, G>(pl, mg, cell, cplane, acc);
+    stiff_column_cell<2, G>(pl, mg, cell, cplane, acc);
+    stiff_column_cell<3, G>(pl, mg, cell, cplane, acc);
+    stiff_column_cell<4, G>(pl, mg, cell, cplane, acc);
+    stiff_column_cell<5, G>(pl, mg, cell, cplane, acc);
+}
+
 template <bool G, bool TS>
 __device__ __forceinline__ void stiff_all(const float *const (&pl)[4], const MoveGuards &mg,
                                           const float *const (&crow)[2], float2 (&acc)[6])
@@ -420,7 +450,8 @@ __device__ __forceinline__ bool pair_tile_inside(const StepArgs<float> &A, int b
 // are issued a plane ahead. The caller synchronises the block before a march
 // that follows another. TIN: pair_tile_inside(A, bx, by) holds, and the
 // x / y limits and guards are compile-time constants.
-template <int NC, bool TS, bool TIN, bool COH = false>
+// CM: per-cell media (TS is then unused).
+template <int NC, bool TS, bool TIN, bool COH = false, bool CM = false>
 __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, const StepArgs<float> &A,
                                                   const float *tab, unsigned char *smem, int bx, int by,
                                                   int zb, int ze, PairPhases &ph)
@@ -574,10 +605,16 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
             mg.zlo = z >= 1;
             mg.zhi = z <= nz - 2;
             const uint16_t lab[2] = {(uint16_t)(lab2 & 0xFFFFu), (uint16_t)(lab2 >> 16)};
-            const float *const crow[2] = {tab + (lab[0] & LAB_MAT) * TAB36, tab + (lab[1] & LAB_MAT) * TAB36};
             float2 acc[6];
-            if (fast) stiff_all<false, TS>(pl, mg, crow, acc);
-            else stiff_all<true, TS>(pl, mg, crow, acc);
+            if constexpr (CM) {
+                const float *const cell = A.c21 + (long long)z * sz + col;
+                if (fast) stiff_all_cell<false>(pl, mg, cell, A.cplane, acc);
+                else stiff_all_cell<true>(pl, mg, cell, A.cplane, acc);
+            } else {
+                const float *const crow[2] = {tab + (lab[0] & LAB_MAT) * TAB36, tab + (lab[1] & LAB_MAT) * TAB36};
+                if (fast) stiff_all<false, TS>(pl, mg, crow, acc);
+                else stiff_all<true, TS>(pl, mg, crow, acc);
+            }
             const float *sc = sslots + (us & 1) * PS_SSLOT + cs;
             float dmp[2];
             {
@@ -722,7 +759,7 @@ __host__ __device__ constexpr int pair_last_inside_y(int ny) { return ny < 19 ? 
 // Launch grid: (tiles x, tiles y, z-chunks of A.zc planes). Blocks that run
 // at the same time march the same planes of neighbouring tiles, so the tile
 // halos they share are read from DRAM once and from L2 after that.
-template <int NC, bool TS>
+template <int NC, bool TS, bool CM = false>
 __global__ void __launch_bounds__(PS_N, 2) k_stress_pair(const __grid_constant__ TmapsPairStress M,
                                                          const StepArgs<float> A,
                                                          const float *__restrict__ tab36, int n_mat)
@@ -738,9 +775,9 @@ __global__ void __launch_bounds__(PS_N, 2) k_stress_pair(const __grid_constant__
     interior_first(pair_last_inside_x(A.nx), pair_last_inside_y(A.ny), gridDim.x, gridDim.y,
                    blockIdx.x + gridDim.x * blockIdx.y, bx, by);
     if (pair_tile_inside(A, bx, by))
-        stress_pair_march<NC, TS, true>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
+        stress_pair_march<NC, TS, true, false, CM>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
     else
-        stress_pair_march<NC, TS, false>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
+        stress_pair_march<NC, TS, false, false, CM>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
 }
 
 // ====================================================================== velocity
@@ -884,7 +921,9 @@ __device__ __forceinline__ bool pair_vtile_inside(const StepArgs<float> &A, int 
 // x / y limits and neighbour tests are compile-time constants.
 // bars_at: the three mbarriers (default: the first bytes of smem; the
 // persistent batch kernel keeps separate ones for each phase)
-template <int NC, bool TIN, bool COH = false>
+// CM: per-cell media: the densities themselves are loaded where the table
+// variant loads labels, and the own density's reciprocal is formed in place.
+template <int NC, bool TIN, bool COH = false, bool CM = false>
 __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, const StepArgs<float> &A,
                                                    const float *rho_tab, unsigned char *smem, int bx,
                                                    int by, int zb, int ze, int it0,
@@ -962,10 +1001,31 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
             if (yin) py = __ldg(lab32 + ((b + sy) >> 1));
         }
     };
-    uint32_t lab_c, lab_y, nlab_c, nlab_y;
-    uint16_t lab_x2, nlab_x2;
-    ldlabs(zb, lab_c, lab_x2, lab_y);
-    ldlabs(zb + 1, nlab_c, nlab_x2, nlab_y);
+    uint32_t lab_c = 0, lab_y = 0, nlab_c = 0, nlab_y = 0;
+    uint16_t lab_x2 = 0, nlab_x2 = 0;
+    // per-cell media: the densities at the same places
+    struct Rho {
+        float2 c, y;
+        float x2;
+    };
+    auto ldrho = [&](int z) -> Rho {
+        Rho r{make_float2(0.f, 0.f), make_float2(0.f, 0.f), 0.f};
+        if (out_ok && z < nz) {
+            const float *q = A.rho + (long long)z * sz + col;
+            r.c = ldg2(q);
+            if (xin1) r.x2 = __ldg(q + 2);
+            if (yin) r.y = ldg2(q + sy);
+        }
+        return r;
+    };
+    Rho rho_c{}, nrho{};
+    if constexpr (CM) {
+        rho_c = ldrho(zb);
+        nrho = ldrho(zb + 1);
+    } else {
+        ldlabs(zb, lab_c, lab_x2, lab_y);
+        ldlabs(zb + 1, nlab_c, nlab_x2, nlab_y);
+    }
     int *status = A.status;
 
     issue(0);
@@ -977,9 +1037,15 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
         __syncthreads();   // slot g landed (observed by warp 0); slot g + 2 is free
         issue(i + 2);
         const float2 n3 = ld2col(p3, z + 5), n4 = ld2col(p4, z + 4), n5 = ld2col(p5, z + 4);
-        uint32_t mlab_c, mlab_y;
-        uint16_t mlab_x2;
-        ldlabs(z + 2, mlab_c, mlab_x2, mlab_y);
+        uint32_t mlab_c = 0, mlab_y = 0;
+        uint16_t mlab_x2 = 0;
+        Rho mrho{};
+        if constexpr (CM) {
+            mrho = ldrho(z + 2);
+            if (out_ok && A.rec_kind != 0) lab_c = __ldg(lab32 + (((long long)z * sz + col) >> 1));   // receiver flags
+        } else {
+            ldlabs(z + 2, mlab_c, mlab_x2, mlab_y);
+        }
         const float *slot = slots + sl * PV_SLOT;
         const float *t = slot + tc;
         float2 ax, ay, az;
@@ -1015,15 +1081,23 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
             float r0[2], rn[2][3];
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                const bool xin = c == 0 ? two : xin1;
-                r0[c] = rho_tab[lc[c] & LAB_MAT];
-                rn[c][0] = xin ? rho_tab[lxv[c] & LAB_MAT] : 0.f;
-                rn[c][1] = yin ? rho_tab[lyv[c] & LAB_MAT] : 0.f;
-                rn[c][2] = (z < nz - 1) ? rho_tab[lzv[c] & LAB_MAT] : 0.f;
+                if constexpr (CM) {
+                    r0[c] = pick(rho_c.c, c);
+                    rn[c][0] = c == 0 ? rho_c.c.y : rho_c.x2;
+                    rn[c][1] = pick(rho_c.y, c);
+                    rn[c][2] = pick(nrho.c, c);
+                } else {
+                    const bool xin = c == 0 ? two : xin1;
+                    r0[c] = rho_tab[lc[c] & LAB_MAT];
+                    rn[c][0] = xin ? rho_tab[lxv[c] & LAB_MAT] : 0.f;
+                    rn[c][1] = yin ? rho_tab[lyv[c] & LAB_MAT] : 0.f;
+                    rn[c][2] = (z < nz - 1) ? rho_tab[lzv[c] & LAB_MAT] : 0.f;
+                }
             }
             const bool has_nb[2][3] = {{two, yin, z < nz - 1}, {xin1, yin, z < nz - 1}};
             const float2 r02 = make_float2(r0[0], r0[1]);
-            const float2 y2 = make_float2(__ldg(A.rinv + (lc[0] & LAB_MAT)), __ldg(A.rinv + (lc[1] & LAB_MAT)));
+            const float2 y2 = CM ? make_float2(__frcp_rn(r0[0]), __frcp_rn(r0[1]))
+                                 : make_float2(__ldg(A.rinv + (lc[0] & LAB_MAT)), __ldg(A.rinv + (lc[1] & LAB_MAT)));
             const float2 a2[3] = {ax, ay, az};
             float2 u[3], rv[3], q[3];
             bool fine = true;
@@ -1076,6 +1150,8 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
         }
         lab_c = nlab_c; lab_x2 = nlab_x2; lab_y = nlab_y;
         nlab_c = mlab_c; nlab_x2 = mlab_x2; nlab_y = mlab_y;
+        rho_c = nrho;
+        nrho = mrho;
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
             r3[k] = r3[k + 1];
@@ -1089,7 +1165,7 @@ __device__ __forceinline__ int velocity_pair_march(const TmapsPairVelocity &M, c
     return ze - zb;
 }
 
-template <int NC>
+template <int NC, bool CM = false>
 __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant__ TmapsPairVelocity M,
                                                            const StepArgs<float> A, int n_mat)
 {
@@ -1101,7 +1177,7 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
         fence_mbar_init();
     }
-    const bool rho_smem = pair_rho_in_smem(n_mat);
+    const bool rho_smem = !CM && pair_rho_in_smem(n_mat);
     if (rho_smem)
         for (int i = tid; i < n_mat; i += PV_N) rsm[i] = A.rho[i];
     __syncthreads();
@@ -1111,9 +1187,9 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
     interior_first(A.nx < 36 ? 0 : (A.nx - 36) / PV_OX, A.ny < 20 ? 0 : (A.ny - 20) / PV_OY, gridDim.x,
                    gridDim.y, blockIdx.x + gridDim.x * blockIdx.y, bx, by);
     if (pair_vtile_inside(A, bx, by))
-        velocity_pair_march<NC, true>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
+        velocity_pair_march<NC, true, false, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
     else
-        velocity_pair_march<NC, false>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
+        velocity_pair_march<NC, false, false, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
 }
 
 // ---------------------------------------------------------------- batches

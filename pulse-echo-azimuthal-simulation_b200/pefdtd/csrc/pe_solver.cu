@@ -263,6 +263,8 @@ pe::StepArgs<T> make_args(const PeSolver *S, const PeState *st, int k)
     A.zc = S->zc_s;
     A.status = S->status;
     A.dense = S->variant == PE_KERNEL_DENSE;
+    A.cpitch = S->px;
+    A.cplane = (long long)S->px * S->cfg.ny * S->cfg.nz;
     return A;
 }
 
@@ -284,7 +286,7 @@ void launch_simple_velocity(pe::StepArgs<T> A, int zc, cudaStream_t st)
 template <typename T>
 void launch_stress(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t st)
 {
-    if (S->variant == PE_KERNEL_SIMPLE || S->variant == PE_KERNEL_DENSE) {
+    if (S->variant == PE_KERNEL_SIMPLE || (S->variant == PE_KERNEL_DENSE && !S->pair)) {
         if (S->ty == 8) launch_simple_stress<T, 32, 8>(A0, S->zc_s, st);
         else launch_simple_stress<T, 32, 4>(A0, S->zc_s, st);
         return;
@@ -295,6 +297,11 @@ void launch_stress(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t st
             A.zc = S->zc_ps;
             // stress tiles update columns [30 bx - 1, 30 bx + 29)
             dim3 grid((A.nx + pe::PS_OX) / pe::PS_OX, (A.ny + pe::PS_OY - 1) / pe::PS_OY, (A.nz + A.zc - 1) / A.zc);
+            if (A.dense) {
+                if (A.nc == 4) pe::k_stress_pair<4, false, true><<<grid, pe::PS_N, pe::PS_SMEM_FIXED, st>>>(S->mps, A, nullptr, 0);
+                else pe::k_stress_pair<0, false, true><<<grid, pe::PS_N, pe::PS_SMEM_FIXED, st>>>(S->mps, A, nullptr, 0);
+                return;
+            }
             const int nm = S->cfg.n_mat;
             const size_t sm = pe::stress_pair_smem(nm);
             const bool ts = pe::pair_tab_in_smem(nm);
@@ -320,7 +327,7 @@ void launch_stress(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t st
 template <typename T>
 void launch_velocity(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t st)
 {
-    if (S->variant == PE_KERNEL_SIMPLE || S->variant == PE_KERNEL_DENSE) {
+    if (S->variant == PE_KERNEL_SIMPLE || (S->variant == PE_KERNEL_DENSE && !S->pair)) {
         if (S->ty == 8) launch_simple_velocity<T, 32, 8>(A0, S->zc_v, st);
         else launch_simple_velocity<T, 32, 4>(A0, S->zc_v, st);
         return;
@@ -330,6 +337,12 @@ void launch_velocity(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t 
         if (S->pair) {
             A.zc = S->zc_pv;
             dim3 grid((A.nx + pe::PV_OX - 1) / pe::PV_OX, (A.ny + pe::PV_OY - 1) / pe::PV_OY, (A.nz + A.zc - 1) / A.zc);
+            if (A.dense) {
+                const size_t smc = pe::velocity_pair_smem(0);
+                if (A.nc == 4) pe::k_velocity_pair<4, true><<<grid, pe::PV_N, smc, st>>>(S->mpv, A, 0);
+                else pe::k_velocity_pair<0, true><<<grid, pe::PV_N, smc, st>>>(S->mpv, A, 0);
+                return;
+            }
             const size_t sm = pe::velocity_pair_smem(S->cfg.n_mat);
             if (A.nc == 4)
                 pe::k_velocity_pair<4><<<grid, pe::PV_N, sm, st>>>(S->mpv, A, S->cfg.n_mat);
@@ -470,21 +483,53 @@ int encode_box(CUtensorMap *m, const void *base, CUtensorMapDataType dt, int es,
     return PE_OK;
 }
 
+// Pair kernels for this solve (FP32): in place, on row-padded copies or not at
+// all, and their z-marches.
+int configure_pair(PeSolver *S, int optin)
+{
+    const PeConfig &c = S->cfg;
+    const bool dense = S->variant == PE_KERNEL_DENSE;
+    const int nm = dense ? 0 : c.n_mat;   // per-cell media: no table in shared memory
+    const size_t ps = dense ? pe::PS_SMEM_FIXED : pe::stress_pair_smem(nm), pv = pe::velocity_pair_smem(nm);
+    // per-cell media asked for with an explicit tile run the untiled kernels that have tiles
+    const bool pair_ok = (S->variant == PE_KERNEL_TILED || (dense && c.tile_x <= 0)) && ps <= (size_t)optin &&
+                         pv <= (size_t)optin && encode_fn() != nullptr;
+    S->pair_capable = pair_ok && c.nx % 4 == 0;
+    S->padded = pair_ok && c.nx % 4 != 0;
+    if (!pair_ok) return PE_OK;
+    // the attribute belongs to the kernel, not to this solve: allow the
+    // device maximum so that solves with other table sizes can coexist
+    const void *fns[] = {(const void *)pe::k_stress_pair<4, true>, (const void *)pe::k_stress_pair<4, false>,
+                         (const void *)pe::k_stress_pair<0, true>, (const void *)pe::k_stress_pair<0, false>,
+                         (const void *)pe::k_stress_pair<4, false, true>, (const void *)pe::k_stress_pair<0, false, true>,
+                         (const void *)pe::k_velocity_pair<4>, (const void *)pe::k_velocity_pair<0>,
+                         (const void *)pe::k_velocity_pair<4, true>, (const void *)pe::k_velocity_pair<0, true>};
+    for (const void *f : fns) PE_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+    const long long tps = (long long)((c.nx + pe::PS_OX) / pe::PS_OX) * ((c.ny + pe::PS_OY - 1) / pe::PS_OY);
+    const long long tpv = (long long)((c.nx + pe::PV_OX - 1) / pe::PV_OX) * ((c.ny + pe::PV_OY - 1) / pe::PV_OY);
+    const int sps = occupancy_slots(pe::k_stress_pair<4, true>, pe::PS_N, ps);
+    const int spv = occupancy_slots(pe::k_velocity_pair<4>, pe::PV_N, pv);
+    S->zc_ps = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tps, sps, 3);
+    S->zc_pv = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tpv, spv, 1);
+    return PE_OK;
+}
+
 template <typename T>
 int configure_kernels(PeSolver *S)
 {
     const PeConfig &c = S->cfg;
+    S->px = (c.nx + 3) / 4 * 4;
+    int dev = 0, optin = 0;
+    PE_CUDA(cudaGetDevice(&dev));
+    PE_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     if (S->variant == PE_KERNEL_SIMPLE || S->variant == PE_KERNEL_DENSE) {
         const long long tiles = (long long)((c.nx + S->tx - 1) / S->tx) * ((c.ny + S->ty - 1) / S->ty);
         const int slots = occupancy_slots(pe::k_stress<T, 32, 8>, 32 * S->ty, 0);
         S->zc_s = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tiles, slots, 2);
         S->zc_v = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tiles, slots, 2);
-        return PE_OK;
+        return S->variant == PE_KERNEL_DENSE && std::is_same<T, float>::value ? configure_pair(S, optin) : PE_OK;
     }
     // allow every launch up to the device's opt-in shared memory per block
-    int dev = 0, optin = 0;
-    PE_CUDA(cudaGetDevice(&dev));
-    PE_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const size_t need_s = pe::stress_tiled_smem<T>(c.n_mat), need_v = pe::velocity_tiled_smem<T>(c.n_mat);
     if (need_s > (size_t)optin || need_v > (size_t)optin)
         return fail(PE_ERR_UNSUPPORTED, "tiled kernels need " + std::to_string(need_s) +
@@ -508,30 +553,7 @@ int configure_kernels(PeSolver *S)
     }
     S->zc_s = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, ts, ss, 4);
     S->zc_v = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tv, sv, 3);
-    if constexpr (std::is_same<T, float>::value) {
-        const size_t ps = pe::stress_pair_smem(c.n_mat), pv = pe::velocity_pair_smem(c.n_mat);
-        const bool pair_ok = S->variant == PE_KERNEL_TILED && ps <= (size_t)optin && pv <= (size_t)optin &&
-                             encode_fn() != nullptr;
-        S->pair_capable = pair_ok && c.nx % 4 == 0;
-        S->padded = pair_ok && c.nx % 4 != 0;
-        S->px = (c.nx + 3) / 4 * 4;
-        if (pair_ok) {
-            // the attribute belongs to the kernel, not to this solve: allow the
-            // device maximum so that solves with other table sizes can coexist
-            PE_CUDA(cudaFuncSetAttribute(pe::k_stress_pair<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-            PE_CUDA(cudaFuncSetAttribute(pe::k_stress_pair<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-            PE_CUDA(cudaFuncSetAttribute(pe::k_stress_pair<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-            PE_CUDA(cudaFuncSetAttribute(pe::k_stress_pair<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-            PE_CUDA(cudaFuncSetAttribute(pe::k_velocity_pair<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-            PE_CUDA(cudaFuncSetAttribute(pe::k_velocity_pair<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-            const long long tps = (long long)((c.nx + pe::PS_OX) / pe::PS_OX) * ((c.ny + pe::PS_OY - 1) / pe::PS_OY);
-            const long long tpv = (long long)((c.nx + pe::PV_OX - 1) / pe::PV_OX) * ((c.ny + pe::PV_OY - 1) / pe::PV_OY);
-            const int sps = occupancy_slots(pe::k_stress_pair<4, true>, pe::PS_N, ps);
-            const int spv = occupancy_slots(pe::k_velocity_pair<4>, pe::PV_N, pv);
-            S->zc_ps = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tps, sps, 3);
-            S->zc_pv = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tpv, spv, 1);
-        }
-    }
+    if constexpr (std::is_same<T, float>::value) return configure_pair(S, optin);
     return PE_OK;
 }
 
@@ -741,8 +763,10 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
 
     int rc;
     if ((rc = dev_alloc(&S->lab, sizeof(uint16_t) * ncell))) return rc;
-    if ((rc = dev_alloc(&S->c21, (size_t)es * pe::C21_STRIDE * c.n_mat))) return rc;
-    if ((rc = dev_alloc(&S->rho, (size_t)es * c.n_mat))) return rc;
+    // per-cell media: planes with the pair kernels' row pitch (the untiled kernels read them too)
+    const size_t nplane = (size_t)S->px * c.ny * c.nz;
+    if ((rc = dev_alloc(&S->c21, (size_t)es * (dense ? 21 * nplane : (size_t)pe::C21_STRIDE * c.n_mat)))) return rc;
+    if ((rc = dev_alloc(&S->rho, (size_t)es * (dense ? nplane : (size_t)c.n_mat)))) return rc;
     if ((rc = dev_alloc(&S->step, sizeof(long long)))) return rc;
     if ((rc = dev_alloc(&S->status, sizeof(int)))) return rc;
     PE_CUDA(cudaMemsetAsync(S->status, 0, sizeof(int), st));
@@ -769,11 +793,30 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
         void *c36 = nullptr;
         if ((rc = dev_alloc(&c36, (size_t)es * 36 * c.n_mat))) return rc;
         PE_CUDA(cudaMemcpyAsync(c36, md->ctab, (size_t)es * 36 * c.n_mat, cudaMemcpyHostToDevice, st));
-        if (c.dtype == PE_F64)
-            pe::k_c36_to_c21<double><<<(c.n_mat + 127) / 128, 128, 0, st>>>((const double *)c36, (double *)S->c21, c.n_mat);
-        else
-            pe::k_c36_to_c21<float><<<(c.n_mat + 127) / 128, 128, 0, st>>>((const float *)c36, (float *)S->c21, c.n_mat);
-        PE_CUDA(cudaMemcpyAsync(S->rho, md->rho, (size_t)es * c.n_mat, cudaMemcpyHostToDevice, st));
+        if (dense) {
+            void *rho_rows = nullptr;
+            if ((rc = dev_alloc(&rho_rows, (size_t)es * c.n_mat))) {
+                dev_free(c36);
+                return rc;
+            }
+            PE_CUDA(cudaMemcpyAsync(rho_rows, md->rho, (size_t)es * c.n_mat, cudaMemcpyHostToDevice, st));
+            const unsigned nb = (unsigned)((nplane + 255) / 256);
+            const long long rows = (long long)c.ny * c.nz;
+            if (c.dtype == PE_F64)
+                pe::k_c36_to_planes<double><<<nb, 256, 0, st>>>((const double *)c36, (const double *)rho_rows,
+                                                                (double *)S->c21, (double *)S->rho, c.nx, S->px, rows);
+            else
+                pe::k_c36_to_planes<float><<<nb, 256, 0, st>>>((const float *)c36, (const float *)rho_rows,
+                                                               (float *)S->c21, (float *)S->rho, c.nx, S->px, rows);
+            PE_CUDA(cudaStreamSynchronize(st));
+            dev_free(rho_rows);
+        } else {
+            if (c.dtype == PE_F64)
+                pe::k_c36_to_c21<double><<<(c.n_mat + 127) / 128, 128, 0, st>>>((const double *)c36, (double *)S->c21, c.n_mat);
+            else
+                pe::k_c36_to_c21<float><<<(c.n_mat + 127) / 128, 128, 0, st>>>((const float *)c36, (float *)S->c21, c.n_mat);
+            PE_CUDA(cudaMemcpyAsync(S->rho, md->rho, (size_t)es * c.n_mat, cudaMemcpyHostToDevice, st));
+        }
         if (c.dtype == PE_F32 && !dense) {   // the pair kernels' tables
             if ((rc = dev_alloc(&S->tab36, sizeof(float) * pe::TAB36 * c.n_mat))) return rc;
             pe::k_c21_to_tab36<<<(c.n_mat + 127) / 128, 128, 0, st>>>((const float *)S->c21, S->tab36, c.n_mat);
