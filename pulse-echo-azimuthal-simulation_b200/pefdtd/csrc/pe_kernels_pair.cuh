@@ -168,9 +168,7 @@ __device__ __forceinline__ float2 ldg2_stream(const float *p)
 __device__ __forceinline__ float2 ldcg2(const float *p)
 {
     float2 v;
-    // volatile keeps it behind the grid barrier's asm; without a memory clobber
-    // the arithmetic around it stays free to move
-    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
     return v;
 }
 template <bool COH>
@@ -416,36 +414,6 @@ __device__ __forceinline__ void stiff_all(const float *const (&pl)[4], const Mov
     stiff_column<5, G, TS>(pl, mg, crow, acc);
 }
 
-// The stiffness product of a warp whose cells are all material 0, the fluid
-// couplant (every constant outside the normal block exactly zero, see
-// StepArgs::fluid0): the full product's moved strains only meet zeros there,
-// and fma(0, q, acc) == acc bit for bit for finite q, so the product is nine
-// paired FMAs on three strains. A third to a half of a disk problem's cells
-// are couplant (all of its edge tiles' corners, the planes above and below the
-// disk). The caller has established that every strain of the block so far is
-// finite and small enough for the moves' sums (strain_bad).
-__device__ __forceinline__ void stiff_fluid(const StepArgs<float> &A, const float *const (&pl)[4], float2 (&acc)[6])
-{
-#pragma unroll
-    for (int I = 0; I < 6; ++I) acc[I] = bc2(0.f);
-#pragma unroll
-    for (int J = 0; J < 3; ++J) {
-        const float2 q = lds2(gptr(pl, J, 0, 0));
-#pragma unroll
-        for (int I = 0; I < 3; ++I) acc[I] = fmac2(acc[I], bc2(A.cfl[3 * I + J]), q);
-    }
-}
-// a strain that is not finite, or above 1e19, where a move's sum of four and
-// the square below are still far from overflow
-__device__ __forceinline__ bool strain_bad(const float2 (&g)[6])
-{
-    float2 t = mul2(g[0], g[0]);
-#pragma unroll
-    for (int J = 1; J < 6; ++J) t = fmac2(t, g[J], g[J]);
-    return !(t.x + t.y < 3.0e38f);
-}
-constexpr int PS_BAD = 32;   // byte of a stress block's shared memory: set once strain_bad was seen
-
 // mbarrier phase counters of a block, carried across its marches
 struct PairPhases {
     int v, s;   // v loads / cell-box loads issued (and waited) so far
@@ -584,7 +552,6 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
     };
     uint32_t lab_next = 0u;
     int *status = A.status;
-    volatile int *bad = reinterpret_cast<volatile int *>(smem + PS_BAD);
 
     if (tid == 0) {
         issue_v(q0);
@@ -610,7 +577,6 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
 #pragma unroll
             for (int J = 0; J < 6; ++J)
                 *reinterpret_cast<float2 *>(gs + (ring_base(J) + (ring_planes(J) == 4 ? s4 : r3)) * PS_GST + cg) = g[J];
-            if (!CM && A.fluid0 && strain_bad(g)) *bad = 1;
         }
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
@@ -631,9 +597,6 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
             if (q + 1 <= ze) issue_v(q + 1);
             if (q >= zb + 2 && q < ze) issue_s(q);   // plane z + 1, into the slot plane z - 1 used
         }
-        // the whole warp in the couplant (lanes with no cell to update have label 0)
-        const bool fluid = !CM && A.fluid0 && !*bad &&
-                           __all_sync(0xffffffffu, (lab2 & (LAB_MAT | (uint32_t)LAB_MAT << 16)) == 0u);
         if (z >= zb && any_out) {
             // strain planes z - 1, z, z + 1 were written at iterations i - 2, i - 1, i
             const int zr3 = r3 == 0 ? 2 : r3 - 1;   // plane z modulo 3
@@ -647,8 +610,6 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
                 const float *const cell = A.c21 + (long long)z * sz + col;
                 if (fast) stiff_all_cell<false>(pl, mg, cell, A.cplane, acc);
                 else stiff_all_cell<true>(pl, mg, cell, A.cplane, acc);
-            } else if (fluid) {
-                stiff_fluid(A, pl, acc);
             } else {
                 const float *const crow[2] = {tab + (lab[0] & LAB_MAT) * TAB36, tab + (lab[1] & LAB_MAT) * TAB36};
                 if (fast) stiff_all<false, TS>(pl, mg, crow, acc);
@@ -748,7 +709,6 @@ __device__ __forceinline__ void stress_pair_init(unsigned char *smem)
     float *gs = reinterpret_cast<float *>(smem + 128) + PS_VSLOT + 2 * PS_SSLOT;
     if (threadIdx.x == 0) {
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
-        *reinterpret_cast<int *>(smem + PS_BAD) = 0;
         fence_mbar_init();
     }
     // zero the strain planes' pads (read only by cells that are not updated)
@@ -947,10 +907,6 @@ __device__ __forceinline__ void pair_vel_taps(const StepArgs<float> &A, int z, c
         }
     }
 }
-
-// last interior velocity tile along x / y (pair_vtile_inside), or <= 0
-__host__ __device__ constexpr int pair_vlast_inside_x(int nx) { return nx < 36 ? 0 : (nx - 36) / PV_OX; }
-__host__ __device__ constexpr int pair_vlast_inside_y(int ny) { return ny < 20 ? 0 : (ny - 20) / PV_OY; }
 
 // Every x / y tap of velocity tile (bx, by), and every face-density
 // neighbour, lies inside the grid.
@@ -1228,8 +1184,8 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
     const float *rho_tab = rho_smem ? rsm : A.rho;
     const int zb = blockIdx.z * A.zc, ze = min(zb + A.zc, A.nz);
     int bx, by;
-    interior_first(pair_vlast_inside_x(A.nx), pair_vlast_inside_y(A.ny), gridDim.x, gridDim.y,
-                   blockIdx.x + gridDim.x * blockIdx.y, bx, by);
+    interior_first(A.nx < 36 ? 0 : (A.nx - 36) / PV_OX, A.ny < 20 ? 0 : (A.ny - 20) / PV_OY, gridDim.x,
+                   gridDim.y, blockIdx.x + gridDim.x * blockIdx.y, bx, by);
     if (pair_vtile_inside(A, bx, by))
         velocity_pair_march<NC, true, false, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
     else
@@ -1237,30 +1193,28 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
 }
 
 // ---------------------------------------------------------------- batches
-// Many solves (any grid sizes) advance one step per launch pair. The work of a
-// phase is a list of z-marches, cut so that every resident block has the same
-// load (the host weighs guarded tiles and march start-ups); block b walks
-// items off[b] to off[b + 1] - 1, re-staging a solve's arguments and tables
-// only when the solve changes.
+// Many solves (any grid sizes) advance one step per launch pair. Work items
+// (solve, tile x, tile y, z-chunk) are listed solve by solve and chunk-major
+// within a solve, so blocks that run together march the same planes of
+// neighbouring tiles; each resident block walks a contiguous run of items,
+// re-staging the solve's arguments and tables only when the solve changes.
 // All solves of a pair batch have rows of 16-byte multiples, their own or padded.
-struct PairItem {
-    int solve, bx, by, zb, ze;
-};
 template <int NC, bool TS>
 __global__ void __launch_bounds__(PS_N, 2)
     k_stress_pair_batch(const StepArgs<float> *__restrict__ descs, const TmapsPairStress *__restrict__ maps,
                         const float *const *__restrict__ tabs, const int *__restrict__ n_mats,
-                        const PairItem *__restrict__ items, const int *__restrict__ off, int k)
+                        const BatchItem *__restrict__ items, int n_items, int k)
 {
     extern __shared__ __align__(128) unsigned char smem_pair[];
     __shared__ __align__(16) StepArgs<float> As;
     float *tsm = reinterpret_cast<float *>(smem_pair + PS_SMEM_FIXED);
     stress_pair_init(smem_pair);
-    const int i0 = off[blockIdx.x], i1 = off[blockIdx.x + 1];
+    const int per = (n_items + gridDim.x - 1) / gridDim.x;
+    const int i0 = blockIdx.x * per, i1 = min(n_items, i0 + per);
     int cur = -1;
     PairPhases ph{0, 0};
     for (int it = i0; it < i1; ++it) {
-        const PairItem w = items[it];
+        const BatchItem w = items[it];
         __syncthreads();   // the previous march is finished by every thread
         const bool fresh = w.solve != cur;
         if (fresh) {
@@ -1268,7 +1222,7 @@ __global__ void __launch_bounds__(PS_N, 2)
             if (TS) stage_table(tsm, tabs[w.solve], n_mats[w.solve]);
         }
         __syncthreads();
-        const int zb = w.zb, ze = w.ze;
+        const int zb = w.bz * As.zc, ze = min(zb + As.zc, As.nz);
         const float *tab = TS ? tsm : tabs[w.solve];
         if (pair_tile_inside(As, w.bx, w.by))
             stress_pair_march<NC, TS, true>(maps[w.solve], As, tab, smem_pair, w.bx, w.by, zb, ze, ph);
@@ -1281,8 +1235,8 @@ __global__ void __launch_bounds__(PS_N, 2)
 template <int NC>
 __global__ void __launch_bounds__(PV_N, 2)
     k_velocity_pair_batch(const StepArgs<float> *__restrict__ descs, const TmapsPairVelocity *__restrict__ maps,
-                          const int *__restrict__ n_mats, const PairItem *__restrict__ items,
-                          const int *__restrict__ off, int k)
+                          const int *__restrict__ n_mats, const BatchItem *__restrict__ items, int n_items,
+                          int k)
 {
     extern __shared__ __align__(128) unsigned char smem_pair[];
     __shared__ __align__(16) StepArgs<float> As;
@@ -1292,10 +1246,11 @@ __global__ void __launch_bounds__(PV_N, 2)
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
         fence_mbar_init();
     }
-    const int i0 = off[blockIdx.x], i1 = off[blockIdx.x + 1];
+    const int per = (n_items + gridDim.x - 1) / gridDim.x;
+    const int i0 = blockIdx.x * per, i1 = min(n_items, i0 + per);
     int cur = -1, it0 = 0;
     for (int it = i0; it < i1; ++it) {
-        const PairItem w = items[it];
+        const BatchItem w = items[it];
         __syncthreads();
         const bool fresh = w.solve != cur;
         if (fresh) {
@@ -1303,7 +1258,7 @@ __global__ void __launch_bounds__(PV_N, 2)
             for (int i = threadIdx.x; i < n_mats[w.solve]; i += PV_N) rsm[i] = As.rho[i];
         }
         __syncthreads();
-        const int zb = w.zb, ze = w.ze;
+        const int zb = w.bz * As.zc, ze = min(zb + As.zc, As.nz);
         if (pair_vtile_inside(As, w.bx, w.by))
             it0 += velocity_pair_march<NC, true>(maps[w.solve], As, rsm, smem_pair, w.bx, w.by, zb, ze, it0);
         else
@@ -1372,9 +1327,8 @@ template <int NC, bool TS>
 __global__ void __launch_bounds__(PS_N, 2)
     k_pair_batch_persistent(const StepArgs<float> *__restrict__ descs, const TmapsPairStress *__restrict__ smaps,
                             const TmapsPairVelocity *__restrict__ vmaps, const float *const *__restrict__ tabs,
-                            const int *__restrict__ n_mats, const PairItem *__restrict__ items_s,
-                            const int *__restrict__ off_s, const PairItem *__restrict__ items_v,
-                            const int *__restrict__ off_v, int nk, unsigned *bar, int *status)
+                            const int *__restrict__ n_mats, const BatchItem *__restrict__ items_s, int n_s,
+                            const BatchItem *__restrict__ items_v, int n_v, int nk, unsigned *bar, int *status)
 {
     extern __shared__ __align__(128) unsigned char smem_pair[];
     __shared__ __align__(16) StepArgs<float> As;
@@ -1387,22 +1341,22 @@ __global__ void __launch_bounds__(PS_N, 2)
         fence_mbar_init();
     }
     __syncthreads();
-    const int i0s = off_s[blockIdx.x], i1s = off_s[blockIdx.x + 1];
-    const int i0v = off_v[blockIdx.x], i1v = off_v[blockIdx.x + 1];
+    const int per_s = (n_s + gridDim.x - 1) / gridDim.x, i0s = blockIdx.x * per_s, i1s = min(n_s, i0s + per_s);
+    const int per_v = (n_v + gridDim.x - 1) / gridDim.x, i0v = blockIdx.x * per_v, i1v = min(n_v, i0v + per_v);
     PairPhases ph{0, 0};
     int it0 = 0;
     unsigned nbar = 0;
     for (int k = 0; k < nk; ++k) {
         int cur = -1;
         for (int it = i0s; it < i1s; ++it) {
-            const PairItem w = items_s[it];
+            const BatchItem w = items_s[it];
             __syncthreads();   // the previous march is finished by every thread
             if (w.solve != cur) {
                 copy_args(&As, descs + w.solve, k);
                 if (TS) stage_table(tsm, tabs[w.solve], n_mats[w.solve]);
             }
             __syncthreads();
-            const int zb = w.zb, ze = w.ze;
+            const int zb = w.bz * As.zc, ze = min(zb + As.zc, As.nz);
             const float *tab = TS ? tsm : tabs[w.solve];
             if (pair_tile_inside(As, w.bx, w.by))
                 stress_pair_march<NC, TS, true, true>(smaps[w.solve], As, tab, smem_pair, w.bx, w.by, zb, ze, ph);
@@ -1413,14 +1367,14 @@ __global__ void __launch_bounds__(PS_N, 2)
         grid_barrier(bar, ++nbar * gridDim.x, status);
         cur = -1;
         for (int it = i0v; it < i1v; ++it) {
-            const PairItem w = items_v[it];
+            const BatchItem w = items_v[it];
             __syncthreads();
             if (w.solve != cur) {
                 copy_args(&As, descs + w.solve, k);
                 for (int i = threadIdx.x; i < n_mats[w.solve]; i += PV_N) rsm[i] = As.rho[i];
             }
             __syncthreads();
-            const int zb = w.zb, ze = w.ze;
+            const int zb = w.bz * As.zc, ze = min(zb + As.zc, As.nz);
             if (pair_vtile_inside(As, w.bx, w.by))
                 it0 += velocity_pair_march<NC, true, true>(vmaps[w.solve], As, rsm, smem_pair, w.bx, w.by, zb, ze,
                                                            it0, vbars);
