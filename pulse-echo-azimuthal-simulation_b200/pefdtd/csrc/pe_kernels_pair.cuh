@@ -168,7 +168,9 @@ __device__ __forceinline__ float2 ldg2_stream(const float *p)
 __device__ __forceinline__ float2 ldcg2(const float *p)
 {
     float2 v;
-    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+    // volatile keeps it behind the grid barrier's asm; without a memory clobber
+    // the arithmetic around it stays free to move
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "l"(p));
     return v;
 }
 template <bool COH>
@@ -908,6 +910,10 @@ __device__ __forceinline__ void pair_vel_taps(const StepArgs<float> &A, int z, c
     }
 }
 
+// last interior velocity tile along x / y (pair_vtile_inside), or <= 0
+__host__ __device__ constexpr int pair_vlast_inside_x(int nx) { return nx < 36 ? 0 : (nx - 36) / PV_OX; }
+__host__ __device__ constexpr int pair_vlast_inside_y(int ny) { return ny < 20 ? 0 : (ny - 20) / PV_OY; }
+
 // Every x / y tap of velocity tile (bx, by), and every face-density
 // neighbour, lies inside the grid.
 __device__ __forceinline__ bool pair_vtile_inside(const StepArgs<float> &A, int bx, int by)
@@ -1184,8 +1190,8 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
     const float *rho_tab = rho_smem ? rsm : A.rho;
     const int zb = blockIdx.z * A.zc, ze = min(zb + A.zc, A.nz);
     int bx, by;
-    interior_first(A.nx < 36 ? 0 : (A.nx - 36) / PV_OX, A.ny < 20 ? 0 : (A.ny - 20) / PV_OY, gridDim.x,
-                   gridDim.y, blockIdx.x + gridDim.x * blockIdx.y, bx, by);
+    interior_first(pair_vlast_inside_x(A.nx), pair_vlast_inside_y(A.ny), gridDim.x, gridDim.y,
+                   blockIdx.x + gridDim.x * blockIdx.y, bx, by);
     if (pair_vtile_inside(A, bx, by))
         velocity_pair_march<NC, true, false, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
     else
@@ -1193,28 +1199,30 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
 }
 
 // ---------------------------------------------------------------- batches
-// Many solves (any grid sizes) advance one step per launch pair. Work items
-// (solve, tile x, tile y, z-chunk) are listed solve by solve and chunk-major
-// within a solve, so blocks that run together march the same planes of
-// neighbouring tiles; each resident block walks a contiguous run of items,
-// re-staging the solve's arguments and tables only when the solve changes.
+// Many solves (any grid sizes) advance one step per launch pair. The work of a
+// phase is a list of z-marches, cut so that every resident block has the same
+// load (the host weighs guarded tiles and march start-ups); block b walks
+// items off[b] to off[b + 1] - 1, re-staging a solve's arguments and tables
+// only when the solve changes.
 // All solves of a pair batch have rows of 16-byte multiples, their own or padded.
+struct PairItem {
+    int solve, bx, by, zb, ze;
+};
 template <int NC, bool TS>
 __global__ void __launch_bounds__(PS_N, 2)
     k_stress_pair_batch(const StepArgs<float> *__restrict__ descs, const TmapsPairStress *__restrict__ maps,
                         const float *const *__restrict__ tabs, const int *__restrict__ n_mats,
-                        const BatchItem *__restrict__ items, int n_items, int k)
+                        const PairItem *__restrict__ items, const int *__restrict__ off, int k)
 {
     extern __shared__ __align__(128) unsigned char smem_pair[];
     __shared__ __align__(16) StepArgs<float> As;
     float *tsm = reinterpret_cast<float *>(smem_pair + PS_SMEM_FIXED);
     stress_pair_init(smem_pair);
-    const int per = (n_items + gridDim.x - 1) / gridDim.x;
-    const int i0 = blockIdx.x * per, i1 = min(n_items, i0 + per);
+    const int i0 = off[blockIdx.x], i1 = off[blockIdx.x + 1];
     int cur = -1;
     PairPhases ph{0, 0};
     for (int it = i0; it < i1; ++it) {
-        const BatchItem w = items[it];
+        const PairItem w = items[it];
         __syncthreads();   // the previous march is finished by every thread
         const bool fresh = w.solve != cur;
         if (fresh) {
@@ -1222,7 +1230,7 @@ __global__ void __launch_bounds__(PS_N, 2)
             if (TS) stage_table(tsm, tabs[w.solve], n_mats[w.solve]);
         }
         __syncthreads();
-        const int zb = w.bz * As.zc, ze = min(zb + As.zc, As.nz);
+        const int zb = w.zb, ze = w.ze;
         const float *tab = TS ? tsm : tabs[w.solve];
         if (pair_tile_inside(As, w.bx, w.by))
             stress_pair_march<NC, TS, true>(maps[w.solve], As, tab, smem_pair, w.bx, w.by, zb, ze, ph);
@@ -1235,8 +1243,8 @@ __global__ void __launch_bounds__(PS_N, 2)
 template <int NC>
 __global__ void __launch_bounds__(PV_N, 2)
     k_velocity_pair_batch(const StepArgs<float> *__restrict__ descs, const TmapsPairVelocity *__restrict__ maps,
-                          const int *__restrict__ n_mats, const BatchItem *__restrict__ items, int n_items,
-                          int k)
+                          const int *__restrict__ n_mats, const PairItem *__restrict__ items,
+                          const int *__restrict__ off, int k)
 {
     extern __shared__ __align__(128) unsigned char smem_pair[];
     __shared__ __align__(16) StepArgs<float> As;
@@ -1246,11 +1254,10 @@ __global__ void __launch_bounds__(PV_N, 2)
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
         fence_mbar_init();
     }
-    const int per = (n_items + gridDim.x - 1) / gridDim.x;
-    const int i0 = blockIdx.x * per, i1 = min(n_items, i0 + per);
+    const int i0 = off[blockIdx.x], i1 = off[blockIdx.x + 1];
     int cur = -1, it0 = 0;
     for (int it = i0; it < i1; ++it) {
-        const BatchItem w = items[it];
+        const PairItem w = items[it];
         __syncthreads();
         const bool fresh = w.solve != cur;
         if (fresh) {
@@ -1258,7 +1265,7 @@ __global__ void __launch_bounds__(PV_N, 2)
             for (int i = threadIdx.x; i < n_mats[w.solve]; i += PV_N) rsm[i] = As.rho[i];
         }
         __syncthreads();
-        const int zb = w.bz * As.zc, ze = min(zb + As.zc, As.nz);
+        const int zb = w.zb, ze = w.ze;
         if (pair_vtile_inside(As, w.bx, w.by))
             it0 += velocity_pair_march<NC, true>(maps[w.solve], As, rsm, smem_pair, w.bx, w.by, zb, ze, it0);
         else
@@ -1327,8 +1334,9 @@ template <int NC, bool TS>
 __global__ void __launch_bounds__(PS_N, 2)
     k_pair_batch_persistent(const StepArgs<float> *__restrict__ descs, const TmapsPairStress *__restrict__ smaps,
                             const TmapsPairVelocity *__restrict__ vmaps, const float *const *__restrict__ tabs,
-                            const int *__restrict__ n_mats, const BatchItem *__restrict__ items_s, int n_s,
-                            const BatchItem *__restrict__ items_v, int n_v, int nk, unsigned *bar, int *status)
+                            const int *__restrict__ n_mats, const PairItem *__restrict__ items_s,
+                            const int *__restrict__ off_s, const PairItem *__restrict__ items_v,
+                            const int *__restrict__ off_v, int nk, unsigned *bar, int *status)
 {
     extern __shared__ __align__(128) unsigned char smem_pair[];
     __shared__ __align__(16) StepArgs<float> As;
@@ -1341,22 +1349,22 @@ __global__ void __launch_bounds__(PS_N, 2)
         fence_mbar_init();
     }
     __syncthreads();
-    const int per_s = (n_s + gridDim.x - 1) / gridDim.x, i0s = blockIdx.x * per_s, i1s = min(n_s, i0s + per_s);
-    const int per_v = (n_v + gridDim.x - 1) / gridDim.x, i0v = blockIdx.x * per_v, i1v = min(n_v, i0v + per_v);
+    const int i0s = off_s[blockIdx.x], i1s = off_s[blockIdx.x + 1];
+    const int i0v = off_v[blockIdx.x], i1v = off_v[blockIdx.x + 1];
     PairPhases ph{0, 0};
     int it0 = 0;
     unsigned nbar = 0;
     for (int k = 0; k < nk; ++k) {
         int cur = -1;
         for (int it = i0s; it < i1s; ++it) {
-            const BatchItem w = items_s[it];
+            const PairItem w = items_s[it];
             __syncthreads();   // the previous march is finished by every thread
             if (w.solve != cur) {
                 copy_args(&As, descs + w.solve, k);
                 if (TS) stage_table(tsm, tabs[w.solve], n_mats[w.solve]);
             }
             __syncthreads();
-            const int zb = w.bz * As.zc, ze = min(zb + As.zc, As.nz);
+            const int zb = w.zb, ze = w.ze;
             const float *tab = TS ? tsm : tabs[w.solve];
             if (pair_tile_inside(As, w.bx, w.by))
                 stress_pair_march<NC, TS, true, true>(smaps[w.solve], As, tab, smem_pair, w.bx, w.by, zb, ze, ph);
@@ -1367,14 +1375,14 @@ __global__ void __launch_bounds__(PS_N, 2)
         grid_barrier(bar, ++nbar * gridDim.x, status);
         cur = -1;
         for (int it = i0v; it < i1v; ++it) {
-            const BatchItem w = items_v[it];
+            const PairItem w = items_v[it];
             __syncthreads();
             if (w.solve != cur) {
                 copy_args(&As, descs + w.solve, k);
                 for (int i = threadIdx.x; i < n_mats[w.solve]; i += PV_N) rsm[i] = As.rho[i];
             }
             __syncthreads();
-            const int zb = w.bz * As.zc, ze = min(zb + As.zc, As.nz);
+            const int zb = w.zb, ze = w.ze;
             if (pair_vtile_inside(As, w.bx, w.by))
                 it0 += velocity_pair_march<NC, true, true>(vmaps[w.solve], As, rsm, smem_pair, w.bx, w.by, zb, ze,
                                                            it0, vbars);

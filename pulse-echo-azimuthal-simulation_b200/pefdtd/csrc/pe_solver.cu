@@ -1359,10 +1359,14 @@ struct PeBatch {
     int *nmats = nullptr;
     pe::BatchItem *items_s = nullptr, *items_v = nullptr;
     int n_items_s = 0, n_items_v = 0;
-    // padded solves' items come last in the lists, for the persistent launches:
-    // per-step launches and short runs, which step the callers' states in
-    // place, leave them out (batched(), items_in_use())
-    int n_inplace_s = 0, n_inplace_v = 0;
+    // pair batches: the marches of a phase and each block's share of them, for
+    // the solves stepped in place, and with the padded solves too, which share
+    // the persistent launches (pad_shared())
+    struct PairWork {
+        pe::PairItem *items = nullptr;
+        int *off = nullptr;
+        int grid = 0;
+    } work_s[2], work_v[2];
     bool pad_on = false;            // this run goes through the padded states
     int grid_s = 1, grid_v = 1;
     size_t smem_s = 0, smem_v = 0;
@@ -1386,7 +1390,6 @@ struct PeBatch {
     // of the batched pair solves (k_pair_batch_persistent)
     bool persistent = false;
     unsigned *bar = nullptr;        // grid barrier counter, zeroed before each launch
-    int grid_p = 1;
     size_t smem_p = 0;
 
     ~PeBatch()
@@ -1397,9 +1400,19 @@ struct PeBatch {
         void *bufs[] = {step, status, descs, maps_s, maps_v, nmats, items_s, items_v, pmaps_s, pmaps_v, tabs, bar};
         for (void *b : bufs)
             if (b) dev_free(b);
+        drop_pair_work();
         if (ev_in) cudaEventDestroy(ev_in);
         if (ev_out) cudaEventDestroy(ev_out);
         if (stream) cudaStreamDestroy(stream);
+    }
+
+    void drop_pair_work()
+    {
+        for (PairWork *w : {&work_s[0], &work_s[1], &work_v[0], &work_v[1]}) {
+            dev_free(w->items);
+            dev_free(w->off);
+            *w = PairWork();
+        }
     }
 };
 
@@ -1415,15 +1428,94 @@ bool batched(const PeBatch *B, const PeSolver *S)
     return B->pair_batch ? ((S->pair_capable || (S->padded && pad_shared(B))) && !S->solo)
                          : (B->tma_batch && S->tma_capable);
 }
-void items_in_use(const PeBatch *B, int *n_s, int *n_v)
+
+// Cut the marches of one phase (stress or velocity tiles of the solves taken)
+// into `grid` shares of equal load. With a z-chunk asked for (zc_of(S) > 0)
+// columns are cut there and dealt out in order; else they are cut wherever a
+// share is full, at marches of four planes and more. Load in planes of an
+// interior tile: a guarded tile's plane costs 1.25, a march's start-up 2 planes
+// (stress) or 1 (velocity). Against 40-plane chunks dealt in equal counts, 12
+// solves of 64x96x96 (672 items on 296 blocks: three for some, none for
+// others): 200 steps 106 -> 89 ms.
+struct PairShares {
+    std::vector<pe::PairItem> items;
+    std::vector<int> off;
+};
+PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int grid)
 {
-    *n_s = pad_shared(B) ? B->n_items_s : B->n_inplace_s;
-    *n_v = pad_shared(B) ? B->n_items_v : B->n_inplace_v;
+    struct Col {
+        int solve, bx, by, nz, zc;
+        double w;
+    };
+    std::vector<Col> cols;
+    bool chunked = false;
+    for (int s = 0; s < (int)B->solves.size(); ++s) {
+        const PeSolver *S = B->solves[s];
+        if (S->solo || !(S->pair_capable || (with_padded && S->padded))) continue;
+        const PeConfig &c = S->cfg;
+        const int tx = stress ? (c.nx + pe::PS_OX) / pe::PS_OX : (c.nx + pe::PV_OX - 1) / pe::PV_OX;
+        const int ty = stress ? (c.ny + pe::PS_OY - 1) / pe::PS_OY : (c.ny + pe::PV_OY - 1) / pe::PV_OY;
+        const int hx = stress ? pe::pair_last_inside_x(c.nx) : pe::pair_vlast_inside_x(c.nx);
+        const int hy = stress ? pe::pair_last_inside_y(c.ny) : pe::pair_vlast_inside_y(c.ny);
+        const int zc = c.z_chunk > 0 || B->z_chunk > 0 ? S->zc_s : 0;
+        chunked = chunked || zc > 0;
+        for (int by = 0; by < ty; ++by)
+            for (int bx = 0; bx < tx; ++bx)
+                cols.push_back({s, bx, by, c.nz, zc, bx >= 1 && bx <= hx && by >= 1 && by <= hy ? 1.0 : 1.25});
+    }
+    PairShares P;
+    if (chunked) {   // chunk by chunk within a solve: neighbouring tiles march the same planes together
+        for (size_t i = 0; i < cols.size();) {
+            size_t j = i;
+            while (j < cols.size() && cols[j].solve == cols[i].solve) ++j;
+            const int zc = cols[i].zc > 0 ? cols[i].zc : cols[i].nz;
+            for (int z = 0; z < cols[i].nz; z += zc)
+                for (size_t k = i; k < j; ++k)
+                    P.items.push_back({cols[k].solve, cols[k].bx, cols[k].by, z, std::min(cols[k].nz, z + zc)});
+            i = j;
+        }
+        const int n = (int)P.items.size(), per = std::max(1, (n + grid - 1) / grid);
+        for (int g = 0; g <= grid; ++g) P.off.push_back(std::min(n, g * per));
+        return P;
+    }
+    const double startup = stress ? 2.0 : 1.0;
+    auto cut = [&](double T, PairShares *out) {   // shares used at load T each
+        int used = 1;
+        double load = 0.0;
+        if (out) out->off.push_back(0);
+        for (const Col &c : cols)
+            for (int z = 0; z < c.nz;) {
+                int n = (int)((T - load) / c.w - startup);
+                if (n < std::min(4, c.nz - z)) {
+                    if (load > 0.0) {   // this share is full
+                        ++used;
+                        load = 0.0;
+                        if (out) out->off.push_back((int)out->items.size());
+                        continue;
+                    }
+                    n = std::min(4, c.nz - z);
+                }
+                n = std::min(n, c.nz - z);
+                if (c.nz - z - n < 4 && c.nz - z - n > 0) n = std::max(std::min(4, c.nz - z), c.nz - z - 4);
+                if (out) out->items.push_back({c.solve, c.bx, c.by, z, z + n});
+                load += c.w * (n + startup);
+                z += n;
+            }
+        return used;
+    };
+    double lo = 0.0, hi = 1.0;
+    for (const Col &c : cols) hi += c.w * (c.nz + startup);
+    for (int it = 0; it < 50; ++it) {
+        const double mid = 0.5 * (lo + hi);
+        (cut(mid, nullptr) <= grid ? hi : lo) = mid;
+    }
+    cut(hi, &P);
+    while ((int)P.off.size() <= grid) P.off.push_back((int)P.items.size());
+    return P;
 }
 
 // Pair-kernel layout of an FP32 batch: work items, grids and shared memory.
-int batch_layout_pair(PeBatch *B, int nsm, int optin, std::vector<pe::BatchItem> &is,
-                      std::vector<pe::BatchItem> &iv)
+int batch_layout_pair(PeBatch *B, int nsm, int optin)
 {
     int max_mat = 1;
     B->pair_nc4 = true;
@@ -1467,35 +1559,28 @@ int batch_layout_pair(PeBatch *B, int nsm, int optin, std::vector<pe::BatchItem>
     PE_CUDA(setattr((const void *)pe::k_pair_batch_persistent<0, true>));
     PE_CUDA(setattr((const void *)pe::k_pair_batch_persistent<0, false>));
     B->smem_p = pe::persistent_pair_smem(B->smem_s, B->smem_v);
-    for (int pass = 0; pass < 2; ++pass) {   // solves stepped in place, then padded ones
-        for (int s = 0; s < (int)B->solves.size(); ++s) {
-            PeSolver *S = B->solves[s];
-            if (S->solo || !(pass ? S->padded : S->pair_capable)) continue;
-            const PeConfig &c = S->cfg;
-            const int zc = S->zc_s;
-            const int nzc = (c.nz + zc - 1) / zc;
-            for (int bz = 0; bz < nzc; ++bz) {
-                for (int by = 0; by < (c.ny + pe::PS_OY - 1) / pe::PS_OY; ++by)
-                    for (int bx = 0; bx < (c.nx + pe::PS_OX) / pe::PS_OX; ++bx) is.push_back({s, bx, by, bz});
-                for (int by = 0; by < (c.ny + pe::PV_OY - 1) / pe::PV_OY; ++by)
-                    for (int bx = 0; bx < (c.nx + pe::PV_OX - 1) / pe::PV_OX; ++bx) iv.push_back({s, bx, by, bz});
-            }
-        }
-        if (!pass) {
-            B->n_inplace_s = (int)is.size();
-            B->n_inplace_v = (int)iv.size();
-        }
-    }
     int per_v = 1, per_s = 1, per_p = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_v, pe::k_velocity_pair_batch<4>, pe::PV_N, B->smem_v);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_s, pe::k_stress_pair_batch<4, true>, pe::PS_N, B->smem_s);
-    B->grid_s = std::max(1, std::min((int)is.size(), nsm * std::max(1, per_s)));
-    B->grid_v = std::max(1, std::min((int)iv.size(), nsm * std::max(1, per_v)));
     // the persistent kernel's blocks must all be resident at once (its grid
-    // barriers wait for every block): at most the occupancy times the SMs
+    // barriers wait for every block): at most the occupancy times the SMs. All
+    // three kernels share the cuts, so they take the smallest of the three.
     PE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_p, pe::k_pair_batch_persistent<4, true>, pe::PS_N,
                                                           B->smem_p));
-    B->grid_p = std::max(1, std::min((int)std::max(is.size(), iv.size()), nsm * std::max(1, per_p)));
+    const int grid = nsm * std::max(1, std::min(per_p, std::min(per_s, per_v)));
+    B->drop_pair_work();
+    for (int k = 0; k < 2; ++k)
+        for (int stress = 0; stress < 2; ++stress) {
+            const PairShares P = cut_pair_work(B, stress != 0, k == 1, grid);
+            PeBatch::PairWork &W = stress ? B->work_s[k] : B->work_v[k];
+            if (P.items.empty()) continue;
+            int rc;
+            if ((rc = dev_alloc(&W.items, sizeof(pe::PairItem) * P.items.size()))) return rc;
+            if ((rc = dev_alloc(&W.off, sizeof(int) * P.off.size()))) return rc;
+            PE_CUDA(cudaMemcpy(W.items, P.items.data(), sizeof(pe::PairItem) * P.items.size(), cudaMemcpyHostToDevice));
+            PE_CUDA(cudaMemcpy(W.off, P.off.data(), sizeof(int) * P.off.size(), cudaMemcpyHostToDevice));
+            W.grid = grid;
+        }
     return PE_OK;
 }
 
@@ -1523,11 +1608,9 @@ int batch_layout(PeBatch *B)
         for (PeSolver *S : B->solves) any = any || S->pair_capable || S->padded;
         if (any) {
             B->pair_batch = true;
-            int rc0 = batch_layout_pair(B, nsm, optin, is, iv);
+            int rc0 = batch_layout_pair(B, nsm, optin);
             if (rc0 == PE_ERR_UNSUPPORTED) {
                 B->pair_batch = false;
-                is.clear();
-                iv.clear();
             } else if (rc0) {
                 return rc0;
             }
@@ -1567,10 +1650,6 @@ int batch_layout(PeBatch *B)
     }
     B->n_items_s = (int)is.size();
     B->n_items_v = (int)iv.size();
-    if (!B->pair_batch) {
-        B->n_inplace_s = B->n_items_s;
-        B->n_inplace_v = B->n_items_v;
-    }
     if (B->items_s) dev_free(B->items_s);
     if (B->items_v) dev_free(B->items_v);
     B->items_s = B->items_v = nullptr;
@@ -1638,7 +1717,8 @@ int launch_pair_persistent(PeBatch *B, int len)
 {
     PE_CUDA(cudaMemsetAsync(B->bar, 0, sizeof(unsigned), B->stream));
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)B->grid_p, 1, 1);
+    const PeBatch::PairWork &ws = B->work_s[pad_shared(B)], &wv = B->work_v[pad_shared(B)];
+    lc.gridDim = dim3((unsigned)ws.grid, 1, 1);
     lc.blockDim = dim3(pe::PS_N, 1, 1);
     lc.dynamicSmemBytes = B->smem_p;
     lc.stream = B->stream;
@@ -1651,19 +1731,17 @@ int launch_pair_persistent(PeBatch *B, int len)
     const float *const *tabs = B->tabs;
     const pe::TmapsPairStress *ms = B->pmaps_s;
     const pe::TmapsPairVelocity *mv = B->pmaps_v;
-    const int *nm = B->nmats;
-    const pe::BatchItem *is = B->items_s, *iv = B->items_v;
-    int ns, nv;
-    items_in_use(B, &ns, &nv);
+    const int *nm = B->nmats, *os = ws.off, *ov = wv.off;
+    const pe::PairItem *is = ws.items, *iv = wv.items;
     cudaError_t e;
     if (B->pair_nc4 && B->pair_ts)
-        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, true>, d, ms, mv, tabs, nm, is, ns, iv, nv, len, B->bar, B->status);
+        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, true>, d, ms, mv, tabs, nm, is, os, iv, ov, len, B->bar, B->status);
     else if (B->pair_nc4)
-        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, false>, d, ms, mv, tabs, nm, is, ns, iv, nv, len, B->bar, B->status);
+        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, false>, d, ms, mv, tabs, nm, is, os, iv, ov, len, B->bar, B->status);
     else if (B->pair_ts)
-        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<0, true>, d, ms, mv, tabs, nm, is, ns, iv, nv, len, B->bar, B->status);
+        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<0, true>, d, ms, mv, tabs, nm, is, os, iv, ov, len, B->bar, B->status);
     else
-        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<0, false>, d, ms, mv, tabs, nm, is, ns, iv, nv, len, B->bar, B->status);
+        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<0, false>, d, ms, mv, tabs, nm, is, os, iv, ov, len, B->bar, B->status);
     if (e != cudaSuccess) return fail(PE_ERR_CUDA, std::string("persistent batch launch: ") + cudaGetErrorString(e));
     B->launches += 1;
     return PE_OK;
@@ -1673,31 +1751,29 @@ template <typename T>
 int batch_chunk(PeBatch *B, int len)
 {
     const dim3 block(pe::TB_X, pe::TB_Y, 1);
-    int n_s, n_v;
-    items_in_use(B, &n_s, &n_v);
+    const PeBatch::PairWork &ws = B->work_s[pad_shared(B)], &wv = B->work_v[pad_shared(B)];
     if constexpr (std::is_same<T, float>::value) {
-        if (B->pair_batch && B->persistent && n_s > 0) {
+        if (B->pair_batch && B->persistent && ws.grid > 0) {
             const int rc = launch_pair_persistent(B, len);
             if (rc) return rc;
         }
     }
     for (int k = 0; k < len; ++k) {
         if constexpr (std::is_same<T, float>::value) {
-            if (B->pair_batch && !B->persistent && n_s > 0) {
+            if (B->pair_batch && !B->persistent && ws.grid > 0) {
                 const pe::StepArgs<float> *d = (const pe::StepArgs<float> *)B->descs;
-                const int ns = n_s, nv = n_v;
                 if (B->pair_nc4 && B->pair_ts)
-                    pe::k_stress_pair_batch<4, true><<<B->grid_s, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, B->items_s, ns, k);
+                    pe::k_stress_pair_batch<4, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
                 else if (B->pair_nc4)
-                    pe::k_stress_pair_batch<4, false><<<B->grid_s, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, B->items_s, ns, k);
+                    pe::k_stress_pair_batch<4, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
                 else if (B->pair_ts)
-                    pe::k_stress_pair_batch<0, true><<<B->grid_s, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, B->items_s, ns, k);
+                    pe::k_stress_pair_batch<0, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
                 else
-                    pe::k_stress_pair_batch<0, false><<<B->grid_s, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, B->items_s, ns, k);
+                    pe::k_stress_pair_batch<0, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
                 if (B->pair_nc4)
-                    pe::k_velocity_pair_batch<4><<<B->grid_v, pe::PV_N, B->smem_v, B->stream>>>(d, B->pmaps_v, B->nmats, B->items_v, nv, k);
+                    pe::k_velocity_pair_batch<4><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, B->pmaps_v, B->nmats, wv.items, wv.off, k);
                 else
-                    pe::k_velocity_pair_batch<0><<<B->grid_v, pe::PV_N, B->smem_v, B->stream>>>(d, B->pmaps_v, B->nmats, B->items_v, nv, k);
+                    pe::k_velocity_pair_batch<0><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, B->pmaps_v, B->nmats, wv.items, wv.off, k);
                 B->launches += 2;
             }
         }
