@@ -404,16 +404,16 @@ bool same_state(const PeState &a, const PeState &b)
 // time of a launch, in planes marched at the full-SM rate: (planes per chunk +
 // start-up planes) x waves, a wave being one block on every slot. Kernels with
 // one block per SM run their waves in step, so waves count whole. With two per
-// SM, a launch that leaves every SM at most one block runs its planes in 0.7
+// SM, a launch that leaves every SM at most one block runs its planes in 0.8
 // of the time (measured 1.75 us a plane alone and 2.65 with two blocks per SM
 // for the stress kernel, 1.55 and 1.95 for the velocity kernel); one that fits
-// one wave waits for its slowest, guarded, blocks (1.15); beyond that the
-// blocks drift apart and the tail costs about half a wave, not a whole one.
-// Against whole waves throughout (which preferred one full wave): velocity
-// kernel on 96x160x160 56 -> 51 us (20 -> 8 planes), on 20x24x28 14.5 -> 12.5
-// us (4 -> 2 planes). A shorter march must be worth 2 %: longer ones re-read
-// less of the z halo.
-int pick_zchunk(int nz, long long tiles, int slots, int startup)
+// one wave waits for its slowest, guarded, blocks (`one_wave`: 1.15 stress,
+// 1.3 velocity); beyond that the blocks drift apart, and the tail costs
+// between the fraction and the whole of a wave. Against whole waves throughout
+// (which preferred one full wave): velocity kernel on 96x160x160 59 -> 54 us
+// (20 -> 8 planes), on 20x24x28 14.5 -> 12.5 us (4 -> 2 planes). A shorter
+// march must be worth 2 %: longer ones re-read less of the z halo.
+int pick_zchunk(int nz, long long tiles, int slots, int startup, double one_wave = 1.0)
 {
     int nsm = 148, dev = 0;
     cudaGetDevice(&dev);
@@ -424,7 +424,11 @@ int pick_zchunk(int nz, long long tiles, int slots, int startup)
         const int zc = (nz + nch - 1) / nch;
         const long long blocks = tiles * ((nz + zc - 1) / zc);
         double waves = (double)((blocks + slots - 1) / slots);
-        if (slots > nsm) waves = blocks <= nsm ? 0.7 : (blocks <= slots ? 1.15 : (double)blocks / slots + 0.5);
+        if (slots > nsm) {
+            if (blocks <= nsm) waves = 0.8;
+            else if (blocks <= slots) waves = one_wave;
+            else waves = 0.5 * (waves + (double)blocks / slots + 0.5);
+        }
         const double cost = waves * (zc + startup);
         if (cost < 0.98 * best) {
             best = cost;
@@ -509,8 +513,8 @@ int configure_pair(PeSolver *S, int optin)
     const long long tpv = (long long)((c.nx + pe::PV_OX - 1) / pe::PV_OX) * ((c.ny + pe::PV_OY - 1) / pe::PV_OY);
     const int sps = occupancy_slots(pe::k_stress_pair<4, true>, pe::PS_N, ps);
     const int spv = occupancy_slots(pe::k_velocity_pair<4>, pe::PV_N, pv);
-    S->zc_ps = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tps, sps, 3);
-    S->zc_pv = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tpv, spv, 1);
+    S->zc_ps = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tps, sps, 3, 1.15);
+    S->zc_pv = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tpv, spv, 1, 1.3);
     return PE_OK;
 }
 
