@@ -71,6 +71,10 @@ struct StepArgs {
     int dense;
     int cpitch;
     long long cplane;
+    // material 0 has no shear constants (the couplant): its normal block, rows
+    // then columns (pair kernels)
+    int fluid0;
+    T cfl[9];
 };
 
 // ---------------------------------------------------------------- helpers

@@ -416,6 +416,36 @@ __device__ __forceinline__ void stiff_all(const float *const (&pl)[4], const Mov
     stiff_column<5, G, TS>(pl, mg, crow, acc);
 }
 
+// The stiffness product of a warp whose cells are all material 0, the fluid
+// couplant (every constant outside the normal block exactly zero, see
+// StepArgs::fluid0): the full product's moved strains only meet zeros there,
+// and fma(0, q, acc) == acc bit for bit for finite q, so the product is nine
+// paired FMAs on three strains. A third to a half of a disk problem's cells
+// are couplant (all of its edge tiles' corners, the planes above and below the
+// disk). The caller has established that every strain of the block so far is
+// finite and small enough for the moves' sums (strain_bad).
+__device__ __forceinline__ void stiff_fluid(const StepArgs<float> &A, const float *const (&pl)[4], float2 (&acc)[6])
+{
+#pragma unroll
+    for (int I = 0; I < 6; ++I) acc[I] = bc2(0.f);
+#pragma unroll
+    for (int J = 0; J < 3; ++J) {
+        const float2 q = lds2(gptr(pl, J, 0, 0));
+#pragma unroll
+        for (int I = 0; I < 3; ++I) acc[I] = fmac2(acc[I], bc2(A.cfl[3 * I + J]), q);
+    }
+}
+// a strain that is not finite, or above 1e19, where a move's sum of four and
+// the square below are still far from overflow
+__device__ __forceinline__ bool strain_bad(const float2 (&g)[6])
+{
+    float2 t = mul2(g[0], g[0]);
+#pragma unroll
+    for (int J = 1; J < 6; ++J) t = fmac2(t, g[J], g[J]);
+    return !(t.x + t.y < 3.0e38f);
+}
+constexpr int PS_BAD = 32;   // byte of a stress block's shared memory: set once strain_bad was seen
+
 // mbarrier phase counters of a block, carried across its marches
 struct PairPhases {
     int v, s;   // v loads / cell-box loads issued (and waited) so far
@@ -554,6 +584,7 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
     };
     uint32_t lab_next = 0u;
     int *status = A.status;
+    volatile int *bad = reinterpret_cast<volatile int *>(smem + PS_BAD);
 
     if (tid == 0) {
         issue_v(q0);
@@ -579,6 +610,7 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
 #pragma unroll
             for (int J = 0; J < 6; ++J)
                 *reinterpret_cast<float2 *>(gs + (ring_base(J) + (ring_planes(J) == 4 ? s4 : r3)) * PS_GST + cg) = g[J];
+            if (!CM && A.fluid0 && strain_bad(g)) *bad = 1;
         }
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
@@ -599,6 +631,9 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
             if (q + 1 <= ze) issue_v(q + 1);
             if (q >= zb + 2 && q < ze) issue_s(q);   // plane z + 1, into the slot plane z - 1 used
         }
+        // the whole warp in the couplant (lanes with no cell to update have label 0)
+        const bool fluid = !CM && A.fluid0 && !*bad &&
+                           __all_sync(0xffffffffu, (lab2 & (LAB_MAT | (uint32_t)LAB_MAT << 16)) == 0u);
         if (z >= zb && any_out) {
             // strain planes z - 1, z, z + 1 were written at iterations i - 2, i - 1, i
             const int zr3 = r3 == 0 ? 2 : r3 - 1;   // plane z modulo 3
@@ -612,6 +647,8 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
                 const float *const cell = A.c21 + (long long)z * sz + col;
                 if (fast) stiff_all_cell<false>(pl, mg, cell, A.cplane, acc);
                 else stiff_all_cell<true>(pl, mg, cell, A.cplane, acc);
+            } else if (fluid) {
+                stiff_fluid(A, pl, acc);
             } else {
                 const float *const crow[2] = {tab + (lab[0] & LAB_MAT) * TAB36, tab + (lab[1] & LAB_MAT) * TAB36};
                 if (fast) stiff_all<false, TS>(pl, mg, crow, acc);
@@ -711,6 +748,7 @@ __device__ __forceinline__ void stress_pair_init(unsigned char *smem)
     float *gs = reinterpret_cast<float *>(smem + 128) + PS_VSLOT + 2 * PS_SSLOT;
     if (threadIdx.x == 0) {
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
+        *reinterpret_cast<int *>(smem + PS_BAD) = 0;
         fence_mbar_init();
     }
     // zero the strain planes' pads (read only by cells that are not updated)

@@ -9,6 +9,7 @@
 // same graph serves every chunk. This is the reference's Python step loop
 // (sim/core/fdtd.py:1786-1816) moved onto the device.
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -196,6 +197,8 @@ struct PeSolver {
     int px = 0;                 // padded row length
     void *pfields = nullptr;    // nine padded fields
     PeState pst{};
+    bool fluid0 = false;        // material 0 has only normal constants (StepArgs::fluid0)
+    float cfl[9] = {};
     uint16_t *lab_p = nullptr;
     float *dvol_p = nullptr;
     long long *src_idx_p = nullptr, *rec_cell_p = nullptr;   // probe cells in the padded layout
@@ -265,6 +268,8 @@ pe::StepArgs<T> make_args(const PeSolver *S, const PeState *st, int k)
     A.dense = S->variant == PE_KERNEL_DENSE;
     A.cpitch = S->px;
     A.cplane = (long long)S->px * S->cfg.ny * S->cfg.nz;
+    A.fluid0 = S->fluid0;
+    for (int k = 0; k < 9; ++k) A.cfl[k] = (T)S->cfl[k];
     return A;
 }
 
@@ -822,6 +827,20 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
             PE_CUDA(cudaMemcpyAsync(S->rho, md->rho, (size_t)es * c.n_mat, cudaMemcpyHostToDevice, st));
         }
         if (c.dtype == PE_F32 && !dense) {   // the pair kernels' tables
+            // nonzero constants of at least 1 Pa: a product with a strain then
+            // never rounds to zero, whose sign the skipped terms could change
+            const float *c0 = (const float *)md->ctab;
+            S->fluid0 = true;
+            for (int I = 0; I < 6; ++I)
+                for (int J = 0; J < 6; ++J) {
+                    const float v = c0[std::min(I, J) * 6 + std::max(I, J)];
+                    if (I < 3 && J < 3) {
+                        S->fluid0 = S->fluid0 && (v == 0.0f || std::fabs(v) >= 1.0f);
+                        S->cfl[3 * I + J] = v;
+                    } else {
+                        S->fluid0 = S->fluid0 && v == 0.0f;
+                    }
+                }
             if ((rc = dev_alloc(&S->tab36, sizeof(float) * pe::TAB36 * c.n_mat))) return rc;
             pe::k_c21_to_tab36<<<(c.n_mat + 127) / 128, 128, 0, st>>>((const float *)S->c21, S->tab36, c.n_mat);
             if ((rc = dev_alloc(&S->rinv, sizeof(float) * c.n_mat))) return rc;
