@@ -180,6 +180,16 @@ __device__ __forceinline__ float2 ld2_column(const float *p)
     else return ldg2_stream(p);
 }
 
+// Programmatic dependent launch: the step kernels follow one another with
+// nothing between them, so each is launched while its predecessor's last
+// blocks still run, sets up its block (barriers, table, pads: nothing a kernel
+// writes) and only then waits for the predecessor to have finished and its
+// writes to be visible. pdl_release lets the successor be launched; no-ops in
+// an ordinary launch. The column loads are L2-coherent (COH) in these
+// launches: the read-only path is for data nothing writes during the launch.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // ======================================================================== stress
 // Tap limits near the grid faces. The reference skips a tap whose reach
 // leaves the grid (sim/core/fdtd.py:1141-1162, :1215-1236): tap j of a
@@ -806,18 +816,20 @@ __global__ void __launch_bounds__(PS_N, 2) k_stress_pair(const __grid_constant__
 {
     extern __shared__ __align__(128) unsigned char smem_pair[];
     float *tsm = reinterpret_cast<float *>(smem_pair + PS_SMEM_FIXED);
+    pdl_release();
     stress_pair_init(smem_pair);
     if (TS) stage_table(tsm, tab36, n_mat);
     __syncthreads();
+    pdl_wait();
     const int zb = blockIdx.z * A.zc, ze = min(zb + A.zc, A.nz);
     PairPhases ph{0, 0};
     int bx, by;
     interior_first(pair_last_inside_x(A.nx), pair_last_inside_y(A.ny), gridDim.x, gridDim.y,
                    blockIdx.x + gridDim.x * blockIdx.y, bx, by);
     if (pair_tile_inside(A, bx, by))
-        stress_pair_march<NC, TS, true, false, CM>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
+        stress_pair_march<NC, TS, true, true, CM>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
     else
-        stress_pair_march<NC, TS, false, false, CM>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
+        stress_pair_march<NC, TS, false, true, CM>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
 }
 
 // ====================================================================== velocity
@@ -1217,6 +1229,7 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
     unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem_pair);
     float *rsm = reinterpret_cast<float *>(smem_pair + 128) + 3 * PV_SLOT;
     const int tid = threadIdx.x;
+    pdl_release();
     if (tid == 0) {
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
         fence_mbar_init();
@@ -1225,15 +1238,16 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
     if (rho_smem)
         for (int i = tid; i < n_mat; i += PV_N) rsm[i] = A.rho[i];
     __syncthreads();
+    pdl_wait();
     const float *rho_tab = rho_smem ? rsm : A.rho;
     const int zb = blockIdx.z * A.zc, ze = min(zb + A.zc, A.nz);
     int bx, by;
     interior_first(pair_vlast_inside_x(A.nx), pair_vlast_inside_y(A.ny), gridDim.x, gridDim.y,
                    blockIdx.x + gridDim.x * blockIdx.y, bx, by);
     if (pair_vtile_inside(A, bx, by))
-        velocity_pair_march<NC, true, false, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
+        velocity_pair_march<NC, true, true, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
     else
-        velocity_pair_march<NC, false, false, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
+        velocity_pair_march<NC, false, true, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
 }
 
 // ---------------------------------------------------------------- batches

@@ -288,6 +288,24 @@ void launch_simple_velocity(pe::StepArgs<T> A, int zc, cudaStream_t st)
     pe::k_velocity<T, TX, TY><<<grid, dim3(TX, TY, 1), 0, st>>>(A);
 }
 
+// launch that may start while its predecessor on the stream still drains
+// (programmatic dependent launch; the kernel waits before it reads a field)
+template <typename... P, typename... Q>
+void launch_chained(void (*fn)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, Q... args)
+{
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = dim3((unsigned)threads, 1, 1);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    cudaLaunchKernelEx(&lc, fn, static_cast<P>(args)...);   // errors surface in the caller's cudaGetLastError
+}
+
 template <typename T>
 void launch_stress(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t st)
 {
@@ -303,17 +321,17 @@ void launch_stress(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t st
             // stress tiles update columns [30 bx - 1, 30 bx + 29)
             dim3 grid((A.nx + pe::PS_OX) / pe::PS_OX, (A.ny + pe::PS_OY - 1) / pe::PS_OY, (A.nz + A.zc - 1) / A.zc);
             if (A.dense) {
-                if (A.nc == 4) pe::k_stress_pair<4, false, true><<<grid, pe::PS_N, pe::PS_SMEM_FIXED, st>>>(S->mps, A, nullptr, 0);
-                else pe::k_stress_pair<0, false, true><<<grid, pe::PS_N, pe::PS_SMEM_FIXED, st>>>(S->mps, A, nullptr, 0);
+                if (A.nc == 4) launch_chained(pe::k_stress_pair<4, false, true>, grid, pe::PS_N, pe::PS_SMEM_FIXED, st, S->mps, A, nullptr, 0);
+                else launch_chained(pe::k_stress_pair<0, false, true>, grid, pe::PS_N, pe::PS_SMEM_FIXED, st, S->mps, A, nullptr, 0);
                 return;
             }
             const int nm = S->cfg.n_mat;
             const size_t sm = pe::stress_pair_smem(nm);
             const bool ts = pe::pair_tab_in_smem(nm);
-            if (A.nc == 4 && ts) pe::k_stress_pair<4, true><<<grid, pe::PS_N, sm, st>>>(S->mps, A, S->tab36, nm);
-            else if (A.nc == 4) pe::k_stress_pair<4, false><<<grid, pe::PS_N, sm, st>>>(S->mps, A, S->tab36, nm);
-            else if (ts) pe::k_stress_pair<0, true><<<grid, pe::PS_N, sm, st>>>(S->mps, A, S->tab36, nm);
-            else pe::k_stress_pair<0, false><<<grid, pe::PS_N, sm, st>>>(S->mps, A, S->tab36, nm);
+            if (A.nc == 4 && ts) launch_chained(pe::k_stress_pair<4, true>, grid, pe::PS_N, sm, st, S->mps, A, S->tab36, nm);
+            else if (A.nc == 4) launch_chained(pe::k_stress_pair<4, false>, grid, pe::PS_N, sm, st, S->mps, A, S->tab36, nm);
+            else if (ts) launch_chained(pe::k_stress_pair<0, true>, grid, pe::PS_N, sm, st, S->mps, A, S->tab36, nm);
+            else launch_chained(pe::k_stress_pair<0, false>, grid, pe::PS_N, sm, st, S->mps, A, S->tab36, nm);
             return;
         }
     }
@@ -344,15 +362,15 @@ void launch_velocity(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t 
             dim3 grid((A.nx + pe::PV_OX - 1) / pe::PV_OX, (A.ny + pe::PV_OY - 1) / pe::PV_OY, (A.nz + A.zc - 1) / A.zc);
             if (A.dense) {
                 const size_t smc = pe::velocity_pair_smem(0);
-                if (A.nc == 4) pe::k_velocity_pair<4, true><<<grid, pe::PV_N, smc, st>>>(S->mpv, A, 0);
-                else pe::k_velocity_pair<0, true><<<grid, pe::PV_N, smc, st>>>(S->mpv, A, 0);
+                if (A.nc == 4) launch_chained(pe::k_velocity_pair<4, true>, grid, pe::PV_N, smc, st, S->mpv, A, 0);
+                else launch_chained(pe::k_velocity_pair<0, true>, grid, pe::PV_N, smc, st, S->mpv, A, 0);
                 return;
             }
             const size_t sm = pe::velocity_pair_smem(S->cfg.n_mat);
             if (A.nc == 4)
-                pe::k_velocity_pair<4><<<grid, pe::PV_N, sm, st>>>(S->mpv, A, S->cfg.n_mat);
+                launch_chained(pe::k_velocity_pair<4>, grid, pe::PV_N, sm, st, S->mpv, A, S->cfg.n_mat);
             else
-                pe::k_velocity_pair<0><<<grid, pe::PV_N, sm, st>>>(S->mpv, A, S->cfg.n_mat);
+                launch_chained(pe::k_velocity_pair<0>, grid, pe::PV_N, sm, st, S->mpv, A, S->cfg.n_mat);
             return;
         }
     }
