@@ -40,6 +40,7 @@ struct AdjArgs {
     const T *c21;      // (n_mat, C21_STRIDE)
     const T *rho;
     const float *rinv;  // (n_mat,) RN32(1 / rho) (FP32 solves), or null
+    const float *tab36; // (n_mat, 36) column-split stiffness (FP32 solves), or null
     const float *dz, *dy, *dx, *dvol;
     int nz, ny, nx;
     long long sy, sz;
@@ -592,5 +593,489 @@ __global__ void k_adj_velfin(AdjArgs<T> A)
 }
 
 #undef ADJ_DISPATCH
+
+// ======================================================================== pairs
+// FP32 adjoint kernels with two x-adjacent cells per thread, on grids of even
+// nx with 8-byte aligned fields. The one-cell kernels above are bound by their
+// instructions (k_adj_stress: 1460 per warp, half of them loads and address
+// arithmetic; issue 57-81 %, DRAM 10-31 %). A pair reads every y / z tap as one
+// 64-bit load for both cells, the eight or nine x taps of a row as five, and a
+// moved quantity's row as two, forms differences and sums as paired
+// instructions, and folds the two taps of a coefficient into one difference
+// and one fused multiply-add where the kernels above round four times. On
+// 96x160x160 (one reverse step, us): k_adj_vel 105 -> 67, k_adj_strain 47 ->
+// 28, k_adj_stress 183 -> 123, k_adj_velfin 79 -> 44, k_adj_vel_u 23 -> 17.
+// Blocks: 16 lanes (32 columns) x 16 rows of one plane. NC: the compile-time
+// tap count (0 = runtime): with it every load of a thread is issued before the
+// first is waited for, where a test per tap split them into nine serial groups.
+constexpr int AP_BX = 32, AP_BY = 16, AP_N = 256;
+
+__device__ __forceinline__ float2 ldp(const float *p) { return ldg2(p); }
+
+struct PairCell {
+    long long i;   // cell 0 (x even)
+    int iz, iy, ix;
+};
+__device__ __forceinline__ bool adj_pair_cell(const AdjArgs<float> &A, PairCell &c)
+{
+    c.ix = blockIdx.x * AP_BX + 2 * (threadIdx.x & 15);
+    c.iy = blockIdx.y * AP_BY + (threadIdx.x >> 4);
+    c.iz = blockIdx.z;
+    c.i = ((long long)c.iz * A.ny + c.iy) * A.nx + c.ix;
+    return c.ix < A.nx && c.iy < A.ny;
+}
+// adj_block_inside for the pair kernels' tiles
+__device__ __forceinline__ bool adj_pair_inside(const AdjArgs<float> &A)
+{
+    const int x0 = blockIdx.x * AP_BX, y0 = blockIdx.y * AP_BY, z = blockIdx.z;
+    return x0 >= ADJ_MARGIN_LO && x0 + AP_BX - 1 <= A.nx - ADJ_MARGIN_HI && y0 >= ADJ_MARGIN_LO &&
+           y0 + AP_BY - 1 <= A.ny - ADJ_MARGIN_HI && z >= ADJ_MARGIN_LO && z <= A.nz - ADJ_MARGIN_HI;
+}
+__device__ __forceinline__ float2 adj_pair_damp(const AdjArgs<float> &A, const PairCell &c)
+{
+    float2 d = bc2(1.0f);
+    if (A.dz) {
+        const float zy = A.dz[c.iz] * A.dy[c.iy];
+        d = mul2(bc2(zy), make_float2(A.dx[c.ix], A.dx[c.ix + 1]));
+    }
+    if (A.dvol) d = A.dz ? mul2(d, ldp(A.dvol + c.i)) : ldp(A.dvol + c.i);
+    return d;
+}
+__device__ __forceinline__ float2 keep2(float2 v, bool a, bool b) { return make_float2(a ? v.x : 0.0f, b ? v.y : 0.0f); }
+
+// The transposed taps' guards reduce to the cell's own position: the forward
+// cell below exists for y >= 2j + 1, the one above for y <= n - 2j - 2, for
+// forward and backward differences alike (gF / gB at the cells DfT / DbT read).
+struct AdjTapOk {
+    bool lo, hi;
+};
+template <bool G>
+__device__ __forceinline__ AdjTapOk adj_tap_ok(int y, int j, int n)
+{
+    return {!G || y >= 2 * j + 1, !G || y <= n - 2 * j - 2};
+}
+// the two taps of coefficient j: DfT (F) reads y - j - 1 and y + j, DbT y - j
+// and y + j + 1; a tap that does not exist is not loaded and counts zero
+template <bool F>
+__device__ __forceinline__ float2 adj_taps(const float *p, long long s, int j, AdjTapOk k)
+{
+    const float2 v1 = k.lo ? ldp(p + (F ? -j - 1 : -j) * s) : bc2(0.f);
+    const float2 v2 = k.hi ? ldp(p + (F ? j : j + 1) * s) : bc2(0.f);
+    return sub2(v1, v2);
+}
+// a row's values at columns x - 4 .. x + 5 (off the grid: zero)
+template <bool G>
+__device__ __forceinline__ void adj_row10(const float *p, int ix, int nx, float (&W)[10])
+{
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const int o = 2 * k - 4;
+        const float2 v = !G || (ix + o >= 0 && ix + o < nx) ? ldp(p + o) : bc2(0.f);
+        W[2 * k] = v.x;
+        W[2 * k + 1] = v.y;
+    }
+}
+// adj_taps along x, from such a row
+template <bool F>
+__device__ __forceinline__ float2 adj_taps_x(const float (&W)[10], int j, AdjTapOk k0, AdjTapOk k1)
+{
+    const int lo = 4 + (F ? -j - 1 : -j), hi = 4 + (F ? j : j + 1);
+    return make_float2((k0.lo ? W[lo] : 0.f) - (k0.hi ? W[hi] : 0.f), (k1.lo ? W[lo + 1] : 0.f) - (k1.hi ? W[hi + 1] : 0.f));
+}
+
+__global__ void __launch_bounds__(AP_N) k_adj_vel_u_pair(const AdjArgs<float> A)
+{
+    PairCell c;
+    if (!adj_pair_cell(A, c)) return;
+    const float2 d = adj_pair_damp(A, c);
+    const uint32_t l0 = __ldg(reinterpret_cast<const uint32_t *>(A.lab + c.i));
+    const bool xin = c.ix + 2 < A.nx, yin = c.iy < A.ny - 1, zin = c.iz < A.nz - 1;
+    const uint32_t lx = xin ? A.lab[c.i + 2] : 0u;
+    const uint32_t ly = yin ? __ldg(reinterpret_cast<const uint32_t *>(A.lab + c.i + A.sy)) : 0u;
+    const uint32_t lz = zin ? __ldg(reinterpret_cast<const uint32_t *>(A.lab + c.i + A.sz)) : 0u;
+    const int m[2] = {(int)(l0 & LAB_MAT), (int)(l0 >> 16 & LAB_MAT)};
+    const float r0[2] = {A.rho[m[0]], A.rho[m[1]]};
+    const float rx[2] = {r0[1], A.rho[lx & LAB_MAT]};
+    const float ry[2] = {A.rho[ly & LAB_MAT], A.rho[ly >> 16 & LAB_MAT]};
+    const float rz[2] = {A.rho[lz & LAB_MAT], A.rho[lz >> 16 & LAB_MAT]};
+    const float2 sc = mul2(d, bc2(A.dt_h));
+    const float2 v[3] = {mul2(sc, ldp(A.lv[0] + c.i)), mul2(sc, ldp(A.lv[1] + c.i)), mul2(sc, ldp(A.lv[2] + c.i))};
+    float u[3][2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        u[0][k] = adj_div(pick(v[0], k), k == 0 || xin ? 0.5f * (r0[k] + rx[k]) : r0[k], r0[k], A.rinv, m[k]);
+        u[1][k] = adj_div(pick(v[1], k), yin ? 0.5f * (r0[k] + ry[k]) : r0[k], r0[k], A.rinv, m[k]);
+        u[2][k] = adj_div(pick(v[2], k), zin ? 0.5f * (r0[k] + rz[k]) : r0[k], r0[k], A.rinv, m[k]);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) stg2(A.u[q] + c.i, u[q][0], u[q][1]);
+}
+
+// w of both cells for strain J (adj_w_cell)
+template <int J>
+__device__ __forceinline__ void adj_pair_w(const AdjArgs<float> &A, long long i, const float *const (&row)[2],
+                                           const float2 (&e)[6])
+{
+    float4 a[2];
+    float2 b[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        a[k] = ldg4(row[k] + 4 * J);
+        b[k] = ldg2(row[k] + 24 + 2 * J);
+    }
+    auto put = [&](int p, float2 v) { *reinterpret_cast<float2 *>(A.w[adj_widx(J, p)] + i) = v; };
+    if constexpr (J >= 3) {
+        float2 W = mul2(make_float2(a[0].x, a[1].x), e[0]);
+        W = fmac2(W, make_float2(a[0].y, a[1].y), e[1]);
+        put(0, fmac2(W, make_float2(a[0].z, a[1].z), e[2]));
+    }
+    if constexpr (J != 3) put(1, mul2(make_float2(a[0].w, a[1].w), e[3]));
+    if constexpr (J != 4) put(2, mul2(make_float2(b[0].x, b[1].x), e[4]));
+    if constexpr (J != 5) put(3, mul2(make_float2(b[0].y, b[1].y), e[5]));
+}
+
+template <int NC, bool G>
+__device__ __forceinline__ void adj_pair_vel(const AdjArgs<float> &A, const PairCell &c)
+{
+    const long long sy = A.sy, sz = A.sz, i = c.i;
+    const float *ux = A.u[0] + i, *uy = A.u[1] + i, *uz = A.u[2] + i;
+    float X[10], Y[10], Z[10];
+    adj_row10<G>(ux, c.ix, A.nx, X);
+    adj_row10<G>(uy, c.ix, A.nx, Y);
+    adj_row10<G>(uz, c.ix, A.nx, Z);
+    float2 ls[6] = {bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f)};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (NC ? j < NC : j < A.nc) {
+            const float2 cj = bc2(A.c[j]);
+            const AdjTapOk kz = adj_tap_ok<G>(c.iz, j, A.nz), ky = adj_tap_ok<G>(c.iy, j, A.ny);
+            const AdjTapOk k0 = adj_tap_ok<G>(c.ix, j, A.nx), k1 = adj_tap_ok<G>(c.ix + 1, j, A.nx);
+            ls[0] = fmac2(ls[0], cj, adj_taps_x<true>(X, j, k0, k1));
+            ls[1] = fmac2(ls[1], cj, adj_taps<true>(uy, sy, j, ky));
+            ls[2] = fmac2(ls[2], cj, adj_taps<true>(uz, sz, j, kz));
+            ls[3] = fmac2(ls[3], cj, adj_taps<false>(uy, sz, j, kz));
+            ls[3] = fmac2(ls[3], cj, adj_taps<false>(uz, sy, j, ky));
+            ls[4] = fmac2(ls[4], cj, adj_taps<false>(ux, sz, j, kz));
+            ls[4] = fmac2(ls[4], cj, adj_taps_x<false>(Z, j, k0, k1));
+            ls[5] = fmac2(ls[5], cj, adj_taps<false>(ux, sy, j, ky));
+            ls[5] = fmac2(ls[5], cj, adj_taps_x<false>(Y, j, k0, k1));
+        }
+    }
+    float2 e[6];
+#pragma unroll
+    for (int I = 0; I < 6; ++I) {
+        float2 *q = reinterpret_cast<float2 *>(A.ls[I] + i);
+        const float2 v = add2(*q, ls[I]);
+        *q = v;
+        e[I] = mul2(bc2(A.dt), v);
+    }
+    const uint32_t lab = __ldg(reinterpret_cast<const uint32_t *>(A.lab + i));
+    const float *const row[2] = {A.tab36 + (lab & LAB_MAT) * TAB36, A.tab36 + (lab >> 16 & LAB_MAT) * TAB36};
+    adj_pair_w<0>(A, i, row, e);
+    adj_pair_w<1>(A, i, row, e);
+    adj_pair_w<2>(A, i, row, e);
+    adj_pair_w<3>(A, i, row, e);
+    adj_pair_w<4>(A, i, row, e);
+    adj_pair_w<5>(A, i, row, e);
+}
+template <int NC>
+__global__ void __launch_bounds__(AP_N, 4) k_adj_vel_pair(const AdjArgs<float> A)
+{
+    PairCell c;
+    if (!adj_pair_cell(A, c)) return;
+    if (adj_pair_inside(A)) adj_pair_vel<NC, false>(A, c);
+    else adj_pair_vel<NC, true>(A, c);
+}
+
+// strains of v^{n-1} (the forward's taps, a skipped one reading the pair
+// itself twice, as in adj_strain_cell)
+template <int NC, bool G>
+__device__ __forceinline__ void adj_pair_strain(const AdjArgs<float> &A, const PairCell &c)
+{
+    const long long sy = A.sy, sz = A.sz, i = c.i;
+    const float *vx = A.vp[0] + i, *vy = A.vp[1] + i, *vz = A.vp[2] + i;
+    auto tap = [&](const float *p, bool ok, long long hi, long long lo) {
+        return sub2(ldp(ok ? p + hi : p), ldp(ok ? p + lo : p));
+    };
+    float X[10], Y[10], Z[10];
+    adj_row10<G>(vx, c.ix, A.nx, X);
+    adj_row10<G>(vy, c.ix, A.nx, Y);
+    adj_row10<G>(vz, c.ix, A.nx, Z);
+    float2 a[6] = {bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f)};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (NC ? j < NC : j < A.nc) {
+            const float2 cj = bc2(A.c[j]);
+            const bool by = !G || gB(c.iy, j, A.ny), bz = !G || gB(c.iz, j, A.nz);
+            const bool fy = !G || gF(c.iy, j, A.ny), fz = !G || gF(c.iz, j, A.nz);
+            bool bx[2], fx[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                bx[k] = !G || gB(c.ix + k, j, A.nx);
+                fx[k] = !G || gF(c.ix + k, j, A.nx);
+            }
+            a[0] = fmac2(a[0], cj, keep2(make_float2(X[4 + j] - X[3 - j], X[5 + j] - X[4 - j]), bx[0], bx[1]));
+            a[1] = fmac2(a[1], cj, tap(vy, by, j * sy, -(j + 1) * sy));
+            a[2] = fmac2(a[2], cj, tap(vz, bz, j * sz, -(j + 1) * sz));
+            a[3] = fmac2(a[3], cj, tap(vz, fy, (j + 1) * sy, -j * sy));
+            a[3] = fmac2(a[3], cj, tap(vy, fz, (j + 1) * sz, -j * sz));
+            a[4] = fmac2(a[4], cj, keep2(make_float2(Z[5 + j] - Z[4 - j], Z[6 + j] - Z[5 - j]), fx[0], fx[1]));
+            a[4] = fmac2(a[4], cj, tap(vx, fz, (j + 1) * sz, -j * sz));
+            a[5] = fmac2(a[5], cj, keep2(make_float2(Y[5 + j] - Y[4 - j], Y[6 + j] - Y[5 - j]), fx[0], fx[1]));
+            a[5] = fmac2(a[5], cj, tap(vx, fy, (j + 1) * sy, -j * sy));
+        }
+    }
+#pragma unroll
+    for (int J = 0; J < 6; ++J) *reinterpret_cast<float2 *>(A.g[J] + i) = mul2(a[J], bc2(A.inv_h));
+}
+template <int NC>
+__global__ void __launch_bounds__(AP_N, 4) k_adj_strain_pair(const AdjArgs<float> A)
+{
+    PairCell c;
+    if (!adj_pair_cell(A, c)) return;
+    if (adj_pair_inside(A)) adj_pair_strain<NC, false>(A, c);
+    else adj_pair_strain<NC, true>(A, c);
+}
+
+// adj_q for both cells
+template <int P, int J, bool G>
+__device__ __forceinline__ float2 adj_pair_q(const AdjArgs<float> &A, const PairCell &c)
+{
+    constexpr int S = vpos(J);
+    constexpr int DZ = pos_z(P) - pos_z(S), DY = pos_y(P) - pos_y(S), DX = pos_x(P) - pos_x(S);
+    const float *g = A.g[J] + c.i;
+    if constexpr (DZ == 0 && DY == 0 && DX == 0) {
+        return ldp(g);
+    } else {
+        // guards of the z and y axes (both cells), then of x
+        const bool zy = !G || ((DZ <= 0 || c.iz <= A.nz - 2) && (DZ >= 0 || c.iz >= 1) &&
+                               (DY <= 0 || c.iy <= A.ny - 2) && (DY >= 0 || c.iy >= 1));
+        float2 acc = bc2(0.f);
+#pragma unroll
+        for (int a0 = (DZ < 0 ? -1 : 0); a0 <= (DZ > 0 ? 1 : 0); ++a0)
+#pragma unroll
+            for (int a1 = (DY < 0 ? -1 : 0); a1 <= (DY > 0 ? 1 : 0); ++a1) {
+                const float *r = zy ? g + a0 * A.sz + a1 * A.sy : g;
+                const float2 v = ldp(r);
+                if constexpr (DX == 0) {
+                    acc = add2(acc, v);
+                } else if constexpr (DX > 0) {
+                    const float2 w = ldp(!G || c.ix + 2 < A.nx ? r + 2 : r);
+                    acc = add2(acc, make_float2(v.x + v.y, v.y + w.x));
+                } else {
+                    const float2 w = ldp(!G || c.ix >= 2 ? r - 2 : r);
+                    acc = add2(acc, make_float2(w.y + v.x, v.x + v.y));
+                }
+            }
+        acc = mul2(acc, bc2(0.25f));
+        if constexpr (G)
+            acc = keep2(acc, zy && (DX >= 0 || c.ix >= 1), zy && (DX <= 0 || c.ix + 1 <= A.nx - 2));
+        return acc;
+    }
+}
+
+// gradient terms of the stresses at position P: v[slot(I, J)] += e_I q[P][J]
+template <int P, bool G>
+__device__ __forceinline__ void adj_pair_grad(const AdjArgs<float> &A, const PairCell &c, const float2 (&e)[6],
+                                              float2 (&v)[21])
+{
+    const float2 q[6] = {adj_pair_q<P, 0, G>(A, c), adj_pair_q<P, 1, G>(A, c), adj_pair_q<P, 2, G>(A, c),
+                         adj_pair_q<P, 3, G>(A, c), adj_pair_q<P, 4, G>(A, c), adj_pair_q<P, 5, G>(A, c)};
+#pragma unroll
+    for (int I = 0; I < 6; ++I)
+        if (vpos(I) == P) {
+#pragma unroll
+            for (int J = 0; J < 6; ++J) {
+                // I <= J: the term's first product (positions ascend with the index)
+                float2 &t = v[c21_slot(I, J)];
+                t = J >= I ? mul2(e[I], q[J]) : fmac2(t, e[I], q[J]);
+            }
+        }
+}
+
+// adj_t's moved part for both cells: the transposed move of w[P][J]
+template <int J, int P, bool G>
+__device__ __forceinline__ void adj_pair_t(const AdjArgs<float> &A, const PairCell &c, float2 &acc)
+{
+    constexpr int S = vpos(J);
+    constexpr int DZ = pos_z(P) - pos_z(S), DY = pos_y(P) - pos_y(S), DX = pos_x(P) - pos_x(S);
+    if constexpr (DZ != 0 || DY != 0 || DX != 0) {
+        const float *w = A.w[adj_widx(J, P)] + c.i;
+        // the forward guard of axis offset d at forward position y
+        auto ok = [](int y, int d, int n) { return y >= 0 && y < n && (d <= 0 || y <= n - 2) && (d >= 0 || y >= 1); };
+        float2 sum = bc2(0.f);
+#pragma unroll
+        for (int a0 = (DZ < 0 ? -1 : 0); a0 <= (DZ > 0 ? 1 : 0); ++a0)
+#pragma unroll
+            for (int a1 = (DY < 0 ? -1 : 0); a1 <= (DY > 0 ? 1 : 0); ++a1) {
+                const bool zy = !G || (ok(c.iz - a0, DZ, A.nz) && ok(c.iy - a1, DY, A.ny));
+                const float *r = zy ? w - a0 * A.sz - a1 * A.sy : w;
+                float2 v = ldp(r);
+                if constexpr (DX == 0) {
+                    sum = add2(sum, G ? keep2(v, zy, zy) : v);
+                } else {
+                    // the pair and its neighbour on the side of the taps
+                    float2 o = DX > 0 ? ldp(!G || c.ix >= 2 ? r - 2 : r) : ldp(!G || c.ix + 2 < A.nx ? r + 2 : r);
+                    if constexpr (G) {
+                        v = keep2(v, zy && ok(c.ix, DX, A.nx), zy && ok(c.ix + 1, DX, A.nx));
+                        o = DX > 0 ? keep2(o, false, zy && ok(c.ix - 1, DX, A.nx))
+                                   : keep2(o, zy && ok(c.ix + 2, DX, A.nx), false);
+                    }
+                    sum = add2(sum, DX > 0 ? make_float2(o.y + v.x, v.x + v.y) : make_float2(v.x + v.y, v.y + o.x));
+                }
+            }
+        acc = fmac2(acc, bc2(0.25f), sum);
+    }
+}
+template <int J, bool G>
+__device__ __forceinline__ void adj_pair_tJ(const AdjArgs<float> &A, const PairCell &c, const float *const (&row)[2],
+                                            const float2 (&e)[6])
+{
+    float2 acc = bc2(0.f);
+#pragma unroll
+    for (int I = 0; I < 6; ++I)
+        if (vpos(I) == vpos(J))
+            acc = fmac2(acc, make_float2(__ldg(row[0] + c21_slot(I, J)), __ldg(row[1] + c21_slot(I, J))), e[I]);
+    adj_pair_t<J, 0, G>(A, c, acc);
+    adj_pair_t<J, 1, G>(A, c, acc);
+    adj_pair_t<J, 2, G>(A, c, acc);
+    adj_pair_t<J, 3, G>(A, c, acc);
+    *reinterpret_cast<float2 *>(A.t[J] + c.i) = acc;
+}
+template <bool G>
+__device__ __forceinline__ void adj_pair_strain_adjoint(const AdjArgs<float> &A, const PairCell &c,
+                                                        const float *const (&row)[2], const float2 (&e)[6])
+{
+    adj_pair_tJ<0, G>(A, c, row, e);
+    adj_pair_tJ<1, G>(A, c, row, e);
+    adj_pair_tJ<2, G>(A, c, row, e);
+    adj_pair_tJ<3, G>(A, c, row, e);
+    adj_pair_tJ<4, G>(A, c, row, e);
+    adj_pair_tJ<5, G>(A, c, row, e);
+}
+
+__global__ void __launch_bounds__(AP_N, 3) k_adj_stress_pair(const AdjArgs<float> A)
+{
+    // k_adj_stress's per-material sums over the 64 cells of a warp: row
+    // 32 c + lane of the tile holds the terms of cell c of a lane
+    __shared__ float red[AP_N / 32][64][21];
+    PairCell c;
+    const bool live = adj_pair_cell(A, c), inside = adj_pair_inside(A);
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int m[2] = {-1, -1};
+    bool any[2] = {false, false};
+    float2 e[6];
+    if (live) {
+        const uint32_t lab = __ldg(reinterpret_cast<const uint32_t *>(A.lab + c.i));
+        m[0] = lab & LAB_MAT;
+        m[1] = lab >> 16 & LAB_MAT;
+#pragma unroll
+        for (int I = 0; I < 6; ++I) e[I] = mul2(bc2(A.dt), *reinterpret_cast<const float2 *>(A.ls[I] + c.i));
+        float2 v[21];
+        if (inside) {
+            adj_pair_grad<0, false>(A, c, e, v);
+            adj_pair_grad<1, false>(A, c, e, v);
+            adj_pair_grad<2, false>(A, c, e, v);
+            adj_pair_grad<3, false>(A, c, e, v);
+        } else {
+            adj_pair_grad<0, true>(A, c, e, v);
+            adj_pair_grad<1, true>(A, c, e, v);
+            adj_pair_grad<2, true>(A, c, e, v);
+            adj_pair_grad<3, true>(A, c, e, v);
+        }
+#pragma unroll
+        for (int k = 0; k < 21; ++k) {
+            red[warp][lane][k] = v[k].x;
+            red[warp][32 + lane][k] = v[k].y;
+            any[0] = any[0] || v[k].x != 0.0f;
+            any[1] = any[1] || v[k].y != 0.0f;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 21; ++k) red[warp][lane][k] = red[warp][32 + lane][k] = 0.0f;
+    }
+    __syncwarp();
+    double *gtab = A.grad;
+    if (A.grad_rep > 1)
+        gtab += (long long)(((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x * (AP_N / 32) +
+                             blockIdx.x * (AP_N / 32) + warp) %
+                            (unsigned)A.grad_rep) * A.n_mat * 21;
+    const int my0 = any[0] ? m[0] : -1, my1 = any[1] ? m[1] : -1;
+    unsigned rem0 = __ballot_sync(full, any[0]), rem1 = __ballot_sync(full, any[1]);
+    while (rem0 | rem1) {
+        const int from0 = __shfl_sync(full, my0, __ffs(rem0) - 1), from1 = __shfl_sync(full, my1, __ffs(rem1) - 1);
+        const int mm = rem0 ? from0 : from1;
+        const unsigned k0 = __ballot_sync(full, my0 == mm), k1 = __ballot_sync(full, my1 == mm);
+        rem0 &= ~k0;
+        rem1 &= ~k1;
+        if (lane < 21) {
+            double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;   // four chains, for latency
+#pragma unroll
+            for (int r = 0; r < 32; r += 2) {
+                if (k0 >> r & 1u) v0 += (double)red[warp][r][lane];
+                if (k0 >> r & 2u) v1 += (double)red[warp][r + 1][lane];
+                if (k1 >> r & 1u) v2 += (double)red[warp][32 + r][lane];
+                if (k1 >> r & 2u) v3 += (double)red[warp][32 + r + 1][lane];
+            }
+            atomicAdd(gtab + (long long)mm * 21 + lane, (v0 + v1) + (v2 + v3));
+        }
+    }
+    if (!live) return;
+    const float *const row[2] = {A.c21 + (long long)m[0] * C21_STRIDE, A.c21 + (long long)m[1] * C21_STRIDE};
+    if (inside) adj_pair_strain_adjoint<false>(A, c, row, e);
+    else adj_pair_strain_adjoint<true>(A, c, row, e);
+    const float2 d = adj_pair_damp(A, c);
+#pragma unroll
+    for (int I = 0; I < 6; ++I) {
+        float2 *q = reinterpret_cast<float2 *>(A.ls[I] + c.i);
+        *q = mul2(d, *q);
+    }
+}
+
+template <int NC, bool G>
+__device__ __forceinline__ void adj_pair_velfin(const AdjArgs<float> &A, const PairCell &c)
+{
+    const long long sy = A.sy, sz = A.sz, i = c.i;
+    const float *t1 = A.t[0] + i, *t2 = A.t[1] + i, *t3 = A.t[2] + i;
+    const float *t4 = A.t[3] + i, *t5 = A.t[4] + i, *t6 = A.t[5] + i;
+    float X[10], Y[10], Z[10];
+    adj_row10<G>(t1, c.ix, A.nx, X);
+    adj_row10<G>(t6, c.ix, A.nx, Y);
+    adj_row10<G>(t5, c.ix, A.nx, Z);
+    float2 gx = bc2(0.f), gy = bc2(0.f), gz = bc2(0.f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (NC ? j < NC : j < A.nc) {
+            const float2 cj = bc2(A.c[j]);
+            const AdjTapOk kz = adj_tap_ok<G>(c.iz, j, A.nz), ky = adj_tap_ok<G>(c.iy, j, A.ny);
+            const AdjTapOk k0 = adj_tap_ok<G>(c.ix, j, A.nx), k1 = adj_tap_ok<G>(c.ix + 1, j, A.nx);
+            gx = fmac2(gx, cj, adj_taps_x<false>(X, j, k0, k1));
+            gx = fmac2(gx, cj, adj_taps<true>(t5, sz, j, kz));
+            gx = fmac2(gx, cj, adj_taps<true>(t6, sy, j, ky));
+            gy = fmac2(gy, cj, adj_taps<false>(t2, sy, j, ky));
+            gy = fmac2(gy, cj, adj_taps<true>(t4, sz, j, kz));
+            gy = fmac2(gy, cj, adj_taps_x<true>(Y, j, k0, k1));
+            gz = fmac2(gz, cj, adj_taps<false>(t3, sz, j, kz));
+            gz = fmac2(gz, cj, adj_taps<true>(t4, sy, j, ky));
+            gz = fmac2(gz, cj, adj_taps_x<true>(Z, j, k0, k1));
+        }
+    }
+    const float2 d = adj_pair_damp(A, c), ih = bc2(A.inv_h);
+    const float2 r[3] = {gx, gy, gz};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float2 *q = reinterpret_cast<float2 *>(A.lv[k] + i);
+        *q = fmac2(mul2(ih, r[k]), d, *q);
+    }
+}
+template <int NC>
+__global__ void __launch_bounds__(AP_N, 4) k_adj_velfin_pair(const AdjArgs<float> A)
+{
+    PairCell c;
+    if (!adj_pair_cell(A, c)) return;
+    if (adj_pair_inside(A)) adj_pair_velfin<NC, false>(A, c);
+    else adj_pair_velfin<NC, true>(A, c);
+}
 
 }  // namespace pe

@@ -1068,6 +1068,7 @@ int adjoint_step_t(PeSolver *S, const PeAdjoint *adj, int64_t n, const void *res
     A.c21 = (const T *)S->c21;
     A.rho = (const T *)S->rho;
     A.rinv = S->rinv;
+    A.tab36 = S->tab36;
     A.dz = S->dz;
     A.dy = S->dy;
     A.dx = S->dx;
@@ -1091,6 +1092,29 @@ int adjoint_step_t(PeSolver *S, const PeAdjoint *adj, int64_t n, const void *res
         pe::k_adj_inject<T><<<(S->n_rec + 127) / 128, 128, 0, st>>>(A, S->rec_cell, S->rec_pos, (const T *)S->rec_w,
                                                                      S->ent_group, S->n_rec, row, c.record,
                                                                      c.damped_record);
+    }
+    if constexpr (std::is_same<T, float>::value) {
+        // two cells per thread where a row's pairs are 64-bit units of every field
+        bool pairs = c.nx % 2 == 0 && S->tab36 && ((uintptr_t)adj->scratch % 8) == 0 && ((uintptr_t)S->dvol % 8) == 0;
+        for (int i = 0; i < 3; ++i) pairs = pairs && ((uintptr_t)A.lv[i] % 8) == 0 && ((uintptr_t)A.vp[i] % 8) == 0;
+        for (int i = 0; i < 6; ++i) pairs = pairs && ((uintptr_t)A.ls[i] % 8) == 0;
+        if (pairs) {
+            const dim3 pg((unsigned)((c.nx + pe::AP_BX - 1) / pe::AP_BX), (unsigned)((c.ny + pe::AP_BY - 1) / pe::AP_BY),
+                          (unsigned)c.nz);
+            pe::k_adj_vel_u_pair<<<pg, pe::AP_N, 0, st>>>(A);
+            if (A.nc == 4) {
+                pe::k_adj_vel_pair<4><<<pg, pe::AP_N, 0, st>>>(A);
+                pe::k_adj_strain_pair<4><<<pg, pe::AP_N, 0, st>>>(A);
+            } else {
+                pe::k_adj_vel_pair<0><<<pg, pe::AP_N, 0, st>>>(A);
+                pe::k_adj_strain_pair<0><<<pg, pe::AP_N, 0, st>>>(A);
+            }
+            pe::k_adj_stress_pair<<<pg, pe::AP_N, 0, st>>>(A);
+            if (A.nc == 4) pe::k_adj_velfin_pair<4><<<pg, pe::AP_N, 0, st>>>(A);
+            else pe::k_adj_velfin_pair<0><<<pg, pe::AP_N, 0, st>>>(A);
+            PE_CUDA(cudaGetLastError());
+            return PE_OK;
+        }
     }
     // cell kernels: 32 x 8 blocks over (x tiles, y tiles, z planes)
     const dim3 ab(pe::ADJ_BX, pe::ADJ_BY, 1);
