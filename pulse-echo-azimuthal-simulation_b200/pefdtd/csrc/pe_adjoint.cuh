@@ -603,8 +603,8 @@ __global__ void k_adj_velfin(AdjArgs<T> A)
 // moved quantity's row as two, forms differences and sums as paired
 // instructions, and folds the two taps of a coefficient into one difference
 // and one fused multiply-add where the kernels above round four times. On
-// 96x160x160 (one reverse step, us): k_adj_vel 105 -> 67, k_adj_strain 47 ->
-// 28, k_adj_stress 183 -> 123, k_adj_velfin 79 -> 44, k_adj_vel_u 23 -> 17.
+// 96x160x160 (one reverse step, us): k_adj_vel 105 -> 88, k_adj_strain 47 ->
+// 31, k_adj_stress 183 -> 135, k_adj_velfin 79 -> 53, k_adj_vel_u 23 -> 18.
 // Blocks: 16 lanes (32 columns) x 16 rows of one plane. NC: the compile-time
 // tap count (0 = runtime): with it every load of a thread is issued before the
 // first is waited for, where a test per tap split them into nine serial groups.
@@ -855,21 +855,20 @@ __device__ __forceinline__ float2 adj_pair_q(const AdjArgs<float> &A, const Pair
         for (int a0 = (DZ < 0 ? -1 : 0); a0 <= (DZ > 0 ? 1 : 0); ++a0)
 #pragma unroll
             for (int a1 = (DY < 0 ? -1 : 0); a1 <= (DY > 0 ? 1 : 0); ++a1) {
-                const float *r = zy ? g + a0 * A.sz + a1 * A.sy : g;
-                const float2 v = ldp(r);
+                const float *r = g + a0 * A.sz + a1 * A.sy;
+                const float2 v = zy ? ldp(r) : bc2(0.f);
                 if constexpr (DX == 0) {
                     acc = add2(acc, v);
                 } else if constexpr (DX > 0) {
-                    const float2 w = ldp(!G || c.ix + 2 < A.nx ? r + 2 : r);
+                    const float2 w = zy && (!G || c.ix + 2 < A.nx) ? ldp(r + 2) : bc2(0.f);
                     acc = add2(acc, make_float2(v.x + v.y, v.y + w.x));
                 } else {
-                    const float2 w = ldp(!G || c.ix >= 2 ? r - 2 : r);
+                    const float2 w = zy && (!G || c.ix >= 2) ? ldp(r - 2) : bc2(0.f);
                     acc = add2(acc, make_float2(w.y + v.x, v.x + v.y));
                 }
             }
         acc = mul2(acc, bc2(0.25f));
-        if constexpr (G)
-            acc = keep2(acc, zy && (DX >= 0 || c.ix >= 1), zy && (DX <= 0 || c.ix + 1 <= A.nx - 2));
+        if constexpr (G && DX != 0) acc = keep2(acc, DX >= 0 || c.ix >= 1, DX <= 0 || c.ix + 1 <= A.nx - 2);
         return acc;
     }
 }
@@ -909,18 +908,17 @@ __device__ __forceinline__ void adj_pair_t(const AdjArgs<float> &A, const PairCe
 #pragma unroll
             for (int a1 = (DY < 0 ? -1 : 0); a1 <= (DY > 0 ? 1 : 0); ++a1) {
                 const bool zy = !G || (ok(c.iz - a0, DZ, A.nz) && ok(c.iy - a1, DY, A.ny));
-                const float *r = zy ? w - a0 * A.sz - a1 * A.sy : w;
-                float2 v = ldp(r);
+                const float *r = w - a0 * A.sz - a1 * A.sy;
+                float2 v = zy ? ldp(r) : bc2(0.f);
                 if constexpr (DX == 0) {
-                    sum = add2(sum, G ? keep2(v, zy, zy) : v);
+                    sum = add2(sum, v);
                 } else {
-                    // the pair and its neighbour on the side of the taps
-                    float2 o = DX > 0 ? ldp(!G || c.ix >= 2 ? r - 2 : r) : ldp(!G || c.ix + 2 < A.nx ? r + 2 : r);
-                    if constexpr (G) {
-                        v = keep2(v, zy && ok(c.ix, DX, A.nx), zy && ok(c.ix + 1, DX, A.nx));
-                        o = DX > 0 ? keep2(o, false, zy && ok(c.ix - 1, DX, A.nx))
-                                   : keep2(o, zy && ok(c.ix + 2, DX, A.nx), false);
-                    }
+                    // the pair and its neighbour on the side of the taps; of the
+                    // forward cells in the grid the x guard drops only the last
+                    // column (DX > 0) or the first (DX < 0)
+                    const bool in = zy && (!G || (DX > 0 ? c.ix >= 2 : c.ix + 2 < A.nx));
+                    const float2 o = in ? ldp(DX > 0 ? r - 2 : r + 2) : bc2(0.f);
+                    if constexpr (G) v = keep2(v, DX > 0 || c.ix >= 1, DX < 0 || c.ix + 1 <= A.nx - 2);
                     sum = add2(sum, DX > 0 ? make_float2(o.y + v.x, v.x + v.y) : make_float2(v.x + v.y, v.y + o.x));
                 }
             }
