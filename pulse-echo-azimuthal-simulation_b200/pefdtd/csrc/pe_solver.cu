@@ -1169,24 +1169,30 @@ int pe_solver_adjoint_segment(PeSolver *S, const PeState *state, const PeAdjoint
     if (pad && (rc = pad_in(S, state, st))) return rc;
     const size_t fb = (size_t)S->esize * (size_t)S->ncell;   // bytes of one field
     char *hist = (char *)v_hist;
-    // recompute the segment, keeping v before every step
+    // recompute the segment, keeping v before every step. The step counter is
+    // set once per chunk (a kernel's samples go to row k of the chunk's buffer),
+    // and v goes out in one copy where its fields lie back to back
+    const bool v_together = (char *)use->v[1] == (char *)use->v[0] + fb && (char *)use->v[2] == (char *)use->v[1] + fb;
     for (int64_t n = a; n < b; ++n) {
+        char *h = hist + (size_t)(n - a) * 3 * fb;
         if (pad) {
-            PeState h{};
-            for (int c = 0; c < 3; ++c) h.v[c] = hist + ((size_t)(n - a) * 3 + c) * fb;
-            if ((rc = repitch(S, use, S->px, &h, 0, 3, st))) return rc;
+            PeState hv{};
+            for (int c = 0; c < 3; ++c) hv.v[c] = h + c * fb;
+            if ((rc = repitch(S, use, S->px, &hv, 0, 3, st))) return rc;
+        } else if (v_together) {
+            PE_CUDA(cudaMemcpyAsync(h, use->v[0], 3 * fb, cudaMemcpyDeviceToDevice, st));
         } else {
             for (int c = 0; c < 3; ++c)
-                PE_CUDA(cudaMemcpyAsync(hist + ((size_t)(n - a) * 3 + c) * fb, state->v[c], fb,
-                                        cudaMemcpyDeviceToDevice, st));
+                PE_CUDA(cudaMemcpyAsync(h + c * fb, use->v[c], fb, cudaMemcpyDeviceToDevice, st));
         }
-        pe::k_step_set<<<1, 1, 0, st>>>(S->step, n);
+        const int k = (int)((n - a) % S->chunk);
+        if (k == 0) pe::k_step_set<<<1, 1, 0, st>>>(S->step, n);
         if (S->cfg.dtype == PE_F64) {
-            pe::StepArgs<double> A = make_args<double>(S, use, 0);
+            pe::StepArgs<double> A = make_args<double>(S, use, k);
             launch_stress<double>(S, A, st);
             launch_velocity<double>(S, A, st);
         } else {
-            pe::StepArgs<float> A = make_args<float>(S, use, 0);
+            pe::StepArgs<float> A = make_args<float>(S, use, k);
             launch_stress<float>(S, A, st);
             launch_velocity<float>(S, A, st);
         }
