@@ -46,20 +46,9 @@ constexpr int PS_SSZP = 512;                                      // ... padded 
 constexpr int PS_GW = 32, PS_GOFF = 8, PS_GST = 2 * PS_GOFF + PS_GW * PS_ROWS;   // strain plane: pad, 32 x 16, pad
 constexpr int PS_VSLOT = 3 * PS_VSZ;
 constexpr int PS_SSLOT = 6 * PS_SSZP;
-// Strain ring: the update of plane z reads g4 and g5 at planes z - 1 and z,
-// the other four components at z and z + 1 (the half-cell moves,
-// sim/core/fdtd.py:612-633). While it runs, the strains of plane z + 2 are
-// written; with four planes for g4, g5 and three for the others they never
-// overwrite what the update reads, so one block barrier per plane suffices.
-__host__ __device__ constexpr int ring_planes(int J) { return (J == 3 || J == 4) ? 4 : 3; }
-__host__ __device__ constexpr int ring_base(int J)   // first plane of component J, in planes
-{
-    return J < 3 ? 3 * J : (J == 5 ? 9 : (J == 3 ? 12 : 16));
-}
-constexpr int PS_RING = 20;   // strain planes held
 // shared memory of a stress block: mbarriers (v, cell slot 0, cell slot 1),
 // one v slot, two cell slots, the strain ring, then the material table
-constexpr size_t PS_SMEM_FIXED = 128 + sizeof(float) * ((size_t)PS_VSLOT + 2 * (size_t)PS_SSLOT + (size_t)PS_RING * PS_GST);
+constexpr size_t PS_SMEM_FIXED = 128 + sizeof(float) * ((size_t)PS_VSLOT + 2 * (size_t)PS_SSLOT + (size_t)RING_PLANES * PS_GST);
 constexpr int TAB36 = 36;   // material: columns J as [C0J..C3J] at 4J, then [C4J, C5J] at 24 + 2J
 // velocity
 // two velocity blocks of 256 threads share an SM, so that one block's
@@ -746,7 +735,7 @@ __device__ __forceinline__ void stage_table(float *dst, const float *src, int n_
 __device__ __forceinline__ void stress_pair_zero_pads(unsigned char *smem)
 {
     float *gs = reinterpret_cast<float *>(smem + 128) + PS_VSLOT + 2 * PS_SSLOT;
-    for (int i = threadIdx.x; i < PS_RING * 2 * PS_GOFF; i += blockDim.x) {
+    for (int i = threadIdx.x; i < RING_PLANES * 2 * PS_GOFF; i += blockDim.x) {
         const int p = i / (2 * PS_GOFF), k = i % (2 * PS_GOFF);
         gs[p * PS_GST + (k < PS_GOFF ? k : PS_GST - 2 * PS_GOFF + k)] = 0.f;
     }
@@ -762,7 +751,7 @@ __device__ __forceinline__ void stress_pair_init(unsigned char *smem)
         fence_mbar_init();
     }
     // zero the strain planes' pads (read only by cells that are not updated)
-    for (int i = threadIdx.x; i < PS_RING * 2 * PS_GOFF; i += blockDim.x) {
+    for (int i = threadIdx.x; i < RING_PLANES * 2 * PS_GOFF; i += blockDim.x) {
         const int p = i / (2 * PS_GOFF), k = i % (2 * PS_GOFF);
         gs[p * PS_GST + (k < PS_GOFF ? k : PS_GST - 2 * PS_GOFF + k)] = 0.f;
     }

@@ -80,7 +80,7 @@ __device__ __forceinline__ void load_c21(const T *Cr, bool shared, T Cm[24])
         const double2 *p = reinterpret_cast<const double2 *>(Cr);
 #pragma unroll
         for (int k = 0; k < 12; ++k) {
-            const double2 u = __ldg(p + k);
+            const double2 u = shared ? p[k] : __ldg(p + k);
             Cm[2 * k] = u.x; Cm[2 * k + 1] = u.y;
         }
     }

@@ -43,6 +43,18 @@ constexpr int KS_SW = 36, KS_SH = 16, KS_SSZ = KS_SW * KS_SH;   // stress s cent
 constexpr int KV_SW = 40, KV_SH = 24, KV_SSZ = KV_SW * KV_SH;   // velocity s tile
 constexpr int KV_CW = 32, KV_CH = 16, KV_CSZ = KV_CW * KV_CH;   // velocity centres
 
+// Strain ring: the update of plane z reads g4 and g5 at planes z - 1 and z,
+// the other four components at z and z + 1 (the half-cell moves,
+// sim/core/fdtd.py:612-633). While it runs, the strains of plane z + 2 are
+// written; with four planes for g4, g5 and three for the others they never
+// overwrite what the update reads, so one block barrier per plane suffices.
+__host__ __device__ constexpr int ring_planes(int J) { return (J == 3 || J == 4) ? 4 : 3; }
+__host__ __device__ constexpr int ring_base(int J)   // first plane of component J, in planes
+{
+    return J < 3 ? 3 * J : (J == 5 ? 9 : (J == 3 ? 12 : 16));
+}
+constexpr int RING_PLANES = 20;   // strain planes held
+
 // slot sizes in elements of T (each box padded to 128 bytes)
 template <typename T>
 __host__ __device__ constexpr int pad128(int elems)
@@ -56,16 +68,28 @@ __host__ __device__ constexpr int ks_slot_s() { return 6 * pad128<T>(KS_SSZ) + p
 template <typename T>
 __host__ __device__ constexpr int kv_slot() { return 5 * pad128<T>(KV_SSZ) + 4 * pad128<T>(KV_CSZ); }
 
+// Stress slots: three in FP32 (boxes issued two planes ahead); two in FP64,
+// whose boxes are twice as large: 193 KB with the strain ring, which leaves
+// 34 KB for the material table. Three would not fit a block, and the cp.async
+// kernels that ran FP64 before read the table through L1 behind a block
+// barrier: 64x96x96, one step, 56 + 24 us against 48.5 + 20 here.
+template <typename T>
+__host__ __device__ constexpr int ks_slots() { return sizeof(T) == 8 ? 2 : 3; }
+template <typename T>
+__host__ __device__ constexpr bool table_in_smem_tma(int n_mat)
+{
+    return sizeof(T) == 4 ? table_in_smem<T>(n_mat) : n_mat <= 180;
+}
 template <typename T>
 __host__ __device__ constexpr size_t stress_tma_smem(int n_mat)
 {
-    return 128 + sizeof(T) * (3 * (size_t)(ks_slot_v<T>() + ks_slot_s<T>()) + (size_t)3 * 6 * TB_N +
-                              (table_in_smem<T>(n_mat) ? (size_t)n_mat * C21_STRIDE : 0));
+    return 128 + sizeof(T) * (ks_slots<T>() * (size_t)(ks_slot_v<T>() + ks_slot_s<T>()) + (size_t)RING_PLANES * TB_N +
+                              (table_in_smem_tma<T>(n_mat) ? (size_t)n_mat * C21_STRIDE : 0));
 }
 template <typename T>
 __host__ __device__ constexpr size_t velocity_tma_smem(int n_mat)
 {
-    return 128 + sizeof(T) * (3 * (size_t)kv_slot<T>() + (table_in_smem<T>(n_mat) ? (size_t)n_mat : 0));
+    return 128 + sizeof(T) * (3 * (size_t)kv_slot<T>() + (table_in_smem_tma<T>(n_mat) ? (size_t)n_mat : 0));
 }
 
 // ---------------------------------------------------------------- PTX helpers
@@ -114,6 +138,11 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 
 __device__ __forceinline__ int floor4(int x) { return x & ~3; }
 
+template <int N>
+struct Int {
+    static constexpr int value = N;
+};
+
 // ---------------------------------------------------------------- strains (one column)
 // NC: compile-time tap count (0 = runtime A.nc); ZIN: every z tap inside the grid;
 // EDGE: x / y guards needed.
@@ -154,7 +183,7 @@ __device__ __forceinline__ void stress_tma_run(const TmapsStress &M, const StepA
                                                const T *tab, bool tab_smem, bool has_dvol,
                                                int bx, int by, int bz)
 {
-    constexpr int PV = pad128<T>(KS_VSZ), PS = pad128<T>(KS_SSZ);
+    constexpr int PV = pad128<T>(KS_VSZ), PS = pad128<T>(KS_SSZ), NS = ks_slots<T>();
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TB_X + tx;
     const int nx = A.nx, ny = A.ny, nz = A.nz;
     const long long sy = A.sy, sz = A.sz;
@@ -176,7 +205,7 @@ __device__ __forceinline__ void stress_tma_run(const TmapsStress &M, const StepA
     auto issue = [&](int i) {
         const int p = q0 + i;
         if (!leader || p > ze) return;
-        const int slot = i % 3;
+        const int slot = i % NS;
         unsigned long long *bar = bars + slot;
         const int ps = p - 1;
         const bool with_s = ps >= zb && ps < ze;
@@ -186,7 +215,7 @@ __device__ __forceinline__ void stress_tma_run(const TmapsStress &M, const StepA
 #pragma unroll
         for (int f = 0; f < 3; ++f) tma_load_3d(dv + f * PV, &M.vt[f], xv, Y0 - T_H, p, bar);
         if (with_s) {
-            T *ds = sslots + (size_t)(((ps - zb) % 3 + 3) % 3) * 7 * PS;
+            T *ds = sslots + (size_t)((ps - zb) % NS) * 7 * PS;
 #pragma unroll
             for (int f = 0; f < 6; ++f) tma_load_3d(ds + f * PS, &M.sc[f], xs, Y0, ps, bar);
             if (has_dvol) tma_load_3d(ds + 6 * PS, &M.dv, xs, Y0, ps, bar);
@@ -222,27 +251,25 @@ __device__ __forceinline__ void stress_tma_run(const TmapsStress &M, const StepA
     uint16_t lab_next = (is_out && zb < nz) ? A.lab[(long long)zb * sz + col] : 0;
     int *status = A.status;
 
-    issue(0);
-    issue(1);
+#pragma unroll
+    for (int i = 0; i < NS - 1; ++i) issue(i);
     const int n_it = ze - q0 + 1;
     for (int i = 0; i < n_it; ++i) {
         const int q = q0 + i;
-        mbar_wait(bars + i % 3, (unsigned)(i / 3) & 1u, status);
-        __syncthreads();   // also: every thread is done with the slot refilled below
-        issue(i + 2);
+        mbar_wait(bars + i % NS, (unsigned)(i / NS) & 1u, status);
         const T nzv = ldcol(pz, q + 4), nyv = ldcol(py, q + 5), nxv = ldcol(px, q + 5);
         const int z = q - 1;
         const uint16_t lab = lab_next;
         if (is_out && z >= zb && q < ze) lab_next = A.lab[(long long)q * sz + col];
         {
-            const T *t = vslots + (size_t)(i % 3) * 3 * PV + tcv;
+            const T *t = vslots + (size_t)(i % NS) * 3 * PV + tcv;
             T g[6];
             const bool zin = q >= T_H && q <= nz - 1 - T_H;
             if (zin) strain_column<T, NC, true, EDGE>(A, q, t, t + PV, t + 2 * PV, KS_VW, rz, ry, rx, xb, xf, yb, yf, g);
             else strain_column<T, NC, false, EDGE>(A, q, t, t + PV, t + 2 * PV, KS_VW, rz, ry, rx, xb, xf, yb, yf, g);
-            T *gw = gs + (size_t)(i % 3) * 6 * TB_N + tid;
+            const int r3 = (q + 3) % 3, r4 = q & 3;   // ring slots of plane q
 #pragma unroll
-            for (int J = 0; J < 6; ++J) gw[J * TB_N] = g[J];
+            for (int J = 0; J < 6; ++J) gs[(ring_base(J) + (ring_planes(J) == 4 ? r4 : r3)) * TB_N + tid] = g[J];
         }
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
@@ -253,42 +280,68 @@ __device__ __forceinline__ void stress_tma_run(const TmapsStress &M, const StepA
         rz[7] = nzv;
         ry[7] = nyv;
         rx[7] = nxv;
+        // strains of q written, the updates of z - 1 done: the one barrier of a
+        // plane; the slots refilled now were last read before it
         __syncthreads();
+        issue(i + NS - 1);
         if (z >= zb && is_out) {
-            // strain planes z-1, z, z+1 were written at iterations i-2, i-1, i
-            const T *gm = gs + (size_t)((i + 1) % 3) * 6 * TB_N + tid;
-            const T *g0 = gs + (size_t)((i + 2) % 3) * 6 * TB_N + tid;
-            const T *gp = gs + (size_t)(i % 3) * 6 * TB_N + tid;
+            // J = 3, 4 at planes z - 1 and z, the others at z and z + 1
+            const T *const p4[2] = {gs + ((z - 1) & 3) * TB_N + tid, gs + (z & 3) * TB_N + tid};
+            const T *const p3[2] = {gs + (z % 3) * TB_N + tid, gs + ((z + 1) % 3) * TB_N + tid};
             auto G = [&](int J, int dz, int dy, int dx) -> T {
-                const T *b = dz < 0 ? gm : (dz > 0 ? gp : g0);
-                return b[J * TB_N + dy * TB_X + dx];
+                const T *b = (J == 3 || J == 4) ? p4[dz + 1] : p3[dz];
+                return b[ring_base(J) * TB_N + dy * TB_X + dx];
             };
             const bool zlo = z >= 1, zhi = z <= nz - 2;
-            T q0v[6], q1v[6], q2v[6], q3v[6];
-            qrow<0>(G, zlo, zhi, ylo, yhi, xlo, xhi, q0v);
-            qrow<1>(G, zlo, zhi, ylo, yhi, xlo, xhi, q1v);
-            qrow<2>(G, zlo, zhi, ylo, yhi, xlo, xhi, q2v);
-            qrow<3>(G, zlo, zhi, ylo, yhi, xlo, xhi, q3v);
-            const T *sc = sslots + (size_t)((z - zb) % 3) * 7 * PS + tcs;
-            T Cm[24];
-            load_c21(tab + (size_t)(lab & LAB_MAT) * C21_STRIDE, tab_smem, Cm);
+            const T *sc = sslots + (size_t)((z - zb) % NS) * 7 * PS + tcs;
+            const T *Cr = tab + (size_t)(lab & LAB_MAT) * C21_STRIDE;
+            T acc[6];
+            if (sizeof(T) == 8 && tab_smem) {
+                // column by column: six constants and four moved strains live at
+                // a time (in FP64 a whole row and all moved strains take 96 registers)
+#pragma unroll
+                for (int I = 0; I < 6; ++I) acc[I] = T(0);
+                auto column = [&](auto j) {
+                    constexpr int J = decltype(j)::value;
+                    const T q0 = qval<0, J, T>(G, zlo, zhi, ylo, yhi, xlo, xhi);
+                    const T q1 = qval<1, J, T>(G, zlo, zhi, ylo, yhi, xlo, xhi);
+                    const T q2 = qval<2, J, T>(G, zlo, zhi, ylo, yhi, xlo, xhi);
+                    const T q3 = qval<3, J, T>(G, zlo, zhi, ylo, yhi, xlo, xhi);
+#pragma unroll
+                    for (int I = 0; I < 6; ++I)
+                        acc[I] = fmac(acc[I], Cr[c21_slot(I, J)], I < 3 ? q0 : (I == 3 ? q1 : (I == 4 ? q2 : q3)));
+                };
+                column(Int<0>());
+                column(Int<1>());
+                column(Int<2>());
+                column(Int<3>());
+                column(Int<4>());
+                column(Int<5>());
+            } else {
+                T q0v[6], q1v[6], q2v[6], q3v[6];
+                qrow<0>(G, zlo, zhi, ylo, yhi, xlo, xhi, q0v);
+                qrow<1>(G, zlo, zhi, ylo, yhi, xlo, xhi, q1v);
+                qrow<2>(G, zlo, zhi, ylo, yhi, xlo, xhi, q2v);
+                qrow<3>(G, zlo, zhi, ylo, yhi, xlo, xhi, q3v);
+                T Cm[24];
+                load_c21(Cr, tab_smem, Cm);
+                acc[0] = row_dot(Cm, 0, q0v);
+                acc[1] = row_dot(Cm, 1, q0v);
+                acc[2] = row_dot(Cm, 2, q0v);
+                acc[3] = row_dot(Cm, 3, q1v);
+                acc[4] = row_dot(Cm, 4, q2v);
+                acc[5] = row_dot(Cm, 5, q3v);
+            }
             float d = 1.0f;
             if (A.dz) {
                 d = A.dz[z] * dyx;
                 d = d * dxx;
             }
             if (has_dvol) {
-                const float dvv = reinterpret_cast<const float *>(sslots + (size_t)((z - zb) % 3) * 7 * PS + 6 * PS)[tcs];
+                const float dvv = reinterpret_cast<const float *>(sslots + (size_t)((z - zb) % NS) * 7 * PS + 6 * PS)[tcs];
                 d = A.dz ? d * dvv : dvv;
             }
             const T dmp = (T)d;
-            T acc[6];
-            acc[0] = row_dot(Cm, 0, q0v);
-            acc[1] = row_dot(Cm, 1, q0v);
-            acc[2] = row_dot(Cm, 2, q0v);
-            acc[3] = row_dot(Cm, 3, q1v);
-            acc[4] = row_dot(Cm, 4, q2v);
-            acc[5] = row_dot(Cm, 5, q3v);
             T sv[6];
 #pragma unroll
             for (int I = 0; I < 6; ++I) {
@@ -328,15 +381,15 @@ __device__ __forceinline__ void stress_tma_block(const TmapsStress &M, const Ste
 {
     unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem);
     T *vslots = reinterpret_cast<T *>(smem + 128);
-    T *sslots = vslots + 3 * (size_t)ks_slot_v<T>();
-    T *gs = sslots + 3 * (size_t)ks_slot_s<T>();
-    T *tsm = gs + (size_t)3 * 6 * TB_N;
+    T *sslots = vslots + ks_slots<T>() * (size_t)ks_slot_v<T>();
+    T *gs = sslots + ks_slots<T>() * (size_t)ks_slot_s<T>();
+    T *tsm = gs + (size_t)RING_PLANES * TB_N;
     const int tid = threadIdx.y * TB_X + threadIdx.x;
     if (tid == 0) {
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
         fence_mbar_init();
     }
-    const bool tab_smem = table_in_smem<T>(n_mat);
+    const bool tab_smem = table_in_smem_tma<T>(n_mat);
     if (tab_smem && load_table)
         for (int i = tid; i < n_mat * C21_STRIDE; i += TB_N) tsm[i] = A.c21[i];
     __syncthreads();
@@ -536,7 +589,7 @@ __device__ __forceinline__ void velocity_tma_block(const TmapsVelocity &M, const
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
         fence_mbar_init();
     }
-    const bool tab_smem = table_in_smem<T>(n_mat);
+    const bool tab_smem = table_in_smem_tma<T>(n_mat);
     if (tab_smem && load_table)
         for (int i = tid; i < n_mat; i += TB_N) rsm[i] = A.rho[i];
     __syncthreads();

@@ -568,9 +568,9 @@ int configure_kernels(PeSolver *S)
     const long long tv = (long long)((c.nx + pe::TB_X - 1) / pe::TB_X) * ((c.ny + pe::TB_Y - 1) / pe::TB_Y);
     int ss = occupancy_slots(pe::k_stress_t<T>, pe::TB_X * pe::TB_Y, need_s);
     int sv = occupancy_slots(pe::k_velocity_t<T>, pe::TB_X * pe::TB_Y, need_v);
-    // TMA path: rows must be whole 16-byte units (box x-origins are multiples of 4 elements)
+    // TMA path: rows must be whole 16-byte units (box x-origins are multiples of 4 elements, of 16 bytes and more)
     const size_t tms = pe::stress_tma_smem<T>(c.n_mat), tmv = pe::velocity_tma_smem<T>(c.n_mat);
-    S->tma_capable = c.nx % 4 == 0 && tms <= (size_t)optin && tmv <= (size_t)optin &&
+    S->tma_capable = c.nx % (16 / (int)sizeof(T)) == 0 && tms <= (size_t)optin && tmv <= (size_t)optin &&
                      encode_fn() != nullptr;
     if (S->tma_capable) {
         PE_CUDA(cudaFuncSetAttribute(pe::k_stress_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
@@ -1497,7 +1497,7 @@ bool pad_shared(const PeBatch *B) { return B->pad_on && B->persistent; }
 bool batched(const PeBatch *B, const PeSolver *S)
 {
     return B->pair_batch ? ((S->pair_capable || (S->padded && pad_shared(B))) && !S->solo)
-                         : (B->tma_batch && S->tma_capable);
+                         : (B->tma_batch && S->tma_capable && S->cfg.nx % 4 == 0);
 }
 
 // Cut the marches of one phase (stress or velocity tiles of the solves taken)
