@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <initializer_list>
 #include <mutex>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -34,10 +35,11 @@
 
 namespace {
 
-constexpr int ENV_T = 128;               // threads per envelope block
-constexpr int ENV_R = 4;                 // outputs per thread (strided by ENV_T)
+constexpr int ENV_T = 64;                // threads per envelope block
+constexpr int ENV_R = 8;                 // outputs per thread
 constexpr int ENV_TILE = ENV_T * ENV_R;  // outputs per block
 constexpr int ENV_KC = 512;              // input samples staged per pass
+constexpr int TAB_B = 8;                 // blocks per tap table
 constexpr int RED_T = 256;               // threads per reduction block
 constexpr int FILT_MAX = 8;              // filter taps (order <= 7)
 constexpr int PAD_MAX = 3 * FILT_MAX;    // scipy's default padlen bound
@@ -57,42 +59,120 @@ __device__ double hilbert_tap(long long j, long long N)
     return ((c - ((m & 1) ? -1.0 : 1.0)) / s) / (double)N;
 }
 
-// One block: ENV_TILE outputs of one trace; the whole trace is swept in
-// ENV_KC-sample passes, the kernel taps a pass needs staged beside them.
-template <typename T>
-__global__ void __launch_bounds__(ENV_T) k_envelope(const T *__restrict__ x, const long long *__restrict__ off,
-                                                    const long long *__restrict__ tiles, double *__restrict__ env)
+// Tap tables g[0 .. N-1] of the distinct lengths of a batch: table k has
+// tabn[k] taps from tab[tabo[k]].
+__global__ void __launch_bounds__(256) k_hilbert_table(const long long *__restrict__ tabn,
+                                                       const long long *__restrict__ tabo, double *__restrict__ tab)
 {
-    __shared__ double xs[ENV_KC];
-    __shared__ double gs[ENV_TILE + ENV_KC - 1];
-    const long long tr = tiles[2 * blockIdx.x], n0 = tiles[2 * blockIdx.x + 1];
-    const long long base = off[tr], N = off[tr + 1] - base;
+    const int k = blockIdx.x / TAB_B;
+    const long long N = tabn[k];
+    double *g = tab + tabo[k];
+    for (long long j = (blockIdx.x % TAB_B) * 256 + threadIdx.x; j < N; j += TAB_B * 256) g[j] = hilbert_tap(j, N);
+}
+
+// shared-memory place of a staged tap: one pad per window, so that lanes whose
+// windows start ENV_R taps apart read different banks
+__device__ __forceinline__ int tap_at(int u) { return u + (unsigned)u / ENV_R; }
+
+// ENV_TILE outputs of one trace from n0 (a multiple of ENV_TILE); the whole
+// trace is swept in ENV_KC-sample passes, the taps a pass needs staged beside
+// its samples. S = 1 (odd N): thread t holds eight consecutive outputs. S = 2
+// (even N): the taps of even offsets are exactly zero, so an output meets only
+// the samples of the other parity; thread t holds eight outputs of parity
+// t & 1. Per sample a thread loads the sample and one new tap of its sliding
+// window for eight fused multiply-adds, in the order of the samples. (One tap
+// and one sample per two multiply-adds, every even offset included, and the
+// taps evaluated again by every block, took 409 us for 36 records of 6000
+// samples.) A skipped product with a sample that is not finite would have been
+// NaN, and is set so.
+template <typename T, int S>
+__device__ __forceinline__ void envelope_tile(const T *__restrict__ x, const double *__restrict__ tab, long long base,
+                                              long long N, long long n0, double *xs, double *gs,
+                                              double *__restrict__ env)
+{
+    constexpr int NI = ENV_KC / S;             // samples an output meets per pass
+    constexpr int NG = ENV_TILE / S + NI - (S == 1 ? 1 : 0);   // taps staged
     const int t = threadIdx.x;
+    const int p = S == 2 ? t & 1 : 0, grp = S == 2 ? t >> 1 : t;
+    const int base_u = ENV_R * grp + NI - 1 + p;
+    const double *xp = xs + (S == 2 ? (1 - p) * (NI + 2) : 0);   // (the pads: other banks)
+    const long long hop = (long long)S * ENV_T % N;
     double acc[ENV_R];
 #pragma unroll
     for (int r = 0; r < ENV_R; ++r) acc[r] = 0.0;
     for (long long k0 = 0; k0 < N; k0 += ENV_KC) {
         __syncthreads();
-        for (int i = t; i < ENV_KC; i += ENV_T) xs[i] = (k0 + i < N) ? rd(x, base + k0 + i) : 0.0;
-        // gs[u] = g[n0 - k0 - (ENV_KC - 1) + u]: output n0 + t + ENV_T r and
-        // input k0 + kk meet at u = t + ENV_T r - kk + ENV_KC - 1
-        const long long j0 = n0 - k0 - (ENV_KC - 1);
-        for (int u = t; u < ENV_TILE + ENV_KC - 1; u += ENV_T) gs[u] = hilbert_tap(j0 + u, N);
-        __syncthreads();
-        const int kmax = (int)((N - k0) < ENV_KC ? (N - k0) : ENV_KC);
-        const double *gp = gs + t + ENV_KC - 1;
-#pragma unroll 4
-        for (int kk = 0; kk < kmax; ++kk) {
-            const double xv = xs[kk];
+        int bad = 0;   // samples that are not finite: bit 0 among the even ones, bit 1 the odd ones
+        for (int i = t; i < ENV_KC; i += ENV_T) {
+            const double v = (k0 + i < N) ? rd(x, base + k0 + i) : 0.0;
+            xs[S == 2 ? (i & 1) * (NI + 2) + (i >> 1) : i] = v;
+            if (S == 2 && !(fabs(v) <= 1.7976931348623157e308)) bad |= 1 << (i & 1);
+        }
+        long long m = (n0 - k0 + (S == 2 ? -1 + 2LL * (t - (NI - 1)) : t - (NI - 1))) % N;
+        if (m < 0) m += N;
+        for (int u = t; u < NG; u += ENV_T) {
+            gs[tap_at(u)] = tab[m];
+            m += hop;
+            if (m >= N) m -= N;
+        }
+        bool skip_bad = false;
+        if (S == 2) {
+            const int b0 = __syncthreads_or(bad & 1), b1 = __syncthreads_or(bad & 2);
+            skip_bad = p ? b1 != 0 : b0 != 0;
+        } else {
+            __syncthreads();
+        }
+        // eight samples at a time: w holds the taps base_u - i0 + r, m the eight
+        // below them, which are the next w in reverse
+        double w[ENV_R];
+        const double *mp[ENV_R];   // their places move down one padded window per eight samples
 #pragma unroll
-            for (int r = 0; r < ENV_R; ++r) acc[r] = fma(xv, gp[r * ENV_T - kk], acc[r]);
+        for (int r = 0; r < ENV_R; ++r) {
+            w[r] = gs[tap_at(base_u + r)];
+            mp[r] = gs + tap_at(base_u - 1 - r);
+        }
+        for (int i0 = 0; i0 < NI; i0 += ENV_R) {
+            double xv[ENV_R], m8[ENV_R];
+#pragma unroll
+            for (int i = 0; i < ENV_R; ++i) {
+                xv[i] = xp[i0 + i];
+                m8[i] = *mp[i];   // the last one of all lies in the pad before gs and is not used
+                mp[i] -= ENV_R + 1;
+            }
+#pragma unroll
+            for (int i = 0; i < ENV_R; ++i)
+#pragma unroll
+                for (int r = 0; r < ENV_R; ++r) acc[r] = fma(xv[i], r >= i ? w[r - i] : m8[i - r - 1], acc[r]);
+#pragma unroll
+            for (int r = 0; r < ENV_R; ++r) w[r] = m8[ENV_R - 1 - r];
+        }
+        if (skip_bad) {
+#pragma unroll
+            for (int r = 0; r < ENV_R; ++r) acc[r] = NAN;
         }
     }
 #pragma unroll
     for (int r = 0; r < ENV_R; ++r) {
-        const long long n = n0 + t + (long long)ENV_T * r;
+        const long long n = n0 + p + (long long)S * (ENV_R * grp + r);
         if (n < N) env[base + n] = hypot(rd(x, base + n), acc[r]);
     }
+}
+
+// One block per tile: tiles holds (trace, first output) pairs, tro the tap
+// table's offset of each trace.
+template <typename T>
+__global__ void __launch_bounds__(ENV_T) k_envelope(const T *__restrict__ x, const long long *__restrict__ off,
+                                                    const long long *__restrict__ tiles,
+                                                    const long long *__restrict__ tro, const double *__restrict__ tab,
+                                                    double *__restrict__ env)
+{
+    __shared__ double xs[ENV_KC + 2];
+    __shared__ double gs_pad[ENV_R + 1 + (ENV_TILE + ENV_KC) / ENV_R * (ENV_R + 1) + 1];
+    double *const gs = gs_pad + ENV_R + 1;
+    const long long tr = tiles[2 * blockIdx.x], n0 = tiles[2 * blockIdx.x + 1];
+    const long long base = off[tr], N = off[tr + 1] - base;
+    if (N & 1) envelope_tile<T, 1>(x, tab + tro[tr], base, N, n0, xs, gs, env);
+    else envelope_tile<T, 2>(x, tab + tro[tr], base, N, n0, xs, gs, env);
 }
 
 struct Filt {
@@ -331,7 +411,7 @@ cudaError_t stage(Staged &s, cudaStream_t st, std::initializer_list<std::pair<co
     size_t at = 0;
     for (auto &q : parts) {
         dst.push_back(a.p + at);
-        if (q.second) {
+        if (q.first && q.second) {   // a part without a source is device scratch
             e = cudaMemcpyAsync(a.p + at, q.first, q.second, cudaMemcpyHostToDevice, st);
             if (e != cudaSuccess) return e;
         }
@@ -369,15 +449,37 @@ extern "C" int pe_trace_envelope(const void *x_dev, int32_t dtype, const int64_t
             tiles.push_back(n0);
         }
     if (tiles.size() / 2 > 0x7fffffffULL) return PE_ERR_UNSUPPORTED;
+    // one tap table per distinct length
+    std::unordered_map<long long, long long> at;
+    std::vector<long long> tabn, tabo, tro;
+    long long taps = 0;
+    for (int i = 0; i < batch; ++i) {
+        const long long n = off[i + 1] - off[i];
+        const auto it = at.emplace(n, taps);
+        if (it.second) {
+            tabn.push_back(n);
+            tabo.push_back(taps);
+            taps += n;
+        }
+        tro.push_back(it.first->second);
+    }
+    if (tabn.size() > 0x7fffffffULL / TAB_B) return PE_ERR_UNSUPPORTED;
     cudaStream_t st = (cudaStream_t)stream;
     Staged s;
     std::vector<void *> d;
-    cudaError_t e = stage(s, st, {{off, sizeof(int64_t) * (batch + 1)}, {tiles.data(), sizeof(long long) * tiles.size()}}, d);
+    const size_t l = sizeof(long long);
+    cudaError_t e = stage(s, st,
+                          {{off, sizeof(int64_t) * (batch + 1)}, {tiles.data(), l * tiles.size()}, {tro.data(), l * batch},
+                           {tabn.data(), l * tabn.size()}, {tabo.data(), l * tabo.size()},
+                           {nullptr, sizeof(double) * (size_t)taps}},
+                          d);
     if (e == cudaSuccess) {
         const unsigned nb = (unsigned)(tiles.size() / 2);
-        const long long *doff = (const long long *)d[0], *dtl = (const long long *)d[1];
-        if (dtype == PE_F32) k_envelope<float><<<nb, ENV_T, 0, st>>>((const float *)x_dev, doff, dtl, env_dev);
-        else k_envelope<double><<<nb, ENV_T, 0, st>>>((const double *)x_dev, doff, dtl, env_dev);
+        const long long *doff = (const long long *)d[0], *dtl = (const long long *)d[1], *dtr = (const long long *)d[2];
+        double *tab = (double *)d[5];
+        k_hilbert_table<<<(unsigned)tabn.size() * TAB_B, 256, 0, st>>>((const long long *)d[3], (const long long *)d[4], tab);
+        if (dtype == PE_F32) k_envelope<float><<<nb, ENV_T, 0, st>>>((const float *)x_dev, doff, dtl, dtr, tab, env_dev);
+        else k_envelope<double><<<nb, ENV_T, 0, st>>>((const double *)x_dev, doff, dtl, dtr, tab, env_dev);
     }
     return finish(e, st);
 }
