@@ -22,6 +22,7 @@
 // computed on the host exactly as the reference's Python computes them.
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <algorithm>
 #include <initializer_list>
 #include <mutex>
@@ -408,15 +409,22 @@ cudaError_t stage(Staged &s, cudaStream_t st, std::initializer_list<std::pair<co
         }
         a.cap = want;
     }
-    size_t at = 0;
+    // one copy for all parts; a part without a source is device scratch, after
+    // the last part with one
+    size_t at = 0, upload = 0;
     for (auto &q : parts) {
         dst.push_back(a.p + at);
-        if (q.first && q.second) {   // a part without a source is device scratch
-            e = cudaMemcpyAsync(a.p + at, q.first, q.second, cudaMemcpyHostToDevice, st);
-            if (e != cudaSuccess) return e;
-        }
+        at += (q.second + 255) & ~size_t(255);
+        if (q.first) upload = at;
+    }
+    std::vector<char> host(upload);
+    at = 0;
+    for (auto &q : parts) {
+        if (q.first && q.second) std::memcpy(host.data() + at, q.first, q.second);
         at += (q.second + 255) & ~size_t(255);
     }
+    // pageable: the source is staged before the call returns
+    if (upload) return cudaMemcpyAsync(a.p, host.data(), upload, cudaMemcpyHostToDevice, st);
     return cudaSuccess;
 }
 

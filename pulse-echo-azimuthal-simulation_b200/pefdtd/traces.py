@@ -51,6 +51,12 @@ def _as_list(xs):
     return [xs]
 
 
+def _flat(x):
+    """A host record as a 1-D array, float32 kept, anything else float64."""
+    a = np.asarray(x)
+    return np.ascontiguousarray((a if a.dtype == np.float32 else a.astype(np.float64)).reshape(-1))
+
+
 class _Packed:
     """Traces packed back to back in one device array (f32 when every
     trace is f32, else f64) with their host offsets."""
@@ -59,23 +65,22 @@ class _Packed:
         xs = _as_list(xs)
         if not xs:
             raise ValueError("no traces")
-        ts = []
-        for x in xs:
-            if isinstance(x, torch.Tensor):
-                t = x.detach().reshape(-1)
-            else:
-                a = np.asarray(x)
-                if a.dtype != np.float32:
-                    a = a.astype(np.float64)
-                t = torch.from_numpy(np.ascontiguousarray(a.reshape(-1)))
-            if t.numel() == 0:
-                raise ValueError("empty trace")
-            ts.append(t)
-        f32 = all(t.dtype == torch.float32 for t in ts)
-        dt = torch.float32 if f32 else torch.float64
-        self.x = torch.cat([t.to(device=dev, dtype=dt) for t in ts]).contiguous()
+        if any(isinstance(x, torch.Tensor) for x in xs):
+            ts = [x.detach().reshape(-1) if isinstance(x, torch.Tensor) else torch.from_numpy(_flat(x)) for x in xs]
+            f32 = all(t.dtype == torch.float32 for t in ts)
+            dt = torch.float32 if f32 else torch.float64
+            lens = [t.numel() for t in ts]
+            x = torch.cat([t.to(device=dev, dtype=dt) for t in ts]).contiguous()
+        else:   # host records: packed on the host, one copy (72 of them cost 1.5 ms)
+            ts = [_flat(x) for x in xs]
+            f32 = all(t.dtype == np.float32 for t in ts)
+            lens = [t.size for t in ts]
+            x = torch.from_numpy(np.concatenate(ts, dtype=np.float32 if f32 else np.float64)).to(dev)
+        if min(lens) == 0:
+            raise ValueError("empty trace")
+        self.x = x
         self.dtype = _capi.PE_F32 if f32 else _capi.PE_F64
-        self.lens = np.array([t.numel() for t in ts], np.int64)
+        self.lens = np.array(lens, np.int64)
         self.off = np.zeros(len(ts) + 1, np.int64)
         np.cumsum(self.lens, out=self.off[1:])
         self.batch = len(ts)
