@@ -40,6 +40,7 @@ struct AdjArgs {
     const T *c21;      // (n_mat, C21_STRIDE)
     const T *rho;
     const float *rinv;  // (n_mat,) RN32(1 / rho) (FP32 solves), or null
+    float neg0;         // -0 (prod2)
     const float *tab36; // (n_mat, 36) column-split stiffness (FP32 solves), or null
     const float *dz, *dy, *dx, *dvol;
     int nz, ny, nx;
@@ -600,17 +601,23 @@ __global__ void k_adj_velfin(AdjArgs<T> A)
 // instructions (k_adj_stress: 1460 per warp, half of them loads and address
 // arithmetic; issue 57-81 %, DRAM 10-31 %). A pair reads every y / z tap as one
 // 64-bit load for both cells, the eight or nine x taps of a row as five, and a
-// moved quantity's row as two, forms differences and sums as paired
-// instructions, and folds the two taps of a coefficient into one difference
-// and one fused multiply-add where the kernels above round four times. On
-// 96x160x160 (one reverse step, us): k_adj_vel 105 -> 88, k_adj_strain 47 ->
-// 31, k_adj_stress 183 -> 135, k_adj_velfin 79 -> 53, k_adj_vel_u 23 -> 18.
+// moved quantity's row as two, and forms products and sums as paired
+// instructions, each lane rounded as the one-cell kernels round: the adjoint
+// fields are the same bit for bit (the gradient to the order of its float64
+// sums). On
+// 96x160x160 (one reverse step, us): k_adj_vel 105 -> 93, k_adj_strain 47 ->
+// 33, k_adj_stress 183 -> 150, k_adj_velfin 79 -> 56, k_adj_vel_u 23 -> 18.
 // Blocks: 16 lanes (32 columns) x 16 rows of one plane. NC: the compile-time
 // tap count (0 = runtime): with it every load of a thread is issued before the
 // first is waited for, where a test per tap split them into nine serial groups.
 constexpr int AP_BX = 32, AP_BY = 16, AP_N = 256;
 
 __device__ __forceinline__ float2 ldp(const float *p) { return ldg2(p); }
+// A product that is rounded before it is added. A paired multiplication
+// followed by a paired addition is contracted to one fused instruction where
+// the assembler sees fit (measured, on some of the sums below), and so is a
+// fused multiply-add of a constant -0; one of a -0 that it cannot know is not.
+__device__ __forceinline__ float2 prod2(const AdjArgs<float> &A, float2 a, float2 b) { return fmac2(bc2(A.neg0), a, b); }
 
 struct PairCell {
     long long i;   // cell 0 (x even)
@@ -654,14 +661,20 @@ __device__ __forceinline__ AdjTapOk adj_tap_ok(int y, int j, int n)
 {
     return {!G || y >= 2 * j + 1, !G || y <= n - 2 * j - 2};
 }
+// one coefficient of DfT / DbT: a + c v1 - c v2, every product and sum rounded,
+// in that order
+__device__ __forceinline__ float2 adj_acc(const AdjArgs<float> &A, float2 a, float2 c, float2 v1, float2 v2)
+{
+    return sub2(add2(a, prod2(A, c, v1)), prod2(A, c, v2));
+}
 // the two taps of coefficient j: DfT (F) reads y - j - 1 and y + j, DbT y - j
 // and y + j + 1; a tap that does not exist is not loaded and counts zero
 template <bool F>
-__device__ __forceinline__ float2 adj_taps(const float *p, long long s, int j, AdjTapOk k)
+__device__ __forceinline__ float2 adj_taps(const AdjArgs<float> &A, float2 a, float2 c, const float *p, long long s, int j, AdjTapOk k)
 {
     const float2 v1 = k.lo ? ldp(p + (F ? -j - 1 : -j) * s) : bc2(0.f);
     const float2 v2 = k.hi ? ldp(p + (F ? j : j + 1) * s) : bc2(0.f);
-    return sub2(v1, v2);
+    return adj_acc(A, a, c, v1, v2);
 }
 // a row's values at columns x - 4 .. x + 5 (off the grid: zero)
 template <bool G>
@@ -677,10 +690,11 @@ __device__ __forceinline__ void adj_row10(const float *p, int ix, int nx, float 
 }
 // adj_taps along x, from such a row
 template <bool F>
-__device__ __forceinline__ float2 adj_taps_x(const float (&W)[10], int j, AdjTapOk k0, AdjTapOk k1)
+__device__ __forceinline__ float2 adj_taps_x(const AdjArgs<float> &A, float2 a, float2 c, const float (&W)[10], int j, AdjTapOk k0, AdjTapOk k1)
 {
     const int lo = 4 + (F ? -j - 1 : -j), hi = 4 + (F ? j : j + 1);
-    return make_float2((k0.lo ? W[lo] : 0.f) - (k0.hi ? W[hi] : 0.f), (k1.lo ? W[lo + 1] : 0.f) - (k1.hi ? W[hi + 1] : 0.f));
+    return adj_acc(A, a, c, make_float2(k0.lo ? W[lo] : 0.f, k1.lo ? W[lo + 1] : 0.f),
+                   make_float2(k0.hi ? W[hi] : 0.f, k1.hi ? W[hi + 1] : 0.f));
 }
 
 __global__ void __launch_bounds__(AP_N) k_adj_vel_u_pair(const AdjArgs<float> A)
@@ -725,9 +739,9 @@ __device__ __forceinline__ void adj_pair_w(const AdjArgs<float> &A, long long i,
     }
     auto put = [&](int p, float2 v) { *reinterpret_cast<float2 *>(A.w[adj_widx(J, p)] + i) = v; };
     if constexpr (J >= 3) {
-        float2 W = mul2(make_float2(a[0].x, a[1].x), e[0]);
-        W = fmac2(W, make_float2(a[0].y, a[1].y), e[1]);
-        put(0, fmac2(W, make_float2(a[0].z, a[1].z), e[2]));
+        float2 W = prod2(A, make_float2(a[0].x, a[1].x), e[0]);
+        W = add2(W, prod2(A, make_float2(a[0].y, a[1].y), e[1]));
+        put(0, add2(W, prod2(A, make_float2(a[0].z, a[1].z), e[2])));
     }
     if constexpr (J != 3) put(1, mul2(make_float2(a[0].w, a[1].w), e[3]));
     if constexpr (J != 4) put(2, mul2(make_float2(b[0].x, b[1].x), e[4]));
@@ -744,23 +758,27 @@ __device__ __forceinline__ void adj_pair_vel(const AdjArgs<float> &A, const Pair
     adj_row10<G>(uy, c.ix, A.nx, Y);
     adj_row10<G>(uz, c.ix, A.nx, Z);
     float2 ls[6] = {bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f)};
+    float2 l3 = bc2(0.f), l4 = bc2(0.f), l5 = bc2(0.f);   // the second derivative of a shear stress
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         if (NC ? j < NC : j < A.nc) {
             const float2 cj = bc2(A.c[j]);
             const AdjTapOk kz = adj_tap_ok<G>(c.iz, j, A.nz), ky = adj_tap_ok<G>(c.iy, j, A.ny);
             const AdjTapOk k0 = adj_tap_ok<G>(c.ix, j, A.nx), k1 = adj_tap_ok<G>(c.ix + 1, j, A.nx);
-            ls[0] = fmac2(ls[0], cj, adj_taps_x<true>(X, j, k0, k1));
-            ls[1] = fmac2(ls[1], cj, adj_taps<true>(uy, sy, j, ky));
-            ls[2] = fmac2(ls[2], cj, adj_taps<true>(uz, sz, j, kz));
-            ls[3] = fmac2(ls[3], cj, adj_taps<false>(uy, sz, j, kz));
-            ls[3] = fmac2(ls[3], cj, adj_taps<false>(uz, sy, j, ky));
-            ls[4] = fmac2(ls[4], cj, adj_taps<false>(ux, sz, j, kz));
-            ls[4] = fmac2(ls[4], cj, adj_taps_x<false>(Z, j, k0, k1));
-            ls[5] = fmac2(ls[5], cj, adj_taps<false>(ux, sy, j, ky));
-            ls[5] = fmac2(ls[5], cj, adj_taps_x<false>(Y, j, k0, k1));
+            ls[0] = adj_taps_x<true>(A, ls[0], cj, X, j, k0, k1);
+            ls[1] = adj_taps<true>(A, ls[1], cj, uy, sy, j, ky);
+            ls[2] = adj_taps<true>(A, ls[2], cj, uz, sz, j, kz);
+            ls[3] = adj_taps<false>(A, ls[3], cj, uy, sz, j, kz);
+            l3 = adj_taps<false>(A, l3, cj, uz, sy, j, ky);
+            ls[4] = adj_taps<false>(A, ls[4], cj, ux, sz, j, kz);
+            l4 = adj_taps_x<false>(A, l4, cj, Z, j, k0, k1);
+            ls[5] = adj_taps<false>(A, ls[5], cj, ux, sy, j, ky);
+            l5 = adj_taps_x<false>(A, l5, cj, Y, j, k0, k1);
         }
     }
+    ls[3] = add2(ls[3], l3);
+    ls[4] = add2(ls[4], l4);
+    ls[5] = add2(ls[5], l5);
     float2 e[6];
 #pragma unroll
     for (int I = 0; I < 6; ++I) {
@@ -861,10 +879,10 @@ __device__ __forceinline__ float2 adj_pair_q(const AdjArgs<float> &A, const Pair
                     acc = add2(acc, v);
                 } else if constexpr (DX > 0) {
                     const float2 w = zy && (!G || c.ix + 2 < A.nx) ? ldp(r + 2) : bc2(0.f);
-                    acc = add2(acc, make_float2(v.x + v.y, v.y + w.x));
+                    acc = add2(add2(acc, v), make_float2(v.y, w.x));
                 } else {
                     const float2 w = zy && (!G || c.ix >= 2) ? ldp(r - 2) : bc2(0.f);
-                    acc = add2(acc, make_float2(w.y + v.x, v.x + v.y));
+                    acc = add2(add2(acc, make_float2(w.y, v.x)), v);
                 }
             }
         acc = mul2(acc, bc2(0.25f));
@@ -887,7 +905,7 @@ __device__ __forceinline__ void adj_pair_grad(const AdjArgs<float> &A, const Pai
             for (int J = 0; J < 6; ++J) {
                 // I <= J: the term's first product (positions ascend with the index)
                 float2 &t = v[c21_slot(I, J)];
-                t = J >= I ? mul2(e[I], q[J]) : fmac2(t, e[I], q[J]);
+                t = J >= I ? prod2(A, e[I], q[J]) : add2(t, prod2(A, e[I], q[J]));
             }
         }
 }
@@ -902,7 +920,7 @@ __device__ __forceinline__ void adj_pair_t(const AdjArgs<float> &A, const PairCe
         const float *w = A.w[adj_widx(J, P)] + c.i;
         // the forward guard of axis offset d at forward position y
         auto ok = [](int y, int d, int n) { return y >= 0 && y < n && (d <= 0 || y <= n - 2) && (d >= 0 || y >= 1); };
-        float2 sum = bc2(0.f);
+        const float2 quarter = bc2(0.25f);
 #pragma unroll
         for (int a0 = (DZ < 0 ? -1 : 0); a0 <= (DZ > 0 ? 1 : 0); ++a0)
 #pragma unroll
@@ -911,7 +929,7 @@ __device__ __forceinline__ void adj_pair_t(const AdjArgs<float> &A, const PairCe
                 const float *r = w - a0 * A.sz - a1 * A.sy;
                 float2 v = zy ? ldp(r) : bc2(0.f);
                 if constexpr (DX == 0) {
-                    sum = add2(sum, v);
+                    acc = add2(acc, prod2(A, quarter, v));
                 } else {
                     // the pair and its neighbour on the side of the taps; of the
                     // forward cells in the grid the x guard drops only the last
@@ -919,10 +937,25 @@ __device__ __forceinline__ void adj_pair_t(const AdjArgs<float> &A, const PairCe
                     const bool in = zy && (!G || (DX > 0 ? c.ix >= 2 : c.ix + 2 < A.nx));
                     const float2 o = in ? ldp(DX > 0 ? r - 2 : r + 2) : bc2(0.f);
                     if constexpr (G) v = keep2(v, DX > 0 || c.ix >= 1, DX < 0 || c.ix + 1 <= A.nx - 2);
-                    sum = add2(sum, DX > 0 ? make_float2(o.y + v.x, v.x + v.y) : make_float2(v.x + v.y, v.y + o.x));
+                    const float2 n = DX > 0 ? make_float2(o.y, v.x) : make_float2(v.y, o.x);
+                    acc = add2(acc, prod2(A, quarter, DX > 0 ? v : n));
+                    acc = add2(acc, prod2(A, quarter, DX > 0 ? n : v));
                 }
             }
-        acc = fmac2(acc, bc2(0.25f), sum);
+    }
+}
+// the contribution of position P to t_J: the direct terms at J's own position
+template <int J, int P, bool G>
+__device__ __forceinline__ void adj_pair_tP(const AdjArgs<float> &A, const PairCell &c, const float *const (&row)[2],
+                                            const float2 (&e)[6], float2 &acc)
+{
+    if constexpr (P == vpos(J)) {
+#pragma unroll
+        for (int I = 0; I < 6; ++I)
+            if (vpos(I) == P)
+                acc = add2(acc, prod2(A, make_float2(__ldg(row[0] + c21_slot(I, J)), __ldg(row[1] + c21_slot(I, J))), e[I]));
+    } else {
+        adj_pair_t<J, P, G>(A, c, acc);
     }
 }
 template <int J, bool G>
@@ -930,14 +963,10 @@ __device__ __forceinline__ void adj_pair_tJ(const AdjArgs<float> &A, const PairC
                                             const float2 (&e)[6])
 {
     float2 acc = bc2(0.f);
-#pragma unroll
-    for (int I = 0; I < 6; ++I)
-        if (vpos(I) == vpos(J))
-            acc = fmac2(acc, make_float2(__ldg(row[0] + c21_slot(I, J)), __ldg(row[1] + c21_slot(I, J))), e[I]);
-    adj_pair_t<J, 0, G>(A, c, acc);
-    adj_pair_t<J, 1, G>(A, c, acc);
-    adj_pair_t<J, 2, G>(A, c, acc);
-    adj_pair_t<J, 3, G>(A, c, acc);
+    adj_pair_tP<J, 0, G>(A, c, row, e, acc);
+    adj_pair_tP<J, 1, G>(A, c, row, e, acc);
+    adj_pair_tP<J, 2, G>(A, c, row, e, acc);
+    adj_pair_tP<J, 3, G>(A, c, row, e, acc);
     *reinterpret_cast<float2 *>(A.t[J] + c.i) = acc;
 }
 template <bool G>
@@ -952,7 +981,7 @@ __device__ __forceinline__ void adj_pair_strain_adjoint(const AdjArgs<float> &A,
     adj_pair_tJ<5, G>(A, c, row, e);
 }
 
-__global__ void __launch_bounds__(AP_N, 3) k_adj_stress_pair(const AdjArgs<float> A)
+__global__ void __launch_bounds__(AP_N, 2) k_adj_stress_pair(const AdjArgs<float> A)
 {
     // k_adj_stress's per-material sums over the 64 cells of a warp: row
     // 32 c + lane of the tile holds the terms of cell c of a lane
@@ -1041,30 +1070,32 @@ __device__ __forceinline__ void adj_pair_velfin(const AdjArgs<float> &A, const P
     adj_row10<G>(t1, c.ix, A.nx, X);
     adj_row10<G>(t6, c.ix, A.nx, Y);
     adj_row10<G>(t5, c.ix, A.nx, Z);
-    float2 gx = bc2(0.f), gy = bc2(0.f), gz = bc2(0.f);
+    float2 g[9];   // three derivatives each of gx, gy, gz
+#pragma unroll
+    for (int k = 0; k < 9; ++k) g[k] = bc2(0.f);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         if (NC ? j < NC : j < A.nc) {
             const float2 cj = bc2(A.c[j]);
             const AdjTapOk kz = adj_tap_ok<G>(c.iz, j, A.nz), ky = adj_tap_ok<G>(c.iy, j, A.ny);
             const AdjTapOk k0 = adj_tap_ok<G>(c.ix, j, A.nx), k1 = adj_tap_ok<G>(c.ix + 1, j, A.nx);
-            gx = fmac2(gx, cj, adj_taps_x<false>(X, j, k0, k1));
-            gx = fmac2(gx, cj, adj_taps<true>(t5, sz, j, kz));
-            gx = fmac2(gx, cj, adj_taps<true>(t6, sy, j, ky));
-            gy = fmac2(gy, cj, adj_taps<false>(t2, sy, j, ky));
-            gy = fmac2(gy, cj, adj_taps<true>(t4, sz, j, kz));
-            gy = fmac2(gy, cj, adj_taps_x<true>(Y, j, k0, k1));
-            gz = fmac2(gz, cj, adj_taps<false>(t3, sz, j, kz));
-            gz = fmac2(gz, cj, adj_taps<true>(t4, sy, j, ky));
-            gz = fmac2(gz, cj, adj_taps_x<true>(Z, j, k0, k1));
+            g[0] = adj_taps_x<false>(A, g[0], cj, X, j, k0, k1);
+            g[1] = adj_taps<true>(A, g[1], cj, t5, sz, j, kz);
+            g[2] = adj_taps<true>(A, g[2], cj, t6, sy, j, ky);
+            g[3] = adj_taps<false>(A, g[3], cj, t2, sy, j, ky);
+            g[4] = adj_taps<true>(A, g[4], cj, t4, sz, j, kz);
+            g[5] = adj_taps_x<true>(A, g[5], cj, Y, j, k0, k1);
+            g[6] = adj_taps<false>(A, g[6], cj, t3, sz, j, kz);
+            g[7] = adj_taps<true>(A, g[7], cj, t4, sy, j, ky);
+            g[8] = adj_taps_x<true>(A, g[8], cj, Z, j, k0, k1);
         }
     }
     const float2 d = adj_pair_damp(A, c), ih = bc2(A.inv_h);
-    const float2 r[3] = {gx, gy, gz};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         float2 *q = reinterpret_cast<float2 *>(A.lv[k] + i);
-        *q = fmac2(mul2(ih, r[k]), d, *q);
+        const float2 r = add2(add2(g[3 * k], g[3 * k + 1]), g[3 * k + 2]);
+        *q = add2(prod2(A, d, *q), prod2(A, ih, r));
     }
 }
 template <int NC>

@@ -1069,6 +1069,7 @@ int adjoint_step_t(PeSolver *S, const PeAdjoint *adj, int64_t n, const void *res
     A.rho = (const T *)S->rho;
     A.rinv = S->rinv;
     A.tab36 = S->tab36;
+    A.neg0 = -0.0f;
     A.dz = S->dz;
     A.dy = S->dy;
     A.dx = S->dx;
