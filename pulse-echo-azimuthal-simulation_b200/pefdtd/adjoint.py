@@ -107,13 +107,35 @@ class AdjointSolve:
         self.torch = solve.torch
         self.ckpt = {}
         self.nt = 0
+        # where buffers come from when the work runs on a side stream (None: the current stream's pool)
+        self.alloc_stream = None
+
+    def _new(self, shape, dtype, zero=False):
+        """A device buffer for the current stream. With alloc_stream set its
+        memory comes from that stream's pool: the caching allocator keeps a
+        pool per stream, and a side stream that lives for one call would
+        allocate from the driver each time (cudaMalloc synchronises the device)
+        and leave its pool behind."""
+        torch = self.torch
+        dev = self.solve.device
+        make = torch.zeros if zero else torch.empty
+        cur = torch.cuda.current_stream(dev)
+        if self.alloc_stream is None or self.alloc_stream == cur:
+            return make(shape, dtype=dtype, device=dev)
+        with torch.cuda.stream(self.alloc_stream):
+            t = torch.empty(shape, dtype=dtype, device=dev)
+        # its former user's work, then this stream's; not handed on before this
+        # stream has passed the point where it is freed
+        cur.wait_stream(self.alloc_stream)
+        t.record_stream(cur)
+        return t.zero_() if zero else t
 
     def _save(self, state):
         if self.offload:
             h = self.torch.empty(state.shape, dtype=state.dtype, device="cpu", pin_memory=True)
             h.copy_(state, non_blocking=True)   # stream-ordered before the next steps
             return h
-        return state.clone()
+        return self._new(state.shape, state.dtype).copy_(state)
 
     def forward(self, nt=None):
         """Traces (nt, n_groups) as a device tensor; keeps checkpoints."""
@@ -160,10 +182,10 @@ class AdjointSolve:
             res = torch.as_tensor(np.asarray(residual), dtype=tdt).reshape(nt, ng).to(dev).contiguous()
         L = _bind()
         with torch.cuda.device(dev):
-            lam = torch.zeros((9,) + shape, dtype=tdt, device=dev)
-            scratch = torch.zeros((33,) + shape, dtype=tdt, device=dev)
-            grad = torch.zeros((s.cfg.n_mat, 21), dtype=torch.float64, device=dev)
-            hist = torch.empty((min(self.m, nt), 3) + shape, dtype=tdt, device=dev)
+            lam = self._new((9,) + shape, tdt, zero=True)
+            scratch = self._new((33,) + shape, tdt)   # every field is written before it is read
+            grad = self._new((s.cfg.n_mat, 21), torch.float64, zero=True)
+            hist = self._new((min(self.m, nt), 3) + shape, tdt)
         adj = _PeAdjoint()
         for i in range(3):
             adj.lv[i] = lam[i].data_ptr()
@@ -189,7 +211,7 @@ class AdjointSolve:
                 # then the sub-segments last first, m steps of history each
                 inner = {}
                 for a2 in range(a, b, self.m):
-                    inner[a2] = s.state.clone()
+                    inner[a2] = self._new(s.state.shape, s.state.dtype).copy_(s.state)
                     s.run(a2, min(a2 + self.m, b))
                 for a2 in reversed(sorted(inner)):
                     s.state.copy_(inner[a2])
@@ -269,7 +291,8 @@ def _misfit_gradients_wave(problems, c21s, dobs, opts):
             adjs.append(p.make_adjoint(np.asarray(c, float), inner_every=inner, offload=off))
         streams = [torch.cuda.Stream(device=a.solve.device) for a in adjs]
         for st, a in zip(streams, adjs):
-            st.wait_stream(torch.cuda.current_stream(a.solve.device))
+            a.alloc_stream = torch.cuda.current_stream(a.solve.device)
+            st.wait_stream(a.alloc_stream)
 
         def interleave(jobs):
             live = list(jobs)
