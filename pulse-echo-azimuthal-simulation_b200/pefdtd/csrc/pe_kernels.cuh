@@ -439,7 +439,18 @@ __global__ void k_reduce_traces(const T *rec_val, const T *rec_w, const long lon
     const int k = t / n_groups, g = t % n_groups;
     const T *val = rec_val + (long long)k * n_rec;
     T acc = 0;
-    for (long long e = grp_off[g]; e < grp_off[g + 1]; ++e) {
+    // eight entries' loads in flight ahead of their ordered sums (one at a time
+    // a group of 3200 cells took 274 us a chunk, a load's latency per entry)
+    long long e = grp_off[g];
+    const long long e1 = grp_off[g + 1];
+    for (; e + 8 <= e1; e += 8) {
+        T prod[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) prod[i] = val[e + i] * rec_w[e + i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc = acc + prod[i];
+    }
+    for (; e < e1; ++e) {
         const T prod = val[e] * rec_w[e];
         acc = acc + prod;
     }

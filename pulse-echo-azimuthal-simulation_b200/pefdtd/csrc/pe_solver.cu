@@ -170,7 +170,7 @@ struct PeSolver {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
     cudaGraphExec_t gexec = nullptr;
-    PeState gstate{};
+    PeState gstate{};           // state and traces of the graph, or of a first chunk launched without one
     void *gtraces = nullptr;
     int chunk = 200;
     int tx = 32, ty = 8;        // simple-kernel tile
@@ -1003,12 +1003,19 @@ int pe_solver_run(PeSolver *S, const PeState *state, void *traces, int64_t b, in
     int64_t n = b;
     while (n < e) {
         const int len = (int)std::min<int64_t>(S->chunk, e - n);
-        if (len == S->chunk) {
-            if (!S->gexec || !same_state(S->gstate, *use) || S->gtraces != traces) {
-                if (S->gexec) {
-                    cudaGraphExecDestroy(S->gexec);
-                    S->gexec = nullptr;
-                }
+        if (len == S->chunk && !(same_state(S->gstate, *use) && S->gtraces == traces)) {
+            // the first chunk on these buffers goes out as plain launches: the
+            // GPU works while a second one captures and instantiates the graph
+            // (1-2 ms for 400 launches), and a solve of one chunk never does
+            if (S->gexec) {
+                cudaGraphExecDestroy(S->gexec);
+                S->gexec = nullptr;
+            }
+            S->gstate = *use;
+            S->gtraces = traces;
+            if ((rc = launch_chunk(S, use, traces, len))) return rc;
+        } else if (len == S->chunk) {
+            if (!S->gexec) {
                 cudaGraph_t g = nullptr;
                 PE_CUDA(cudaStreamBeginCapture(S->stream, cudaStreamCaptureModeThreadLocal));
                 const long long before = S->launches;
@@ -1020,8 +1027,6 @@ int pe_solver_run(PeSolver *S, const PeState *state, void *traces, int64_t b, in
                 ce = cudaGraphInstantiate(&S->gexec, g, 0);
                 cudaGraphDestroy(g);
                 if (ce != cudaSuccess) return fail(PE_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
-                S->gstate = *use;
-                S->gtraces = traces;
             }
             PE_CUDA(cudaGraphLaunch(S->gexec, S->stream));
             S->launches += 2LL * len + (S->n_groups > 0 ? 1 : 0) + 1;
