@@ -169,16 +169,6 @@ __device__ __forceinline__ float2 ld2_column(const float *p)
     else return ldg2_stream(p);
 }
 
-// Programmatic dependent launch: the step kernels follow one another with
-// nothing between them, so each is launched while its predecessor's last
-// blocks still run, sets up its block (barriers, table, pads: nothing a kernel
-// writes) and only then waits for the predecessor to have finished and its
-// writes to be visible. pdl_release lets the successor be launched; no-ops in
-// an ordinary launch. The column loads are L2-coherent (COH) in these
-// launches: the read-only path is for data nothing writes during the launch.
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
 // ======================================================================== stress
 // Tap limits near the grid faces. The reference skips a tap whose reach
 // leaves the grid (sim/core/fdtd.py:1141-1162, :1215-1236): tap j of a

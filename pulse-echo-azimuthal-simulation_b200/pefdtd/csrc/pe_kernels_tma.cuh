@@ -138,6 +138,16 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 
 __device__ __forceinline__ int floor4(int x) { return x & ~3; }
 
+// Programmatic dependent launch: the step kernels follow one another with
+// nothing between them, so each is launched while its predecessor's last
+// blocks still run, sets up its block (barriers, table, pads: nothing a kernel
+// writes) and only then waits for the predecessor to have finished and its
+// writes to be visible. pdl_release lets the successor be launched; no-ops in
+// an ordinary launch. The column loads are L2-coherent (COH) in these
+// launches: the read-only path is for data nothing writes during the launch.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 template <int N>
 struct Int {
     static constexpr int value = N;
@@ -224,7 +234,7 @@ __device__ __forceinline__ void stress_tma_run(const TmapsStress &M, const StepA
     // column loads for the z rings: running pointers, one plane ahead
     const T *pz = A.v[2] + col, *py = A.v[1] + col, *px = A.v[0] + col;
     auto ldcol = [&](const T *f, int q) -> T {
-        return (col_ok && q >= 0 && q < nz) ? ldg(f + (long long)q * sz) : T(0);
+        return (col_ok && q >= 0 && q < nz) ? __ldcg(f + (long long)q * sz) : T(0);
     };
     T rz[8], ry[8], rx[8];   // rz[k] <-> plane q-4+k, ry/rx[k] <-> q-3+k
 #pragma unroll
@@ -393,6 +403,7 @@ __device__ __forceinline__ void stress_tma_block(const TmapsStress &M, const Ste
     if (tab_smem && load_table)
         for (int i = tid; i < n_mat * C21_STRIDE; i += TB_N) tsm[i] = A.c21[i];
     __syncthreads();
+    pdl_wait();
     const T *tab = tab_smem ? tsm : A.c21;
     const bool has_dvol = A.dvol != nullptr;
     const int X0 = bx * TS_OX - 1, Y0 = by * TS_OY - 1;
@@ -411,6 +422,7 @@ __global__ void __launch_bounds__(TB_N, 1) k_stress_tma(const __grid_constant__ 
                                                         const StepArgs<T> A, int n_mat)
 {
     extern __shared__ __align__(128) unsigned char smem_tma[];
+    pdl_release();
     stress_tma_block<T>(M, A, n_mat, smem_tma, blockIdx.x, blockIdx.y, blockIdx.z, true);
 }
 
@@ -481,7 +493,7 @@ __device__ __forceinline__ void velocity_tma_run(const TmapsVelocity &M, const S
     };
     const T *p3 = A.s[2] + col, *p4 = A.s[3] + col, *p5 = A.s[4] + col;
     auto ldcol = [&](const T *f, int z) -> T {
-        return (out_ok && z >= 0 && z < nz) ? ldg(f + (long long)z * sz) : T(0);
+        return (out_ok && z >= 0 && z < nz) ? __ldcg(f + (long long)z * sz) : T(0);
     };
     auto ldlab = [&](long long i, bool ok) -> uint16_t { return ok ? A.lab[i] : (uint16_t)0; };
 
@@ -593,6 +605,7 @@ __device__ __forceinline__ void velocity_tma_block(const TmapsVelocity &M, const
     if (tab_smem && load_table)
         for (int i = tid; i < n_mat; i += TB_N) rsm[i] = A.rho[i];
     __syncthreads();
+    pdl_wait();
     const T *rho_tab = tab_smem ? rsm : A.rho;
     const bool has_dvol = A.dvol != nullptr;
     const int x0 = bx * TB_X, y0 = by * TB_Y;
@@ -611,6 +624,7 @@ __global__ void __launch_bounds__(TB_N, 1) k_velocity_tma(const __grid_constant_
                                                           const StepArgs<T> A, int n_mat)
 {
     extern __shared__ __align__(128) unsigned char smem_tma[];
+    pdl_release();
     velocity_tma_block<T>(M, A, n_mat, smem_tma, blockIdx.x, blockIdx.y, blockIdx.z, true);
 }
 

@@ -291,11 +291,11 @@ void launch_simple_velocity(pe::StepArgs<T> A, int zc, cudaStream_t st)
 // launch that may start while its predecessor on the stream still drains
 // (programmatic dependent launch; the kernel waits before it reads a field)
 template <typename... P, typename... Q>
-void launch_chained(void (*fn)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, Q... args)
+void launch_chained(void (*fn)(P...), dim3 grid, dim3 threads, size_t smem, cudaStream_t st, Q... args)
 {
     cudaLaunchConfig_t lc = {};
     lc.gridDim = grid;
-    lc.blockDim = dim3((unsigned)threads, 1, 1);
+    lc.blockDim = threads;
     lc.dynamicSmemBytes = smem;
     lc.stream = st;
     cudaLaunchAttribute at[1];
@@ -339,8 +339,8 @@ void launch_stress(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t st
     dim3 grid((A.nx + pe::TS_OX - 1) / pe::TS_OX, (A.ny + pe::TS_OY - 1) / pe::TS_OY,
               (A.nz + A.zc - 1) / A.zc);
     if (S->tma) {
-        pe::k_stress_tma<T><<<grid, dim3(pe::TB_X, pe::TB_Y, 1), pe::stress_tma_smem<T>(S->cfg.n_mat), st>>>(
-            S->ms, A, S->cfg.n_mat);
+        launch_chained(pe::k_stress_tma<T>, grid, dim3(pe::TB_X, pe::TB_Y, 1), pe::stress_tma_smem<T>(S->cfg.n_mat), st,
+                       S->ms, A, S->cfg.n_mat);
         return;
     }
     pe::k_stress_t<T><<<grid, dim3(pe::TB_X, pe::TB_Y, 1), pe::stress_tiled_smem<T>(S->cfg.n_mat), st>>>(
@@ -378,8 +378,8 @@ void launch_velocity(const PeSolver *S, const pe::StepArgs<T> &A0, cudaStream_t 
     dim3 grid((A.nx + pe::TB_X - 1) / pe::TB_X, (A.ny + pe::TB_Y - 1) / pe::TB_Y,
               (A.nz + A.zc - 1) / A.zc);
     if (S->tma) {
-        pe::k_velocity_tma<T><<<grid, dim3(pe::TB_X, pe::TB_Y, 1), pe::velocity_tma_smem<T>(S->cfg.n_mat),
-                                 st>>>(S->mv, A, S->cfg.n_mat);
+        launch_chained(pe::k_velocity_tma<T>, grid, dim3(pe::TB_X, pe::TB_Y, 1), pe::velocity_tma_smem<T>(S->cfg.n_mat),
+                       st, S->mv, A, S->cfg.n_mat);
         return;
     }
     pe::k_velocity_t<T><<<grid, dim3(pe::TB_X, pe::TB_Y, 1), pe::velocity_tiled_smem<T>(S->cfg.n_mat),
