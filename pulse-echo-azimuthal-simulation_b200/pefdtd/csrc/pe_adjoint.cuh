@@ -75,14 +75,14 @@ __device__ __forceinline__ float adj_damp(const AdjArgs<T> &A, int iz, int iy, i
 // load is independent of the guards, so the gathers of a cell overlap.
 // G: evaluate the guards (false where the caller has established that every
 // tap of the cell along this axis exists: adj_block_inside, adj_inside_x,
-// adj_inside_yz).
-template <typename T, bool G = true, typename F>
+// adj_inside_yz). NC: the compile-time tap count, 0 = nc.
+template <typename T, int NC, bool G = true, typename F>
 __device__ __forceinline__ T DfT(const F &f, int y, int n, const T c[4], int nc)
 {
     T a = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (j < nc) {
+        if (NC ? j < NC : j < nc) {
             const bool p1 = !G || gF(y - j - 1, j, n), p2 = !G || gF(y + j, j, n);
             const T v1 = f(p1 ? -j - 1 : 0), v2 = f(p2 ? j : 0);
             a += c[j] * (p1 ? v1 : T(0));
@@ -91,13 +91,13 @@ __device__ __forceinline__ T DfT(const F &f, int y, int n, const T c[4], int nc)
     }
     return a;
 }
-template <typename T, bool G = true, typename F>
+template <typename T, int NC, bool G = true, typename F>
 __device__ __forceinline__ T DbT(const F &f, int y, int n, const T c[4], int nc)
 {
     T a = 0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (j < nc) {
+        if (NC ? j < NC : j < nc) {
             const bool p1 = !G || gB(y - j, j, n), p2 = !G || gB(y + j + 1, j, n);
             const T v1 = f(p1 ? -j : 0), v2 = f(p2 ? j + 1 : 0);
             a += c[j] * (p1 ? v1 : T(0));
@@ -163,14 +163,14 @@ __device__ __forceinline__ bool adj_inside_yz(const AdjArgs<T> &A)
     return y0 >= ADJ_MARGIN_LO && y0 + ADJ_BY - 1 <= A.ny - ADJ_MARGIN_HI && z >= ADJ_MARGIN_LO &&
            z <= A.nz - ADJ_MARGIN_HI;
 }
-// f<T, GX, GYZ>(args...) for this block's classification (block-uniform)
+// f<T, NC, GX, GYZ>(args...) for this block's classification (block-uniform)
 #define ADJ_DISPATCH(A, f, ...)                                          \
     do {                                                                 \
         const bool in_x_ = adj_inside_x(A), in_yz_ = adj_inside_yz(A);   \
-        if (in_x_ && in_yz_) f<T, false, false>(__VA_ARGS__);            \
-        else if (in_x_) f<T, false, true>(__VA_ARGS__);                  \
-        else if (in_yz_) f<T, true, false>(__VA_ARGS__);                 \
-        else f<T, true, true>(__VA_ARGS__);                              \
+        if (in_x_ && in_yz_) f<T, NC, false, false>(__VA_ARGS__);            \
+        else if (in_x_) f<T, NC, false, true>(__VA_ARGS__);                  \
+        else if (in_yz_) f<T, NC, true, false>(__VA_ARGS__);                 \
+        else f<T, NC, true, true>(__VA_ARGS__);                              \
     } while (0)
 
 // ---------------------------------------------------------------- receivers
@@ -263,7 +263,7 @@ __device__ __forceinline__ void adj_w_cell(const AdjArgs<T> &A, long long i, con
         }
 }
 
-template <typename T, bool GX, bool GYZ>
+template <typename T, int NC, bool GX, bool GYZ>
 __device__ __forceinline__ void adj_vel_cell(const AdjArgs<T> &A, long long i, int iz, int iy, int ix)
 {
     const long long sy = A.sy, sz = A.sz;
@@ -272,19 +272,19 @@ __device__ __forceinline__ void adj_vel_cell(const AdjArgs<T> &A, long long i, i
     auto Y = [&](const T *p) { return [p, sy](int o) { return p[o * sy]; }; };
     auto Z = [&](const T *p) { return [p, sz](int o) { return p[o * sz]; }; };
     T ls[6];
-    ls[0] = A.ls[0][i] + DfT<T, GX>(X(ux), ix, A.nx, A.c, A.nc);
-    ls[1] = A.ls[1][i] + DfT<T, GYZ>(Y(uy), iy, A.ny, A.c, A.nc);
-    ls[2] = A.ls[2][i] + DfT<T, GYZ>(Z(uz), iz, A.nz, A.c, A.nc);
-    ls[3] = A.ls[3][i] + (DbT<T, GYZ>(Z(uy), iz, A.nz, A.c, A.nc) + DbT<T, GYZ>(Y(uz), iy, A.ny, A.c, A.nc));
-    ls[4] = A.ls[4][i] + (DbT<T, GYZ>(Z(ux), iz, A.nz, A.c, A.nc) + DbT<T, GX>(X(uz), ix, A.nx, A.c, A.nc));
-    ls[5] = A.ls[5][i] + (DbT<T, GYZ>(Y(ux), iy, A.ny, A.c, A.nc) + DbT<T, GX>(X(uy), ix, A.nx, A.c, A.nc));
+    ls[0] = A.ls[0][i] + DfT<T, NC, GX>(X(ux), ix, A.nx, A.c, A.nc);
+    ls[1] = A.ls[1][i] + DfT<T, NC, GYZ>(Y(uy), iy, A.ny, A.c, A.nc);
+    ls[2] = A.ls[2][i] + DfT<T, NC, GYZ>(Z(uz), iz, A.nz, A.c, A.nc);
+    ls[3] = A.ls[3][i] + (DbT<T, NC, GYZ>(Z(uy), iz, A.nz, A.c, A.nc) + DbT<T, NC, GYZ>(Y(uz), iy, A.ny, A.c, A.nc));
+    ls[4] = A.ls[4][i] + (DbT<T, NC, GYZ>(Z(ux), iz, A.nz, A.c, A.nc) + DbT<T, NC, GX>(X(uz), ix, A.nx, A.c, A.nc));
+    ls[5] = A.ls[5][i] + (DbT<T, NC, GYZ>(Y(ux), iy, A.ny, A.c, A.nc) + DbT<T, NC, GX>(X(uy), ix, A.nx, A.c, A.nc));
 #pragma unroll
     for (int I = 0; I < 6; ++I) A.ls[I][i] = ls[I];
     adj_w_cell(A, i, ls);   // this cell's ls is final for the step until k_adj_stress damps it
 }
 // eight 256-thread blocks per SM in FP32 (32 registers, no spills; the
 // stiffness columns formed at the end would otherwise take it to 40)
-template <typename T>
+template <typename T, int NC>
 __global__ void __launch_bounds__(ADJ_BX * ADJ_BY, sizeof(T) == 4 ? 8 : 4) k_adj_vel(AdjArgs<T> A)
 {
     long long i;
@@ -292,12 +292,12 @@ __global__ void __launch_bounds__(ADJ_BX * ADJ_BY, sizeof(T) == 4 ? 8 : 4) k_adj
     if (!adj_cell(A, i, iz, iy, ix)) return;
     // two instantiations (all guards or none): the four of ADJ_DISPATCH
     // measured slower here (more registers)
-    if (adj_inside_x(A) && adj_inside_yz(A)) adj_vel_cell<T, false, false>(A, i, iz, iy, ix);
-    else adj_vel_cell<T, true, true>(A, i, iz, iy, ix);
+    if (adj_inside_x(A) && adj_inside_yz(A)) adj_vel_cell<T, NC, false, false>(A, i, iz, iy, ix);
+    else adj_vel_cell<T, NC, true, true>(A, i, iz, iy, ix);
 }
 
 // ---------------------------------------------------------------- strains of v^{n-1}
-template <typename T, bool GX, bool GYZ>
+template <typename T, int NC, bool GX, bool GYZ>
 __device__ __forceinline__ void adj_strain_cell(const AdjArgs<T> &A, long long i, int iz, int iy, int ix)
 {
     const long long sy = A.sy, sz = A.sz;
@@ -310,7 +310,7 @@ __device__ __forceinline__ void adj_strain_cell(const AdjArgs<T> &A, long long i
     };
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        if (j < A.nc) {
+        if (NC ? j < NC : j < A.nc) {
             const T cj = A.c[j];
             const bool bx = !GX || gB(ix, j, A.nx), by = !GYZ || gB(iy, j, A.ny), bz = !GYZ || gB(iz, j, A.nz);
             const bool fx = !GX || gF(ix, j, A.nx), fy = !GYZ || gF(iy, j, A.ny), fz = !GYZ || gF(iz, j, A.nz);
@@ -329,7 +329,7 @@ __device__ __forceinline__ void adj_strain_cell(const AdjArgs<T> &A, long long i
     A.g[0][i] = a1 * ih; A.g[1][i] = a2 * ih; A.g[2][i] = a3 * ih;
     A.g[3][i] = a4 * ih; A.g[4][i] = a5 * ih; A.g[5][i] = a6 * ih;
 }
-template <typename T>
+template <typename T, int NC>
 __global__ void k_adj_strain(AdjArgs<T> A)
 {
     long long i;
@@ -563,7 +563,7 @@ __global__ void k_grad_fold(double *rep, int nrep, long long len, double *grad)
     grad[i] += s;
 }
 
-template <typename T, bool GX, bool GYZ>
+template <typename T, int NC, bool GX, bool GYZ>
 __device__ __forceinline__ void adj_velfin_cell(const AdjArgs<T> &A, long long i, int iz, int iy, int ix)
 {
     const long long sy = A.sy, sz = A.sz;
@@ -574,17 +574,17 @@ __device__ __forceinline__ void adj_velfin_cell(const AdjArgs<T> &A, long long i
     const T *t4 = A.t[3] + i, *t5 = A.t[4] + i, *t6 = A.t[5] + i;
     const T d = (T)adj_damp(A, iz, iy, ix, i);
     const T ih = A.inv_h;
-    const T gx = DbT<T, GX>(X(t1), ix, A.nx, A.c, A.nc) + DfT<T, GYZ>(Z(t5), iz, A.nz, A.c, A.nc) +
-                 DfT<T, GYZ>(Y(t6), iy, A.ny, A.c, A.nc);
-    const T gy = DbT<T, GYZ>(Y(t2), iy, A.ny, A.c, A.nc) + DfT<T, GYZ>(Z(t4), iz, A.nz, A.c, A.nc) +
-                 DfT<T, GX>(X(t6), ix, A.nx, A.c, A.nc);
-    const T gz = DbT<T, GYZ>(Z(t3), iz, A.nz, A.c, A.nc) + DfT<T, GYZ>(Y(t4), iy, A.ny, A.c, A.nc) +
-                 DfT<T, GX>(X(t5), ix, A.nx, A.c, A.nc);
+    const T gx = DbT<T, NC, GX>(X(t1), ix, A.nx, A.c, A.nc) + DfT<T, NC, GYZ>(Z(t5), iz, A.nz, A.c, A.nc) +
+                 DfT<T, NC, GYZ>(Y(t6), iy, A.ny, A.c, A.nc);
+    const T gy = DbT<T, NC, GYZ>(Y(t2), iy, A.ny, A.c, A.nc) + DfT<T, NC, GYZ>(Z(t4), iz, A.nz, A.c, A.nc) +
+                 DfT<T, NC, GX>(X(t6), ix, A.nx, A.c, A.nc);
+    const T gz = DbT<T, NC, GYZ>(Z(t3), iz, A.nz, A.c, A.nc) + DfT<T, NC, GYZ>(Y(t4), iy, A.ny, A.c, A.nc) +
+                 DfT<T, NC, GX>(X(t5), ix, A.nx, A.c, A.nc);
     A.lv[0][i] = d * A.lv[0][i] + ih * gx;
     A.lv[1][i] = d * A.lv[1][i] + ih * gy;
     A.lv[2][i] = d * A.lv[2][i] + ih * gz;
 }
-template <typename T>
+template <typename T, int NC>
 __global__ void k_adj_velfin(AdjArgs<T> A)
 {
     long long i;

@@ -1127,10 +1127,16 @@ int adjoint_step_t(PeSolver *S, const PeAdjoint *adj, int64_t n, const void *res
     const dim3 ag((unsigned)((c.nx + pe::ADJ_BX - 1) / pe::ADJ_BX), (unsigned)((c.ny + pe::ADJ_BY - 1) / pe::ADJ_BY),
                   (unsigned)c.nz);
     pe::k_adj_vel_u<T><<<ag, ab, 0, st>>>(A);
-    pe::k_adj_vel<T><<<ag, ab, 0, st>>>(A);
-    pe::k_adj_strain<T><<<ag, ab, 0, st>>>(A);
+    if (A.nc == 4) {
+        pe::k_adj_vel<T, 4><<<ag, ab, 0, st>>>(A);
+        pe::k_adj_strain<T, 4><<<ag, ab, 0, st>>>(A);
+    } else {
+        pe::k_adj_vel<T, 0><<<ag, ab, 0, st>>>(A);
+        pe::k_adj_strain<T, 0><<<ag, ab, 0, st>>>(A);
+    }
     pe::k_adj_stress<T><<<ag, ab, 0, st>>>(A);
-    pe::k_adj_velfin<T><<<ag, ab, 0, st>>>(A);
+    if (A.nc == 4) pe::k_adj_velfin<T, 4><<<ag, ab, 0, st>>>(A);
+    else pe::k_adj_velfin<T, 0><<<ag, ab, 0, st>>>(A);
     PE_CUDA(cudaGetLastError());
     return PE_OK;
 }
