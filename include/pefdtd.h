@@ -245,8 +245,8 @@ typedef struct PeBatch PeBatch;
 
 int pe_batch_create(int n, const PeConfig *cfgs, const PeMedium *media, const PeProbe *probes,
                     PeBatch **out);
-/* Work layout: planes per z-march (0 = 40) and steps per captured graph
- * (0 = keep). Chosen by pefdtd.autotune. */
+/* Work layout: planes per z-march (0 = FP32 pair batches cut into equal
+ * shares per block, others 40 planes) and steps per captured graph (0 = keep). Chosen by pefdtd.autotune. */
 int pe_batch_schedule(PeBatch *b, int z_chunk, int chunk_steps);
 /* Persistent batch mode (on = 1): one cooperative launch per graph chunk
  * advances every batched solve by the chunk's steps, its blocks alternating

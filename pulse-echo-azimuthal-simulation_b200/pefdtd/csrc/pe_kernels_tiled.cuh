@@ -1,4 +1,6 @@
-// Shared-memory tiled step kernels (the default path).
+// Shared-memory tiled step kernels fed by cp.async: grids whose rows are not
+// 16-byte units, where the pair kernels' padded copies do not serve (FP64,
+// FP32 runs of a few steps, no memory for the copies), and unaligned states.
 //
 // Same arithmetic, term order and explicit FMA placement as the simple
 // kernels in pe_kernels.cuh (and the oracle); only the data movement differs.

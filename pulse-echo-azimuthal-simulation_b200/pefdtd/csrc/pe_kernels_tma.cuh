@@ -1,11 +1,11 @@
-// TMA-fed step kernels (the default path on grids whose rows are 16-byte
-// multiples).
+// TMA-fed one-column step kernels: FP64 on grids whose rows are 16-byte
+// multiples, and the cross-check of the FP32 pair kernels.
 //
 // Same block geometry, arithmetic, term order and explicit FMA placement as
 // pe_kernels_tiled.cuh; the difference is who moves the data. One elected
 // thread per block issues, per plane, a handful of cp.async.bulk.tensor box
 // loads (tile planes with their stencil halo, and the per-cell operands) into
-// one of three shared-memory slots, each tracked by an mbarrier with the
+// one of three shared-memory slots (FP64 stress: two), each tracked by an mbarrier with the
 // transaction byte count; the other threads only wait on that mbarrier. No
 // per-thread address arithmetic is spent on staging. Every wait is bounded:
 // a wait that exceeds its limit records PE_ERR_TIMEOUT in a device status
