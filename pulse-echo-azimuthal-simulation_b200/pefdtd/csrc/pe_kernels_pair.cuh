@@ -1236,6 +1236,7 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
 // items off[b] to off[b + 1] - 1, re-staging a solve's arguments and tables
 // only when the solve changes.
 // All solves of a pair batch have rows of 16-byte multiples, their own or padded.
+static_assert(sizeof(StepArgs<float>) / 4 <= PS_N, "copy_args moves one word per thread of a pair block");
 struct PairItem {
     int solve, bx, by, zb, ze;
 };
