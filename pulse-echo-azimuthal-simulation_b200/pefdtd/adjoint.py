@@ -71,6 +71,8 @@ def adjoint_bytes(shape, nt, checkpoint_every=200, inner_every=None, offload=Fal
     solve = 9 * field + 2 * ncell + (4 * ncell if damp_volume else 0)
     if esize == 4 and shape[2] % 4:   # the solver's row-padded fields, labels, damping volume
         solve += (ncell // shape[2]) * (-(-shape[2] // 4) * 4) * (38 + (4 if damp_volume else 0))
+    elif esize == 8 and shape[2] % 4 == 2 and damp_volume:   # its row-padded damping volume
+        solve += (ncell // shape[2]) * (shape[2] + 2) * 4
     outer = 0 if offload else -(-int(nt) // K) * 9 * field
     inner = (-(-min(K, int(nt)) // m)) * 9 * field if m < K else 0
     hist = min(m, int(nt)) * 3 * field

@@ -590,8 +590,11 @@ int configure_kernels(PeSolver *S)
 int ensure_maps(PeSolver *S, const PeState *st)
 {
     const bool pad = is_padded_state(S, st);
-    const float *const dvol = pad ? S->dvol_p : S->dvol;
-    const int pitch = pad ? S->px : 0;
+    // FP64 rows of 16-byte units can be float rows that are not: the damping
+    // volume then has a row-padded copy for its map
+    const bool pad_dvol = pad || (!S->padded && S->dvol_p);
+    const float *const dvol = pad_dvol ? S->dvol_p : S->dvol;
+    const int pitch = pad ? S->px : 0, dpitch = pad_dvol ? S->px : 0;
     if (!S->tma_capable && !S->pair_capable && !pad) {
         S->tma = false;
         S->pair = false;
@@ -605,7 +608,7 @@ int ensure_maps(PeSolver *S, const PeState *st)
     for (int i = 0; i < 3; ++i) aligned = aligned && ((uintptr_t)st->v[i] % 16) == 0;
     for (int i = 0; i < 6; ++i) aligned = aligned && ((uintptr_t)st->s[i] % 16) == 0;
     S->mstate = *st;
-    S->maps_ok = true;
+    S->maps_ok = !aligned;   // with maps: once the last one is encoded
     S->tma = aligned && S->tma_capable;
     S->pair = aligned && (S->pair_capable || pad);
     if (!aligned) return PE_OK;
@@ -622,30 +625,32 @@ int ensure_maps(PeSolver *S, const PeState *st)
         for (int f = 0; f < 3; ++f)
             if ((rc = encode_box(&S->mpv.vc[f], st->v[f], dt, es, c, pe::PV_OX, pe::PV_OY, pitch))) return rc;
         if (dvol) {
-            if ((rc = encode_box(&S->mps.dv, dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::PS_SW, pe::PS_SH, pitch))) return rc;
-            if ((rc = encode_box(&S->mpv.dv, dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::PV_OX, pe::PV_OY, pitch))) return rc;
+            if ((rc = encode_box(&S->mps.dv, dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::PS_SW, pe::PS_SH, dpitch))) return rc;
+            if ((rc = encode_box(&S->mpv.dv, dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::PV_OX, pe::PV_OY, dpitch))) return rc;
         } else {
             std::memset(&S->mps.dv, 0, sizeof(S->mps.dv));
             std::memset(&S->mpv.dv, 0, sizeof(S->mpv.dv));
         }
     }
-    if (!S->tma) return PE_OK;
-    for (int f = 0; f < 3; ++f)
-        if ((rc = encode_box(&S->ms.vt[f], st->v[f], dt, es, c, pe::KS_VW, pe::KS_VH))) return rc;
-    for (int f = 0; f < 6; ++f)
-        if ((rc = encode_box(&S->ms.sc[f], st->s[f], dt, es, c, pe::KS_SW, pe::KS_SH))) return rc;
-    const int vf[5] = {0, 1, 3, 4, 5};
-    for (int f = 0; f < 5; ++f)
-        if ((rc = encode_box(&S->mv.st[f], st->s[vf[f]], dt, es, c, pe::KV_SW, pe::KV_SH))) return rc;
-    for (int f = 0; f < 3; ++f)
-        if ((rc = encode_box(&S->mv.vc[f], st->v[f], dt, es, c, pe::KV_CW, pe::KV_CH))) return rc;
-    if (S->dvol) {
-        if ((rc = encode_box(&S->ms.dv, S->dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::KS_SW, pe::KS_SH))) return rc;
-        if ((rc = encode_box(&S->mv.dv, S->dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::KV_CW, pe::KV_CH))) return rc;
-    } else {
-        std::memset(&S->ms.dv, 0, sizeof(S->ms.dv));
-        std::memset(&S->mv.dv, 0, sizeof(S->mv.dv));
+    if (S->tma) {
+        for (int f = 0; f < 3; ++f)
+            if ((rc = encode_box(&S->ms.vt[f], st->v[f], dt, es, c, pe::KS_VW, pe::KS_VH))) return rc;
+        for (int f = 0; f < 6; ++f)
+            if ((rc = encode_box(&S->ms.sc[f], st->s[f], dt, es, c, pe::KS_SW, pe::KS_SH))) return rc;
+        const int vf[5] = {0, 1, 3, 4, 5};
+        for (int f = 0; f < 5; ++f)
+            if ((rc = encode_box(&S->mv.st[f], st->s[vf[f]], dt, es, c, pe::KV_SW, pe::KV_SH))) return rc;
+        for (int f = 0; f < 3; ++f)
+            if ((rc = encode_box(&S->mv.vc[f], st->v[f], dt, es, c, pe::KV_CW, pe::KV_CH))) return rc;
+        if (dvol) {
+            if ((rc = encode_box(&S->ms.dv, dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::KS_SW, pe::KS_SH, dpitch))) return rc;
+            if ((rc = encode_box(&S->mv.dv, dvol, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, c, pe::KV_CW, pe::KV_CH, dpitch))) return rc;
+        } else {
+            std::memset(&S->ms.dv, 0, sizeof(S->ms.dv));
+            std::memset(&S->mv.dv, 0, sizeof(S->mv.dv));
+        }
     }
+    S->maps_ok = true;
     return PE_OK;
 }
 
@@ -904,15 +909,22 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
             S->padded = false;
         }
     }
+    // FP64 with nx = 2 mod 4: the TMA kernels' damping boxes need float rows of
+    // 16-byte units; without the memory for them the solve keeps the cp.async kernels
+    if (S->tma_capable && S->dvol && c.nx % 4 != 0 &&
+        dev_alloc(&S->dvol_p, sizeof(float) * (size_t)S->px * c.ny * c.nz) != PE_OK) {
+        cudaGetLastError();
+        S->tma_capable = false;
+    }
+    if (S->dvol_p) {
+        PE_CUDA(cudaMemsetAsync(S->dvol_p, 0, sizeof(float) * (size_t)S->px * c.ny * c.nz, st));
+        PE_CUDA(cudaMemcpy2DAsync(S->dvol_p, sizeof(float) * S->px, S->dvol, sizeof(float) * c.nx,
+                                  sizeof(float) * c.nx, (size_t)c.ny * c.nz, cudaMemcpyDeviceToDevice, st));
+    }
     if (S->padded) {
         const size_t ncp = (size_t)S->px * c.ny * c.nz;
         PE_CUDA(cudaMemsetAsync(S->pfields, 0, 9 * sizeof(float) * ncp, st));
         PE_CUDA(cudaMemsetAsync(S->lab_p, 0, sizeof(uint16_t) * ncp, st));
-        if (S->dvol_p) {
-            PE_CUDA(cudaMemsetAsync(S->dvol_p, 0, sizeof(float) * ncp, st));
-            PE_CUDA(cudaMemcpy2DAsync(S->dvol_p, sizeof(float) * S->px, S->dvol, sizeof(float) * c.nx,
-                                      sizeof(float) * c.nx, (size_t)c.ny * c.nz, cudaMemcpyDeviceToDevice, st));
-        }
         for (int i = 0; i < 3; ++i) S->pst.v[i] = (float *)S->pfields + i * ncp;
         for (int i = 0; i < 6; ++i) S->pst.s[i] = (float *)S->pfields + (3 + i) * ncp;
         auto to_padded = [&](long long q) { return q / c.nx * S->px + q % c.nx; };

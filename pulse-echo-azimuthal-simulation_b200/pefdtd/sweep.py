@@ -276,7 +276,8 @@ def setup_bytes(setup, dtype_size=4):
     cells = nz * ny * nx
     if nx % 4 and dtype_size == 4:
         cells += nz * ny * (-(-nx // 4) * 4)
-    return cells * (9 * dtype_size + 2 + 4) + setup["nt"] * dtype_size + (64 << 20)
+    extra = 4 * nz * ny * (nx + 2) if nx % 4 == 2 and dtype_size == 8 else 0   # row-padded damping volume (FP64)
+    return cells * (9 * dtype_size + 2 + 4) + extra + setup["nt"] * dtype_size + (64 << 20)
 
 
 # ---------------------------------------------------------------- solving
