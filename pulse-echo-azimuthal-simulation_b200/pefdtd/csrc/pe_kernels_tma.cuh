@@ -637,6 +637,16 @@ struct BatchItem {
     int solve, bx, by, bz;
 };
 
+// Dynamic shared memory of a batch launch: each of its solves lays its block
+// out by its own material count, and the solve with the most materials need
+// not be the largest (a table too large for shared memory takes none).
+inline size_t batch_tma_smem(size_t (*need)(int), const int *n_mats, int n)
+{
+    size_t m = 0;
+    for (int i = 0; i < n; ++i) m = need(n_mats[i]) > m ? need(n_mats[i]) : m;
+    return m;
+}
+
 template <typename T>
 __device__ __forceinline__ void copy_args(StepArgs<T> *dst, const StepArgs<T> *src, int k)
 {

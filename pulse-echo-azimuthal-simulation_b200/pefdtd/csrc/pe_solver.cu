@@ -1683,10 +1683,10 @@ template <typename T>
 int batch_layout(PeBatch *B)
 {
     std::vector<pe::BatchItem> is, iv;
-    int max_mat = 1;
+    std::vector<int> nms;   // material counts of the solves the TMA batch kernels may take
     for (int s = 0; s < (int)B->solves.size(); ++s) {
         const PeConfig &c = B->solves[s]->cfg;
-        if (B->solves[s]->tma_capable) max_mat = std::max(max_mat, c.n_mat);
+        if (B->solves[s]->tma_capable) nms.push_back(c.n_mat);
         const int target = c.z_chunk > 0 ? c.z_chunk : (B->z_chunk > 0 ? B->z_chunk : 40);
         const int nch = std::max(1, (c.nz + target - 1) / target);
         const int zc = (c.nz + nch - 1) / nch;
@@ -1712,8 +1712,8 @@ int batch_layout(PeBatch *B)
         }
     }
     if (!B->pair_batch) {
-    B->smem_s = pe::stress_tma_smem<T>(max_mat);
-    B->smem_v = pe::velocity_tma_smem<T>(max_mat);
+    B->smem_s = pe::batch_tma_smem(pe::stress_tma_smem<T>, nms.data(), (int)nms.size());
+    B->smem_v = pe::batch_tma_smem(pe::velocity_tma_smem<T>, nms.data(), (int)nms.size());
     cudaFuncAttributes fa_s{}, fa_v{};
     PE_CUDA(cudaFuncGetAttributes(&fa_s, pe::k_stress_tma_batch<T>));
     PE_CUDA(cudaFuncGetAttributes(&fa_v, pe::k_velocity_tma_batch<T>));
