@@ -1448,9 +1448,21 @@ struct PeBatch {
     int *status = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
-    void *descs = nullptr;
-    pe::TmapsStress *maps_s = nullptr;
-    pe::TmapsVelocity *maps_v = nullptr;
+    // what the launches read and the graph made of them: one set for runs in
+    // place, one for runs through the padded states (pad_on), so that a run of
+    // the one kind leaves alone what queued runs of the other kind read
+    struct Set {
+        void *descs = nullptr;
+        pe::TmapsStress *maps_s = nullptr;
+        pe::TmapsVelocity *maps_v = nullptr;
+        pe::TmapsPairStress *pmaps_s = nullptr;
+        pe::TmapsPairVelocity *pmaps_v = nullptr;
+        std::vector<PeState> states;
+        std::vector<void *> traces;
+        bool uploaded = false;
+        cudaGraphExec_t gexec = nullptr;
+        long long graph_launches = 0;   // kernels in one captured chunk
+    } sets[2];
     int *nmats = nullptr;
     pe::BatchItem *items_s = nullptr, *items_v = nullptr;
     int n_items_s = 0, n_items_v = 0;
@@ -1466,20 +1478,13 @@ struct PeBatch {
     int grid_s = 1, grid_v = 1;
     size_t smem_s = 0, smem_v = 0;
     int z_chunk = 0, chunk = 200;
-    std::vector<PeState> states;
-    std::vector<void *> traces;
-    bool uploaded = false;
-    cudaGraphExec_t gexec = nullptr;
     long long launches = 0;
-    long long graph_launches = 0;   // kernels in one captured chunk
     bool tma_batch = true;          // the batched TMA kernels fit this batch
     // FP32 batches of solves whose rows are 16-byte multiples run the
     // pair-column kernels
     bool pair_batch = false;
     bool pair_ts = false;           // every batched table fits shared memory
     bool pair_nc4 = true;           // every batched solve has four coefficients
-    pe::TmapsPairStress *pmaps_s = nullptr;
-    pe::TmapsPairVelocity *pmaps_v = nullptr;
     const float **tabs = nullptr;
     // persistent mode: one cooperative launch per graph chunk runs every step
     // of the batched pair solves (k_pair_batch_persistent)
@@ -1489,16 +1494,31 @@ struct PeBatch {
 
     ~PeBatch()
     {
-        if (gexec) cudaGraphExecDestroy(gexec);
+        drop_graphs();
         if (stream) cudaStreamSynchronize(stream);
         for (PeSolver *s : solves) pe_solver_destroy(s);
-        void *bufs[] = {step, status, descs, maps_s, maps_v, nmats, items_s, items_v, pmaps_s, pmaps_v, tabs, bar};
+        void *bufs[] = {step, status, nmats, items_s, items_v, tabs, bar};
         for (void *b : bufs)
             if (b) dev_free(b);
+        for (Set &L : sets) {
+            void *own[] = {L.descs, L.maps_s, L.maps_v, L.pmaps_s, L.pmaps_v};
+            for (void *b : own)
+                if (b) dev_free(b);
+        }
         drop_pair_work();
         if (ev_in) cudaEventDestroy(ev_in);
         if (ev_out) cudaEventDestroy(ev_out);
         if (stream) cudaStreamDestroy(stream);
+    }
+
+    Set &set() { return sets[pad_on]; }
+
+    void drop_graphs()
+    {
+        for (Set &L : sets) {
+            if (L.gexec) cudaGraphExecDestroy(L.gexec);
+            L.gexec = nullptr;
+        }
     }
 
     void drop_pair_work()
@@ -1609,6 +1629,15 @@ PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int gr
     return P;
 }
 
+// Host data for the batch's launches: copied on the batch's own stream, behind
+// the launches queued there (a copy on another stream would be ordered with
+// none of them). The source is pageable, so it is read before the call returns.
+int batch_copy(PeBatch *B, void *dst, const void *src, size_t bytes)
+{
+    if (bytes) PE_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, B->stream));
+    return PE_OK;
+}
+
 // Pair-kernel layout of an FP32 batch: work items, grids and shared memory.
 int batch_layout_pair(PeBatch *B, int nsm, int optin)
 {
@@ -1672,8 +1701,8 @@ int batch_layout_pair(PeBatch *B, int nsm, int optin)
             int rc;
             if ((rc = dev_alloc(&W.items, sizeof(pe::PairItem) * P.items.size()))) return rc;
             if ((rc = dev_alloc(&W.off, sizeof(int) * P.off.size()))) return rc;
-            PE_CUDA(cudaMemcpy(W.items, P.items.data(), sizeof(pe::PairItem) * P.items.size(), cudaMemcpyHostToDevice));
-            PE_CUDA(cudaMemcpy(W.off, P.off.data(), sizeof(int) * P.off.size(), cudaMemcpyHostToDevice));
+            if ((rc = batch_copy(B, W.items, P.items.data(), sizeof(pe::PairItem) * P.items.size()))) return rc;
+            if ((rc = batch_copy(B, W.off, P.off.data(), sizeof(int) * P.off.size()))) return rc;
             W.grid = grid;
         }
     return PE_OK;
@@ -1751,36 +1780,39 @@ int batch_layout(PeBatch *B)
     int rc;
     if ((rc = dev_alloc(&B->items_s, sizeof(pe::BatchItem) * is.size()))) return rc;
     if ((rc = dev_alloc(&B->items_v, sizeof(pe::BatchItem) * iv.size()))) return rc;
-    PE_CUDA(cudaMemcpy(B->items_s, is.data(), sizeof(pe::BatchItem) * is.size(), cudaMemcpyHostToDevice));
-    PE_CUDA(cudaMemcpy(B->items_v, iv.data(), sizeof(pe::BatchItem) * iv.size(), cudaMemcpyHostToDevice));
-    if (B->gexec) {
-        cudaGraphExecDestroy(B->gexec);
-        B->gexec = nullptr;
-    }
+    if ((rc = batch_copy(B, B->items_s, is.data(), sizeof(pe::BatchItem) * is.size()))) return rc;
+    if ((rc = batch_copy(B, B->items_v, iv.data(), sizeof(pe::BatchItem) * iv.size()))) return rc;
+    B->drop_graphs();
     return PE_OK;
 }
 
+// The current set's arguments and maps, uploaded again when a caller's buffer
+// is another than the set was made for.
 template <typename T>
 int batch_upload(PeBatch *B, const PeState *states, void *const *traces)
 {
     const int n = (int)B->solves.size();
-    bool same = B->uploaded && (int)B->states.size() == n;
-    for (int s = 0; same && s < n; ++s) same = same_state(B->states[s], states[s]) && B->traces[s] == traces[s];
+    PeBatch::Set &L = B->set();
+    bool same = L.uploaded;
+    for (int s = 0; same && s < n; ++s) same = same_state(L.states[s], states[s]) && L.traces[s] == traces[s];
+    for (int s = 0; s < n; ++s) {
+        PeSolver *S = B->solves[s];
+        if (same && batched(B, S)) continue;
+        // a solve with launches of its own takes its maps from the solver
+        const int rc = ensure_maps(S, B->pad_on && S->padded ? &S->pst : &states[s]);
+        if (rc) return rc;
+        if (batched(B, S) && !(B->pair_batch ? S->pair : S->tma))
+            return fail(PE_ERR_UNSUPPORTED, "batched solves need 16-byte aligned state buffers");
+    }
     if (same) return PE_OK;
     std::vector<pe::StepArgs<T>> descs(n);
     std::vector<pe::TmapsStress> ms(n);
     std::vector<pe::TmapsVelocity> mv(n);
     std::vector<pe::TmapsPairStress> pms(n);
     std::vector<pe::TmapsPairVelocity> pmv(n);
-    std::vector<const float *> tabs(n, nullptr);
     for (int s = 0; s < n; ++s) {
         PeSolver *S = B->solves[s];
-        const PeState *use = B->pad_on && S->padded ? &S->pst : &states[s];
-        int rc = ensure_maps(S, use);
-        if (rc) return rc;
-        if (batched(B, S) && !(B->pair_batch ? S->pair : S->tma))
-            return fail(PE_ERR_UNSUPPORTED, "batched solves need 16-byte aligned state buffers");
-        descs[s] = make_args<T>(S, use, 0);
+        descs[s] = make_args<T>(S, B->pad_on && S->padded ? &S->pst : &states[s], 0);
         descs[s].step = B->step;
         descs[s].status = B->status;
         descs[s].zc = S->zc_s;
@@ -1788,20 +1820,20 @@ int batch_upload(PeBatch *B, const PeState *states, void *const *traces)
         mv[s] = S->mv;
         pms[s] = S->mps;
         pmv[s] = S->mpv;
-        tabs[s] = S->tab36;
     }
-    PE_CUDA(cudaMemcpy(B->descs, descs.data(), sizeof(pe::StepArgs<T>) * n, cudaMemcpyHostToDevice));
-    PE_CUDA(cudaMemcpy(B->maps_s, ms.data(), sizeof(pe::TmapsStress) * n, cudaMemcpyHostToDevice));
-    PE_CUDA(cudaMemcpy(B->maps_v, mv.data(), sizeof(pe::TmapsVelocity) * n, cudaMemcpyHostToDevice));
-    PE_CUDA(cudaMemcpy(B->pmaps_s, pms.data(), sizeof(pe::TmapsPairStress) * n, cudaMemcpyHostToDevice));
-    PE_CUDA(cudaMemcpy(B->pmaps_v, pmv.data(), sizeof(pe::TmapsPairVelocity) * n, cudaMemcpyHostToDevice));
-    PE_CUDA(cudaMemcpy(B->tabs, tabs.data(), sizeof(const float *) * n, cudaMemcpyHostToDevice));
-    B->states.assign(states, states + n);
-    B->traces.assign(traces, traces + n);
-    B->uploaded = true;
-    if (B->gexec) {
-        cudaGraphExecDestroy(B->gexec);
-        B->gexec = nullptr;
+    L.uploaded = false;
+    int rc;
+    if ((rc = batch_copy(B, L.descs, descs.data(), sizeof(pe::StepArgs<T>) * n))) return rc;
+    if ((rc = batch_copy(B, L.maps_s, ms.data(), sizeof(pe::TmapsStress) * n))) return rc;
+    if ((rc = batch_copy(B, L.maps_v, mv.data(), sizeof(pe::TmapsVelocity) * n))) return rc;
+    if ((rc = batch_copy(B, L.pmaps_s, pms.data(), sizeof(pe::TmapsPairStress) * n))) return rc;
+    if ((rc = batch_copy(B, L.pmaps_v, pmv.data(), sizeof(pe::TmapsPairVelocity) * n))) return rc;
+    L.states.assign(states, states + n);
+    L.traces.assign(traces, traces + n);
+    L.uploaded = true;
+    if (L.gexec) {
+        cudaGraphExecDestroy(L.gexec);
+        L.gexec = nullptr;
     }
     return PE_OK;
 }
@@ -1822,10 +1854,10 @@ int launch_pair_persistent(PeBatch *B, int len)
     at[0].val.cooperative = 1;
     lc.attrs = at;
     lc.numAttrs = 1;
-    const pe::StepArgs<float> *d = (const pe::StepArgs<float> *)B->descs;
+    const pe::StepArgs<float> *d = (const pe::StepArgs<float> *)B->set().descs;
     const float *const *tabs = B->tabs;
-    const pe::TmapsPairStress *ms = B->pmaps_s;
-    const pe::TmapsPairVelocity *mv = B->pmaps_v;
+    const pe::TmapsPairStress *ms = B->set().pmaps_s;
+    const pe::TmapsPairVelocity *mv = B->set().pmaps_v;
     const int *nm = B->nmats, *os = ws.off, *ov = wv.off;
     const pe::PairItem *is = ws.items, *iv = wv.items;
     cudaError_t e;
@@ -1846,6 +1878,7 @@ template <typename T>
 int batch_chunk(PeBatch *B, int len)
 {
     const dim3 block(pe::TB_X, pe::TB_Y, 1);
+    const PeBatch::Set &L = B->set();
     const PeBatch::PairWork &ws = B->work_s[pad_shared(B)], &wv = B->work_v[pad_shared(B)];
     if constexpr (std::is_same<T, float>::value) {
         if (B->pair_batch && B->persistent && ws.grid > 0) {
@@ -1856,27 +1889,27 @@ int batch_chunk(PeBatch *B, int len)
     for (int k = 0; k < len; ++k) {
         if constexpr (std::is_same<T, float>::value) {
             if (B->pair_batch && !B->persistent && ws.grid > 0) {
-                const pe::StepArgs<float> *d = (const pe::StepArgs<float> *)B->descs;
+                const pe::StepArgs<float> *d = (const pe::StepArgs<float> *)L.descs;
                 if (B->pair_nc4 && B->pair_ts)
-                    pe::k_stress_pair_batch<4, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
+                    pe::k_stress_pair_batch<4, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
                 else if (B->pair_nc4)
-                    pe::k_stress_pair_batch<4, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
+                    pe::k_stress_pair_batch<4, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
                 else if (B->pair_ts)
-                    pe::k_stress_pair_batch<0, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
+                    pe::k_stress_pair_batch<0, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
                 else
-                    pe::k_stress_pair_batch<0, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, B->pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
+                    pe::k_stress_pair_batch<0, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
                 if (B->pair_nc4)
-                    pe::k_velocity_pair_batch<4><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, B->pmaps_v, B->nmats, wv.items, wv.off, k);
+                    pe::k_velocity_pair_batch<4><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, L.pmaps_v, B->nmats, wv.items, wv.off, k);
                 else
-                    pe::k_velocity_pair_batch<0><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, B->pmaps_v, B->nmats, wv.items, wv.off, k);
+                    pe::k_velocity_pair_batch<0><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, L.pmaps_v, B->nmats, wv.items, wv.off, k);
                 B->launches += 2;
             }
         }
         if (!B->pair_batch && B->n_items_s > 0) {
             pe::k_stress_tma_batch<T><<<B->grid_s, block, B->smem_s, B->stream>>>(
-                (const pe::StepArgs<T> *)B->descs, B->maps_s, B->nmats, B->items_s, B->n_items_s, k);
+                (const pe::StepArgs<T> *)L.descs, L.maps_s, B->nmats, B->items_s, B->n_items_s, k);
             pe::k_velocity_tma_batch<T><<<B->grid_v, block, B->smem_v, B->stream>>>(
-                (const pe::StepArgs<T> *)B->descs, B->maps_v, B->nmats, B->items_v, B->n_items_v, k);
+                (const pe::StepArgs<T> *)L.descs, L.maps_v, B->nmats, B->items_v, B->n_items_v, k);
             B->launches += 2;
         }
         // solves outside the batched launches (rows not whole 16-byte
@@ -1885,7 +1918,7 @@ int batch_chunk(PeBatch *B, int len)
         for (int s = 0; s < (int)B->solves.size(); ++s) {
             PeSolver *S = B->solves[s];
             if (batched(B, S)) continue;
-            pe::StepArgs<T> A = make_args<T>(S, B->pad_on && S->padded ? &S->pst : &B->states[s], k);
+            pe::StepArgs<T> A = make_args<T>(S, B->pad_on && S->padded ? &S->pst : &L.states[s], k);
             A.step = B->step;
             A.status = B->status;
             launch_stress<T>(S, A, B->stream);
@@ -1899,7 +1932,7 @@ int batch_chunk(PeBatch *B, int len)
         const int nthr = len * S->n_groups;
         pe::k_reduce_traces<T><<<(nthr + 127) / 128, 128, 0, B->stream>>>(
             (const T *)S->rec_val, (const T *)S->rec_w, S->grp_off, S->n_groups, S->n_rec, len, B->step,
-            (T *)B->traces[s]);
+            (T *)L.traces[s]);
         B->launches += 1;
     }
     pe::k_step_advance<<<1, 1, 0, B->stream>>>(B->step, len);
@@ -1913,10 +1946,8 @@ int batch_run_t(PeBatch *B, const PeState *states, void *const *traces, int64_t 
 {
     bool pad = false;
     for (const PeSolver *S : B->solves) pad = pad || (B->pair_batch && S->padded && e - b >= PAD_MIN_STEPS);
-    if (pad != B->pad_on) {   // other states and launches than the ones uploaded
-        B->pad_on = pad;
-        B->uploaded = false;
-    }
+    B->pad_on = pad;
+    PeBatch::Set &L = B->set();
     int rc = batch_upload<T>(B, states, traces);
     if (rc) return rc;
     PE_CUDA(cudaEventRecord(B->ev_in, user));
@@ -1928,7 +1959,7 @@ int batch_run_t(PeBatch *B, const PeState *states, void *const *traces, int64_t 
     for (int64_t n = b; n < e;) {
         const int len = (int)std::min<int64_t>(B->chunk, e - n);
         if (len == B->chunk) {
-            if (!B->gexec) {
+            if (!L.gexec) {
                 cudaGraph_t g = nullptr;
                 PE_CUDA(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
                 const long long before = B->launches;
@@ -1936,14 +1967,14 @@ int batch_run_t(PeBatch *B, const PeState *states, void *const *traces, int64_t 
                 cudaError_t ce = cudaStreamEndCapture(B->stream, &g);
                 if (rc) return rc;
                 if (ce != cudaSuccess) return fail(PE_ERR_CUDA, std::string("batch graph capture: ") + cudaGetErrorString(ce));
-                B->graph_launches = B->launches - before;
+                L.graph_launches = B->launches - before;
                 B->launches = before;
-                ce = cudaGraphInstantiate(&B->gexec, g, 0);
+                ce = cudaGraphInstantiate(&L.gexec, g, 0);
                 cudaGraphDestroy(g);
                 if (ce != cudaSuccess) return fail(PE_ERR_CUDA, std::string("batch graph instantiate: ") + cudaGetErrorString(ce));
             }
-            PE_CUDA(cudaGraphLaunch(B->gexec, B->stream));
-            B->launches += B->graph_launches;
+            PE_CUDA(cudaGraphLaunch(L.gexec, B->stream));
+            B->launches += L.graph_launches;
         } else if ((rc = batch_chunk<T>(B, len))) {
             return rc;
         }
@@ -1981,22 +2012,32 @@ int pe_batch_create(int n, const PeConfig *cfgs, const PeMedium *media, const Pe
     int rc;
     if ((rc = dev_alloc(&B->step, sizeof(long long)))) return rc;
     if ((rc = dev_alloc(&B->status, sizeof(int)))) return rc;
-    PE_CUDA(cudaMemset(B->status, 0, sizeof(int)));
     if ((rc = dev_alloc(&B->bar, sizeof(unsigned)))) return rc;
+    bool padded = false;
+    for (const PeSolver *S : B->solves) padded = padded || S->padded;
     const size_t ds = B->dtype == PE_F64 ? sizeof(pe::StepArgs<double>) : sizeof(pe::StepArgs<float>);
-    if ((rc = dev_alloc(&B->descs, ds * n))) return rc;
-    if ((rc = dev_alloc(&B->maps_s, sizeof(pe::TmapsStress) * n))) return rc;
-    if ((rc = dev_alloc(&B->maps_v, sizeof(pe::TmapsVelocity) * n))) return rc;
+    for (int k = 0; k < (padded ? 2 : 1); ++k) {
+        PeBatch::Set &L = B->sets[k];
+        if ((rc = dev_alloc(&L.descs, ds * n))) return rc;
+        if ((rc = dev_alloc(&L.maps_s, sizeof(pe::TmapsStress) * n))) return rc;
+        if ((rc = dev_alloc(&L.maps_v, sizeof(pe::TmapsVelocity) * n))) return rc;
+        if ((rc = dev_alloc(&L.pmaps_s, sizeof(pe::TmapsPairStress) * n))) return rc;
+        if ((rc = dev_alloc(&L.pmaps_v, sizeof(pe::TmapsPairVelocity) * n))) return rc;
+    }
     if ((rc = dev_alloc(&B->nmats, sizeof(int) * n))) return rc;
-    if ((rc = dev_alloc(&B->pmaps_s, sizeof(pe::TmapsPairStress) * n))) return rc;
-    if ((rc = dev_alloc(&B->pmaps_v, sizeof(pe::TmapsPairVelocity) * n))) return rc;
     if ((rc = dev_alloc(&B->tabs, sizeof(const float *) * n))) return rc;
-    std::vector<int> nm(n);
-    for (int s = 0; s < n; ++s) nm[s] = cfgs[s].n_mat;
-    PE_CUDA(cudaMemcpy(B->nmats, nm.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
     PE_CUDA(cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking));
     PE_CUDA(cudaEventCreateWithFlags(&B->ev_in, cudaEventDisableTiming));
     PE_CUDA(cudaEventCreateWithFlags(&B->ev_out, cudaEventDisableTiming));
+    std::vector<int> nm;
+    std::vector<const float *> tabs;
+    for (const PeSolver *S : B->solves) {
+        nm.push_back(S->cfg.n_mat);
+        tabs.push_back(S->tab36);
+    }
+    if ((rc = batch_copy(B.get(), B->nmats, nm.data(), sizeof(int) * n))) return rc;
+    if ((rc = batch_copy(B.get(), B->tabs, tabs.data(), sizeof(const float *) * n))) return rc;
+    PE_CUDA(cudaMemsetAsync(B->status, 0, sizeof(int), B->stream));
     rc = B->dtype == PE_F64 ? batch_layout<double>(B.get()) : batch_layout<float>(B.get());
     if (rc) return rc;
     *out = B.release();
@@ -2006,10 +2047,11 @@ int pe_batch_create(int n, const PeConfig *cfgs, const PeMedium *media, const Pe
 int pe_batch_schedule(PeBatch *B, int z_chunk, int chunk_steps)
 {
     if (!B || z_chunk < 0 || chunk_steps < 0) return fail(PE_ERR_INVALID, "bad schedule");
+    PE_CUDA(cudaStreamSynchronize(B->stream));   // queued runs read the work lists that go
     B->z_chunk = z_chunk;
     if (chunk_steps > 0) B->chunk = chunk_steps;
     for (PeSolver *S : B->solves) S->cfg.z_chunk = 0;
-    B->uploaded = false;
+    for (PeBatch::Set &L : B->sets) L.uploaded = false;
     return B->dtype == PE_F64 ? batch_layout<double>(B) : batch_layout<float>(B);
 }
 
@@ -2020,10 +2062,7 @@ int pe_batch_set_persistent(PeBatch *B, int on)
         return fail(PE_ERR_UNSUPPORTED, "the persistent kernel runs FP32 batches of pair-column solves");
     if (B->persistent != (on != 0)) {
         B->persistent = on != 0;
-        if (B->gexec) {
-            cudaGraphExecDestroy(B->gexec);
-            B->gexec = nullptr;
-        }
+        B->drop_graphs();
     }
     return PE_OK;
 }
