@@ -203,6 +203,10 @@ class AdjointSolve:
                 _capi.check(L.pe_solver_adjoint_segment(s._h, C.byref(s._st), C.byref(adj), hist.data_ptr(),
                                                         a, b, res.data_ptr(), C.c_void_p(stream.cuda_stream)))
 
+        # one set of inner checkpoints for all segments: a buffer that goes back to
+        # another stream's pool is handed on only after this stream has passed
+        # it, and the host would allocate segment after segment ahead of that
+        inner = []
         for a in reversed(sorted(self.ckpt)):
             b = min(a + self.K, nt)
             s.state.copy_(self.ckpt[a], non_blocking=True)
@@ -211,14 +215,15 @@ class AdjointSolve:
             else:
                 # two levels: inner checkpoints every m steps of the segment,
                 # then the sub-segments last first, m steps of history each
-                inner = {}
-                for a2 in range(a, b, self.m):
-                    inner[a2] = self._new(s.state.shape, s.state.dtype).copy_(s.state)
+                starts = range(a, b, self.m)
+                while len(inner) < len(starts):
+                    inner.append(self._new(s.state.shape, s.state.dtype))
+                for a2, buf in zip(starts, inner):
+                    buf.copy_(s.state)
                     s.run(a2, min(a2 + self.m, b))
-                for a2 in reversed(sorted(inner)):
-                    s.state.copy_(inner[a2])
+                for a2, buf in reversed(list(zip(starts, inner))):
+                    s.state.copy_(buf)
                     reverse(a2, min(a2 + self.m, b))
-                del inner
             yield grad
 
 
