@@ -975,11 +975,19 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
 int pe_solver_set_wavelet(PeSolver *S, const void *wavelet, int64_t nt)
 {
     if (!S || (nt > 0 && !wavelet) || nt < 0) return fail(PE_ERR_INVALID, "bad wavelet");
+    void *const old = S->wavelet;
     if (S->wavelet) {
         dev_free(S->wavelet);
         S->wavelet = nullptr;
+        S->nt_wav = 0;
     }
     int rc = dev_alloc(&S->wavelet, (size_t)S->esize * std::max<int64_t>(1, nt));
+    if (S->wavelet != old) {   // the captured graph reads the old buffer
+        if (S->gexec) cudaGraphExecDestroy(S->gexec);
+        S->gexec = nullptr;
+        S->gstate = PeState{};
+        S->gtraces = nullptr;
+    }
     if (rc) return rc;
     if (nt > 0)
         PE_CUDA(cudaMemcpyAsync(S->wavelet, wavelet, (size_t)S->esize * nt, cudaMemcpyHostToDevice, S->stream));
@@ -2070,6 +2078,8 @@ int pe_batch_set_persistent(PeBatch *B, int on)
 int pe_batch_set_wavelet(PeBatch *B, int i, const void *wavelet, int64_t nt)
 {
     if (!B || i < 0 || i >= (int)B->solves.size()) return fail(PE_ERR_INVALID, "bad solve index");
+    PE_CUDA(cudaStreamSynchronize(B->stream));   // queued runs read the old one
+    for (PeBatch::Set &L : B->sets) L.uploaded = false;
     return pe_solver_set_wavelet(B->solves[i], wavelet, nt);
 }
 
