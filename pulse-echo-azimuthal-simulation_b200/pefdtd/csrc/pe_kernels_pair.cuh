@@ -791,6 +791,13 @@ __host__ __device__ constexpr int pair_last_inside_y(int ny) { return ny < 19 ? 
 // Launch grid: (tiles x, tiles y, z-chunks of A.zc planes). Blocks that run
 // at the same time march the same planes of neighbouring tiles, so the tile
 // halos they share are read from DRAM once and from L2 after that.
+// The successor is let in after the march (pdl_release at the end, here and in
+// k_velocity_pair): two blocks share an SM, and a successor let in at the start
+// puts its blocks on the free halves while the march runs, two on some SMs and
+// none on others. us a step with no dependent launch, release at the start,
+// release at the end: 114x48x48 37.3, 45.6, 36.0; 64x96x96 per-cell 47.8, 56.2,
+// 46.6; 160x256x256 469, 475, 469; 20x24x28 in plain launches, ms a call 2.08,
+// 1.90, 1.82.
 template <int NC, bool TS, bool CM = false>
 __global__ void __launch_bounds__(PS_N, 2) k_stress_pair(const __grid_constant__ TmapsPairStress M,
                                                          const StepArgs<float> A,
@@ -798,7 +805,6 @@ __global__ void __launch_bounds__(PS_N, 2) k_stress_pair(const __grid_constant__
 {
     extern __shared__ __align__(128) unsigned char smem_pair[];
     float *tsm = reinterpret_cast<float *>(smem_pair + PS_SMEM_FIXED);
-    pdl_release();
     stress_pair_init(smem_pair);
     if (TS) stage_table(tsm, tab36, n_mat);
     __syncthreads();
@@ -812,6 +818,7 @@ __global__ void __launch_bounds__(PS_N, 2) k_stress_pair(const __grid_constant__
         stress_pair_march<NC, TS, true, true, CM>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
     else
         stress_pair_march<NC, TS, false, true, CM>(M, A, TS ? tsm : tab36, smem_pair, bx, by, zb, ze, ph);
+    pdl_release();
 }
 
 // ====================================================================== velocity
@@ -1211,7 +1218,6 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
     unsigned long long *bars = reinterpret_cast<unsigned long long *>(smem_pair);
     float *rsm = reinterpret_cast<float *>(smem_pair + 128) + 3 * PV_SLOT;
     const int tid = threadIdx.x;
-    pdl_release();
     if (tid == 0) {
         for (int s = 0; s < 3; ++s) mbar_init(bars + s, 1);
         fence_mbar_init();
@@ -1230,6 +1236,7 @@ __global__ void __launch_bounds__(PV_N, 2) k_velocity_pair(const __grid_constant
         velocity_pair_march<NC, true, true, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
     else
         velocity_pair_march<NC, false, true, CM>(M, A, rho_tab, smem_pair, bx, by, zb, ze, 0);
+    pdl_release();
 }
 
 // ---------------------------------------------------------------- batches

@@ -142,7 +142,8 @@ __device__ __forceinline__ int floor4(int x) { return x & ~3; }
 // nothing between them, so each is launched while its predecessor's last
 // blocks still run, sets up its block (barriers, table, pads: nothing a kernel
 // writes) and only then waits for the predecessor to have finished and its
-// writes to be visible. pdl_release lets the successor be launched; no-ops in
+// writes to be visible. pdl_release lets the successor be launched (at the start
+// of the kernels here, which have an SM each to themselves); no-ops in
 // an ordinary launch. The column loads are L2-coherent (COH) in these
 // launches: the read-only path is for data nothing writes during the launch.
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
