@@ -25,6 +25,7 @@
 #include "pe_kernels_tma.cuh"
 #include "pe_kernels_pair.cuh"
 #include "pe_adjoint.cuh"
+#include "pe_march.cuh"
 #include "pefdtd.h"
 
 namespace {
@@ -423,42 +424,12 @@ bool same_state(const PeState &a, const PeState &b)
     return true;
 }
 
-// Planes per z-march: the split of nz into chunks that minimises the modelled
-// time of a launch, in planes marched at the full-SM rate: (planes per chunk +
-// start-up planes) x waves, a wave being one block on every slot. Kernels with
-// one block per SM run their waves in step, so waves count whole. With two per
-// SM, a launch that leaves every SM at most one block runs its planes in 0.8
-// of the time (measured 1.75 us a plane alone and 2.65 with two blocks per SM
-// for the stress kernel, 1.55 and 1.95 for the velocity kernel); one that fits
-// one wave waits for its slowest, guarded, blocks (`one_wave`: 1.15 stress,
-// 1.3 velocity); beyond that the blocks drift apart, and the tail costs
-// between the fraction and the whole of a wave. Against whole waves throughout
-// (which preferred one full wave): velocity kernel on 96x160x160 59 -> 54 us
-// (20 -> 8 planes), on 20x24x28 14.5 -> 12.5 us (4 -> 2 planes). A shorter
-// march must be worth 2 %: longer ones re-read less of the z halo.
-int pick_zchunk(int nz, long long tiles, int slots, int startup, double one_wave = 1.0)
+int device_sms()
 {
     int nsm = 148, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    int best_zc = nz;
-    double best = 1e300;
-    for (int nch = 1; nch <= nz; ++nch) {
-        const int zc = (nz + nch - 1) / nch;
-        const long long blocks = tiles * ((nz + zc - 1) / zc);
-        double waves = (double)((blocks + slots - 1) / slots);
-        if (slots > nsm) {
-            if (blocks <= nsm) waves = 0.8;
-            else if (blocks <= slots) waves = one_wave;
-            else waves = 0.5 * (waves + (double)blocks / slots + 0.5);
-        }
-        const double cost = waves * (zc + startup);
-        if (cost < 0.98 * best) {
-            best = cost;
-            best_zc = zc;
-        }
-    }
-    return best_zc;
+    return nsm;
 }
 
 template <typename K>
@@ -536,8 +507,9 @@ int configure_pair(PeSolver *S, int optin)
     const long long tpv = (long long)((c.nx + pe::PV_OX - 1) / pe::PV_OX) * ((c.ny + pe::PV_OY - 1) / pe::PV_OY);
     const int sps = occupancy_slots(pe::k_stress_pair<4, true>, pe::PS_N, ps);
     const int spv = occupancy_slots(pe::k_velocity_pair<4>, pe::PV_N, pv);
-    S->zc_ps = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tps, sps, 3, 1.15);
-    S->zc_pv = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tpv, spv, 1, 1.3);
+    const int nsm = device_sms();
+    S->zc_ps = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tps, sps, nsm, 0, &pe::STRESS_PAIR_MARCH);
+    S->zc_pv = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tpv, spv, nsm, 0, &pe::VELOCITY_PAIR_MARCH);
     return PE_OK;
 }
 
@@ -552,8 +524,8 @@ int configure_kernels(PeSolver *S)
     if (S->variant == PE_KERNEL_SIMPLE || S->variant == PE_KERNEL_DENSE) {
         const long long tiles = (long long)((c.nx + S->tx - 1) / S->tx) * ((c.ny + S->ty - 1) / S->ty);
         const int slots = occupancy_slots(pe::k_stress<T, 32, 8>, 32 * S->ty, 0);
-        S->zc_s = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tiles, slots, 2);
-        S->zc_v = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tiles, slots, 2);
+        S->zc_s = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tiles, slots, device_sms(), 2, nullptr, 4);
+        S->zc_v = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tiles, slots, device_sms(), 2, nullptr, 4);
         return S->variant == PE_KERNEL_DENSE && std::is_same<T, float>::value ? configure_pair(S, optin) : PE_OK;
     }
     // allow every launch up to the device's opt-in shared memory per block
@@ -578,8 +550,8 @@ int configure_kernels(PeSolver *S)
         ss = occupancy_slots(pe::k_stress_tma<T>, pe::TB_X * pe::TB_Y, tms);
         sv = occupancy_slots(pe::k_velocity_tma<T>, pe::TB_X * pe::TB_Y, tmv);
     }
-    S->zc_s = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, ts, ss, 4);
-    S->zc_v = c.z_chunk > 0 ? c.z_chunk : pick_zchunk(c.nz, tv, sv, 3);
+    S->zc_s = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, ts, ss, device_sms(), 4);
+    S->zc_v = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tv, sv, device_sms(), 3);
     if constexpr (std::is_same<T, float>::value) return configure_pair(S, optin);
     return PE_OK;
 }
