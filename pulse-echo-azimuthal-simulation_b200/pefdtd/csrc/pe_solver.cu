@@ -1452,7 +1452,7 @@ struct PeBatch {
     struct PairWork {
         pe::PairItem *items = nullptr;
         int *off = nullptr;
-        int grid = 0;
+        int grid = 0;   // blocks launched: the shares that are not empty
     } work_s[2], work_v[2];
     bool pad_on = false;            // this run goes through the padded states
     int grid_s = 1, grid_v = 1;
@@ -1525,9 +1525,13 @@ bool batched(const PeBatch *B, const PeSolver *S)
 }
 
 // Cut the marches of one phase (stress or velocity tiles of the solves taken)
-// into `grid` shares of equal load. With a z-chunk asked for (zc_of(S) > 0)
-// columns are cut there and dealt out in order; else they are cut wherever a
-// share is full, at marches of four planes and more. Load in planes of an
+// into at most `grid` shares of equal load. With a z-chunk asked for, by the
+// schedule or one of the solves, columns are cut there (a solve that asks for
+// none at 40 planes) and dealt out in order; else they are cut wherever a
+// share is full, at marches of four planes and more. A launch has a block for
+// each share with marches in it and no more: idle blocks take SM halves, and
+// the busy ones then pair up on the other SMs (two solves of 64x96x96 at
+// 20 planes: 200 steps 20.9 ms with 296 blocks, 18.0 with as many as shares). Load in planes of an
 // interior tile: a guarded tile's plane costs 1.25, a march's start-up 2 planes
 // (stress) or 1 (velocity). Against 40-plane chunks dealt in equal counts, 12
 // solves of 64x96x96 (672 items on 296 blocks: three for some, none for
@@ -1535,6 +1539,7 @@ bool batched(const PeBatch *B, const PeSolver *S)
 struct PairShares {
     std::vector<pe::PairItem> items;
     std::vector<int> off;
+    int used = 0;   // shares with marches in them, the first ones
 };
 PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int grid)
 {
@@ -1552,18 +1557,17 @@ PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int gr
         const int ty = stress ? (c.ny + pe::PS_OY - 1) / pe::PS_OY : (c.ny + pe::PV_OY - 1) / pe::PV_OY;
         const int hx = stress ? pe::pair_last_inside_x(c.nx) : pe::pair_vlast_inside_x(c.nx);
         const int hy = stress ? pe::pair_last_inside_y(c.ny) : pe::pair_vlast_inside_y(c.ny);
-        const int zc = c.z_chunk > 0 || B->z_chunk > 0 ? S->zc_s : 0;
-        chunked = chunked || zc > 0;
+        chunked = chunked || c.z_chunk > 0 || B->z_chunk > 0;
         for (int by = 0; by < ty; ++by)
             for (int bx = 0; bx < tx; ++bx)
-                cols.push_back({s, bx, by, c.nz, zc, bx >= 1 && bx <= hx && by >= 1 && by <= hy ? 1.0 : 1.25});
+                cols.push_back({s, bx, by, c.nz, S->zc_s, bx >= 1 && bx <= hx && by >= 1 && by <= hy ? 1.0 : 1.25});
     }
     PairShares P;
     if (chunked) {   // chunk by chunk within a solve: neighbouring tiles march the same planes together
         for (size_t i = 0; i < cols.size();) {
             size_t j = i;
             while (j < cols.size() && cols[j].solve == cols[i].solve) ++j;
-            const int zc = cols[i].zc > 0 ? cols[i].zc : cols[i].nz;
+            const int zc = cols[i].zc;
             for (int z = 0; z < cols[i].nz; z += zc)
                 for (size_t k = i; k < j; ++k)
                     P.items.push_back({cols[k].solve, cols[k].bx, cols[k].by, z, std::min(cols[k].nz, z + zc)});
@@ -1571,6 +1575,7 @@ PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int gr
         }
         const int n = (int)P.items.size(), per = std::max(1, (n + grid - 1) / grid);
         for (int g = 0; g <= grid; ++g) P.off.push_back(std::min(n, g * per));
+        P.used = (n + per - 1) / per;
         return P;
     }
     const double startup = stress ? 2.0 : 1.0;
@@ -1604,7 +1609,7 @@ PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int gr
         const double mid = 0.5 * (lo + hi);
         (cut(mid, nullptr) <= grid ? hi : lo) = mid;
     }
-    cut(hi, &P);
+    P.used = cut(hi, &P);
     while ((int)P.off.size() <= grid) P.off.push_back((int)P.items.size());
     return P;
 }
@@ -1683,7 +1688,7 @@ int batch_layout_pair(PeBatch *B, int nsm, int optin)
             if ((rc = dev_alloc(&W.off, sizeof(int) * P.off.size()))) return rc;
             if ((rc = batch_copy(B, W.items, P.items.data(), sizeof(pe::PairItem) * P.items.size()))) return rc;
             if ((rc = batch_copy(B, W.off, P.off.data(), sizeof(int) * P.off.size()))) return rc;
-            W.grid = grid;
+            W.grid = P.used;
         }
     return PE_OK;
 }
@@ -1825,7 +1830,7 @@ int launch_pair_persistent(PeBatch *B, int len)
     PE_CUDA(cudaMemsetAsync(B->bar, 0, sizeof(unsigned), B->stream));
     cudaLaunchConfig_t lc = {};
     const PeBatch::PairWork &ws = B->work_s[pad_shared(B)], &wv = B->work_v[pad_shared(B)];
-    lc.gridDim = dim3((unsigned)ws.grid, 1, 1);
+    lc.gridDim = dim3((unsigned)std::max(ws.grid, wv.grid), 1, 1);
     lc.blockDim = dim3(pe::PS_N, 1, 1);
     lc.dynamicSmemBytes = B->smem_p;
     lc.stream = B->stream;
