@@ -588,6 +588,9 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
         const float2 nzv = ld2col(pz, q + 4), nyv = ld2col(py, q + 5), nxv = ld2col(px, q + 5);
         const int z = q - 1;
         const uint32_t lab2 = lab_next;
+        // the whole warp in the couplant (lanes with no cell to update have label
+        // 0); voted on here, ahead of the barrier, where nothing waits for it
+        bool fluid = !CM && A.fluid0 && __all_sync(0xffffffffu, (lab2 & (LAB_MAT | (uint32_t)LAB_MAT << 16)) == 0u);
         lab_next = ldlab(q);
         const bool fast = NC == 4 && TIN && q >= T_H && q <= nz - 1 - T_H;
         if (warp_rows_in) {
@@ -620,11 +623,9 @@ __device__ __forceinline__ void stress_pair_march(const TmapsPairStress &M, cons
             if (q + 1 <= ze) issue_v(q + 1);
             if (q >= zb + 2 && q < ze) issue_s(q);   // plane z + 1, into the slot plane z - 1 used
         }
-        // the whole warp in the couplant (lanes with no cell to update have label
-        // 0) and no large strain so far. The flag is voted on too: a faster warp
+        // ... and no large strain so far. The flag is voted on too: a faster warp
         // may set it while this one reads it, and every lane must take one path
         // (a warp that misses a strain of the next plane has not used it yet).
-        bool fluid = !CM && A.fluid0 && __all_sync(0xffffffffu, (lab2 & (LAB_MAT | (uint32_t)LAB_MAT << 16)) == 0u);
         if (fluid) fluid = __all_sync(0xffffffffu, *bad == 0);
         if (z >= zb && any_out) {
             // strain planes z - 1, z, z + 1 were written at iterations i - 2, i - 1, i
