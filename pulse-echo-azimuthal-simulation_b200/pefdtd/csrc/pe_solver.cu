@@ -481,6 +481,8 @@ int encode_box(CUtensorMap *m, const void *base, CUtensorMapDataType dt, int es,
     return PE_OK;
 }
 
+constexpr long long ORDER2_PAIR_CELLS = 250000;
+
 // Pair kernels for this solve (FP32): in place, on row-padded copies or not at
 // all, and their z-marches.
 int configure_pair(PeSolver *S, int optin)
@@ -489,8 +491,14 @@ int configure_pair(PeSolver *S, int optin)
     const bool dense = S->variant == PE_KERNEL_DENSE;
     const int nm = dense ? 0 : c.n_mat;   // per-cell media: no table in shared memory
     const size_t ps = dense ? pe::PS_SMEM_FIXED : pe::stress_pair_smem(nm), pv = pe::velocity_pair_smem(nm);
-    // per-cell media asked for with an explicit tile run the untiled kernels that have tiles
-    const bool pair_ok = (S->variant == PE_KERNEL_TILED || (dense && c.tile_x <= 0)) && ps <= (size_t)optin &&
+    // Per-cell media asked for with an explicit tile run the untiled kernels that
+    // have tiles, and so do larger grids of order 2: the pair kernels test every
+    // tap below order 8, and with one tap per axis the untiled kernels gain more
+    // (200 steps, ms, pair / untiled: 17x40x40 2.9 / 4.7, 16x24x360 4.4 / 5.1,
+    // 118x56x56 7.1 / 6.0, 64x96x96 10.4 / 8.8, 30x360x60 14.0 / 10.4; at order 4
+    // 118x56x56 7.3 / 7.5, 61x83x117 11.1 / 13.0)
+    const bool untiled = dense && (c.tile_x > 0 || (c.n_coeffs == 1 && S->ncell > ORDER2_PAIR_CELLS));
+    const bool pair_ok = (S->variant == PE_KERNEL_TILED || dense) && !untiled && ps <= (size_t)optin &&
                          pv <= (size_t)optin && encode_fn() != nullptr;
     S->pair_capable = pair_ok && c.nx % 4 == 0;
     S->padded = pair_ok && c.nx % 4 != 0;
