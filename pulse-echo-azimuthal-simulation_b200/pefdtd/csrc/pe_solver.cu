@@ -1458,8 +1458,8 @@ struct PeBatch {
     // the solves stepped in place, and with the padded solves too, which share
     // the persistent launches (pad_shared())
     struct PairWork {
-        pe::PairItem *items = nullptr;
-        int *off = nullptr;
+        pe::PairItem *items = nullptr;   // grid shares of `per` items
+        int per = 0;
         int grid = 0;   // blocks launched: the shares that are not empty
     } work_s[2], work_v[2];
     bool pad_on = false;            // this run goes through the padded states
@@ -1513,7 +1513,6 @@ struct PeBatch {
     {
         for (PairWork *w : {&work_s[0], &work_s[1], &work_v[0], &work_v[1]}) {
             dev_free(w->items);
-            dev_free(w->off);
             *w = PairWork();
         }
     }
@@ -1545,9 +1544,8 @@ bool batched(const PeBatch *B, const PeSolver *S)
 // solves of 64x96x96 (672 items on 296 blocks: three for some, none for
 // others): 200 steps 106 -> 89 ms.
 struct PairShares {
-    std::vector<pe::PairItem> items;
-    std::vector<int> off;
-    int used = 0;   // shares with marches in them, the first ones
+    std::vector<pe::PairItem> items;   // `used` shares of `per` items, padded with empty ones
+    int per = 0, used = 0;
 };
 PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int grid)
 {
@@ -1581,16 +1579,17 @@ PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int gr
                     P.items.push_back({cols[k].solve, cols[k].bx, cols[k].by, z, std::min(cols[k].nz, z + zc)});
             i = j;
         }
-        const int n = (int)P.items.size(), per = std::max(1, (n + grid - 1) / grid);
-        for (int g = 0; g <= grid; ++g) P.off.push_back(std::min(n, g * per));
-        P.used = (n + per - 1) / per;
+        const int n = (int)P.items.size();
+        P.per = std::max(1, (n + grid - 1) / grid);
+        P.used = (n + P.per - 1) / P.per;
+        P.items.resize((size_t)P.used * P.per, pe::PairItem{0, 0, 0, 0, 0});
         return P;
     }
     const double startup = stress ? 2.0 : 1.0;
-    auto cut = [&](double T, PairShares *out) {   // shares used at load T each
+    std::vector<std::vector<pe::PairItem>> shares(1);
+    auto cut = [&](double T, bool keep) {   // shares used at load T each
         int used = 1;
         double load = 0.0;
-        if (out) out->off.push_back(0);
         for (const Col &c : cols)
             for (int z = 0; z < c.nz;) {
                 int n = (int)((T - load) / c.w - startup);
@@ -1598,14 +1597,14 @@ PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int gr
                     if (load > 0.0) {   // this share is full
                         ++used;
                         load = 0.0;
-                        if (out) out->off.push_back((int)out->items.size());
+                        if (keep) shares.emplace_back();
                         continue;
                     }
                     n = std::min(4, c.nz - z);
                 }
                 n = std::min(n, c.nz - z);
                 if (c.nz - z - n < 4 && c.nz - z - n > 0) n = std::max(std::min(4, c.nz - z), c.nz - z - 4);
-                if (out) out->items.push_back({c.solve, c.bx, c.by, z, z + n});
+                if (keep) shares.back().push_back({c.solve, c.bx, c.by, z, z + n});
                 load += c.w * (n + startup);
                 z += n;
             }
@@ -1615,10 +1614,14 @@ PairShares cut_pair_work(const PeBatch *B, bool stress, bool with_padded, int gr
     for (const Col &c : cols) hi += c.w * (c.nz + startup);
     for (int it = 0; it < 50; ++it) {
         const double mid = 0.5 * (lo + hi);
-        (cut(mid, nullptr) <= grid ? hi : lo) = mid;
+        (cut(mid, false) <= grid ? hi : lo) = mid;
     }
-    P.used = cut(hi, &P);
-    while ((int)P.off.size() <= grid) P.off.push_back((int)P.items.size());
+    if (!cols.empty()) P.used = cut(hi, true);
+    for (const auto &q : shares) P.per = std::max(P.per, (int)q.size());
+    for (int g = 0; g < P.used; ++g) {
+        P.items.insert(P.items.end(), shares[g].begin(), shares[g].end());
+        P.items.resize((size_t)(g + 1) * P.per, pe::PairItem{0, 0, 0, 0, 0});
+    }
     return P;
 }
 
@@ -1693,9 +1696,8 @@ int batch_layout_pair(PeBatch *B, int nsm, int optin)
             if (P.items.empty()) continue;
             int rc;
             if ((rc = dev_alloc(&W.items, sizeof(pe::PairItem) * P.items.size()))) return rc;
-            if ((rc = dev_alloc(&W.off, sizeof(int) * P.off.size()))) return rc;
             if ((rc = batch_copy(B, W.items, P.items.data(), sizeof(pe::PairItem) * P.items.size()))) return rc;
-            if ((rc = batch_copy(B, W.off, P.off.data(), sizeof(int) * P.off.size()))) return rc;
+            W.per = P.per;
             W.grid = P.used;
         }
     return PE_OK;
@@ -1851,17 +1853,18 @@ int launch_pair_persistent(PeBatch *B, int len)
     const float *const *tabs = B->tabs;
     const pe::TmapsPairStress *ms = B->set().pmaps_s;
     const pe::TmapsPairVelocity *mv = B->set().pmaps_v;
-    const int *nm = B->nmats, *os = ws.off, *ov = wv.off;
+    const int *nm = B->nmats;
+    const int ps = ws.per, pv = wv.per, ns = ws.grid * ps, nv = wv.grid * pv;
     const pe::PairItem *is = ws.items, *iv = wv.items;
     cudaError_t e;
     if (B->pair_nc4 && B->pair_ts)
-        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, true>, d, ms, mv, tabs, nm, is, os, iv, ov, len, B->bar, B->status);
+        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, true>, d, ms, mv, tabs, nm, is, ns, ps, iv, nv, pv, len, B->bar, B->status);
     else if (B->pair_nc4)
-        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, false>, d, ms, mv, tabs, nm, is, os, iv, ov, len, B->bar, B->status);
+        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<4, false>, d, ms, mv, tabs, nm, is, ns, ps, iv, nv, pv, len, B->bar, B->status);
     else if (B->pair_ts)
-        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<0, true>, d, ms, mv, tabs, nm, is, os, iv, ov, len, B->bar, B->status);
+        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<0, true>, d, ms, mv, tabs, nm, is, ns, ps, iv, nv, pv, len, B->bar, B->status);
     else
-        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<0, false>, d, ms, mv, tabs, nm, is, os, iv, ov, len, B->bar, B->status);
+        e = cudaLaunchKernelEx(&lc, pe::k_pair_batch_persistent<0, false>, d, ms, mv, tabs, nm, is, ns, ps, iv, nv, pv, len, B->bar, B->status);
     if (e != cudaSuccess) return fail(PE_ERR_CUDA, std::string("persistent batch launch: ") + cudaGetErrorString(e));
     B->launches += 1;
     return PE_OK;
@@ -1884,17 +1887,17 @@ int batch_chunk(PeBatch *B, int len)
             if (B->pair_batch && !B->persistent && ws.grid > 0) {
                 const pe::StepArgs<float> *d = (const pe::StepArgs<float> *)L.descs;
                 if (B->pair_nc4 && B->pair_ts)
-                    pe::k_stress_pair_batch<4, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
+                    pe::k_stress_pair_batch<4, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.per, k);
                 else if (B->pair_nc4)
-                    pe::k_stress_pair_batch<4, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
+                    pe::k_stress_pair_batch<4, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.per, k);
                 else if (B->pair_ts)
-                    pe::k_stress_pair_batch<0, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
+                    pe::k_stress_pair_batch<0, true><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.per, k);
                 else
-                    pe::k_stress_pair_batch<0, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.off, k);
+                    pe::k_stress_pair_batch<0, false><<<ws.grid, pe::PS_N, B->smem_s, B->stream>>>(d, L.pmaps_s, B->tabs, B->nmats, ws.items, ws.per, k);
                 if (B->pair_nc4)
-                    pe::k_velocity_pair_batch<4><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, L.pmaps_v, B->nmats, wv.items, wv.off, k);
+                    pe::k_velocity_pair_batch<4><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, L.pmaps_v, B->nmats, wv.items, wv.per, k);
                 else
-                    pe::k_velocity_pair_batch<0><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, L.pmaps_v, B->nmats, wv.items, wv.off, k);
+                    pe::k_velocity_pair_batch<0><<<wv.grid, pe::PV_N, B->smem_v, B->stream>>>(d, L.pmaps_v, B->nmats, wv.items, wv.per, k);
                 B->launches += 2;
             }
         }
