@@ -367,20 +367,32 @@ __global__ void __launch_bounds__(RED_T) k_analyse(const T *__restrict__ x, cons
 }
 
 // Device copies of a call's small host arrays (offsets, windows, time
-// steps) go to one grow-only buffer per device, held (mutex) for the whole
-// call: every entry point synchronises its stream before returning, so the
-// next call may reuse the buffer, and after the first calls on a device no
-// call allocates or frees device memory (cudaFree would also synchronise
-// the device).
+// steps) and the envelope's tap tables go to one buffer per device, held
+// (mutex) for the whole call: every entry point synchronises its stream before
+// returning, so the next call may reuse the buffer, and after the first calls
+// on a device no call of ordinary size allocates or frees device memory
+// (cudaFree would also synchronise the device). A buffer above STAGE_KEEP
+// (tables of many or very long lengths) goes back to the driver with the call.
 struct StageArea {
     std::mutex mu;
     char *p = nullptr;
     size_t cap = 0;
 };
 constexpr int STAGE_DEVICES = 64;
+constexpr size_t STAGE_KEEP = (size_t)16 << 20;
 
+// One call's hold on its device's area; declared before the call's work, and
+// so released after finish() has synchronised the stream.
 struct Staged {
+    StageArea *area = nullptr;
     std::unique_lock<std::mutex> lock;
+    ~Staged()
+    {
+        if (!area || area->cap <= STAGE_KEEP) return;
+        cudaFree(area->p);
+        area->p = nullptr;
+        area->cap = 0;
+    }
 };
 
 cudaError_t stage(Staged &s, cudaStream_t st, std::initializer_list<std::pair<const void *, size_t>> parts,
@@ -393,12 +405,13 @@ cudaError_t stage(Staged &s, cudaStream_t st, std::initializer_list<std::pair<co
     if (dev < 0 || dev >= STAGE_DEVICES) return cudaErrorInvalidDevice;
     StageArea &a = areas[dev];
     s.lock = std::unique_lock<std::mutex>(a.mu);
+    s.area = &a;
     size_t total = 0;
     for (auto &q : parts) total += (q.second + 255) & ~size_t(255);
     if (total > a.cap) {
         // grow geometrically, so that a run of ever larger calls reallocates
         // (and synchronises the device in cudaFree) only O(log) times
-        const size_t want = std::max(total, std::max(a.cap * 2, (size_t)1 << 16));
+        const size_t want = std::max(total, std::min(STAGE_KEEP, std::max(a.cap * 2, (size_t)1 << 16)));
         if (a.p) cudaFree(a.p);
         a.p = nullptr;
         a.cap = 0;
