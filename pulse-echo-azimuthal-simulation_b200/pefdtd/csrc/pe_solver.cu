@@ -163,7 +163,8 @@ struct PeSolver {
     long long *grp_off = nullptr;
     int *ent_group = nullptr;   // group of each receiver entry (caller order)
     int n_rec = 0, n_groups = 0;
-    void *rec_val = nullptr;
+    void *rec_val = nullptr;    // (rec_rows, n_rec) samples of a chunk
+    int rec_rows = 0;
     void *wavelet = nullptr;
     long long nt_wav = 0;
     long long *step = nullptr;
@@ -658,6 +659,24 @@ int repitch(const PeSolver *S, const PeState *from, int spitch, const PeState *t
 int pad_in(const PeSolver *S, const PeState *state, cudaStream_t st) { return repitch(S, state, 0, &S->pst, S->px, 9, st); }
 int pad_out(const PeSolver *S, const PeState *state, cudaStream_t st) { return repitch(S, &S->pst, S->px, state, 0, 9, st); }
 
+// Room for the receivers' samples of `rows` steps. The caller has finished the
+// work that uses the buffer there is.
+int reserve_records(PeSolver *S, int rows, cudaStream_t st)
+{
+    if (rows <= S->rec_rows) return PE_OK;
+    const size_t bytes = (size_t)S->esize * std::max(1, S->n_rec) * rows;
+    void *p = nullptr;
+    const int rc = dev_alloc(&p, bytes);
+    if (rc) return rc;
+    PE_CUDA(cudaMemsetAsync(p, 0, bytes, st));
+    if (S->rec_val) dev_free(S->rec_val);
+    S->rec_val = p;
+    S->rec_rows = rows;
+    if (S->gexec) cudaGraphExecDestroy(S->gexec);   // it writes to the old buffer
+    S->gexec = nullptr;
+    return PE_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -925,8 +944,7 @@ int pe_solver_create(const PeConfig *cfg, const PeMedium *md, const PeProbe *pr,
     if ((rc = dev_alloc(&S->rec_pos, sizeof(int) * nr))) return rc;
     if ((rc = dev_alloc(&S->rec_w, (size_t)es * nr))) return rc;
     if ((rc = dev_alloc(&S->grp_off, sizeof(long long) * (S->n_groups + 1)))) return rc;
-    if ((rc = dev_alloc(&S->rec_val, (size_t)es * nr * S->chunk))) return rc;
-    PE_CUDA(cudaMemsetAsync(S->rec_val, 0, (size_t)es * nr * S->chunk, st));
+    if ((rc = reserve_records(S.get(), S->chunk, st))) return rc;
     if (n_rec > 0) {
         PE_CUDA(cudaMemcpyAsync(S->rec_cell, rcell_sorted.data(), sizeof(long long) * n_rec, cudaMemcpyHostToDevice, st));
         PE_CUDA(cudaMemcpyAsync(S->rec_pos, rpos_sorted.data(), sizeof(int) * n_rec, cudaMemcpyHostToDevice, st));
@@ -2025,6 +2043,8 @@ int pe_batch_create(int n, const PeConfig *cfgs, const PeMedium *media, const Pe
     PE_CUDA(cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking));
     PE_CUDA(cudaEventCreateWithFlags(&B->ev_in, cudaEventDisableTiming));
     PE_CUDA(cudaEventCreateWithFlags(&B->ev_out, cudaEventDisableTiming));
+    for (PeSolver *S : B->solves)
+        if ((rc = reserve_records(S, B->chunk, B->stream))) return rc;
     std::vector<int> nm;
     std::vector<const float *> tabs;
     for (const PeSolver *S : B->solves) {
@@ -2044,10 +2064,14 @@ int pe_batch_schedule(PeBatch *B, int z_chunk, int chunk_steps)
 {
     if (!B || z_chunk < 0 || chunk_steps < 0) return fail(PE_ERR_INVALID, "bad schedule");
     PE_CUDA(cudaStreamSynchronize(B->stream));   // queued runs read the work lists that go
+    for (PeBatch::Set &L : B->sets) L.uploaded = false;
+    for (PeSolver *S : B->solves) {
+        const int rc = reserve_records(S, chunk_steps, B->stream);
+        if (rc) return rc;
+    }
     B->z_chunk = z_chunk;
     if (chunk_steps > 0) B->chunk = chunk_steps;
     for (PeSolver *S : B->solves) S->cfg.z_chunk = 0;
-    for (PeBatch::Set &L : B->sets) L.uploaded = false;
     return B->dtype == PE_F64 ? batch_layout<double>(B) : batch_layout<float>(B);
 }
 
