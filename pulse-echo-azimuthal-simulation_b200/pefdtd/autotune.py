@@ -2,7 +2,8 @@
 
 Picks, by timing the batch itself on its own device, the planes per z-march
 (the work-item size: shorter marches give more items and better balance
-across the 148 SMs, longer ones spend less on each march's start-up planes),
+across the 148 SMs, longer ones spend less on each march's start-up planes;
+or equal shares cut wherever a block is full, the layout of an untuned batch),
 the number of steps per captured CUDA graph, and the launch mode: one
 stress and one velocity launch per step, or one persistent launch per graph
 chunk (pefdtd.batch.BatchSolver.set_persistent). The tile shapes are not a
@@ -17,7 +18,7 @@ from __future__ import annotations
 import json
 import os
 
-Z_CANDIDATES = (16, 24, 32, 40, 56, 80, 120, 160)
+Z_CANDIDATES = (0, 16, 24, 32, 40, 56, 80, 120, 160)   # 0: equal shares per block
 CHUNK_CANDIDATES = (50, 100, 200, 400)
 
 
@@ -73,7 +74,8 @@ def tune_batch(batch, steps=None, use_cache=True):
     """Choose and apply (z_chunk, chunk_steps); returns them with timings."""
     key = batch_key(batch)
     db = _load() if use_cache else {}
-    if use_cache and key in db and "persistent" in db[key]:
+    # (an entry from before the launch mode or the equal shares were choices is tuned again)
+    if use_cache and key in db and "persistent" in db[key] and "0" in db[key].get("ms_per_step_by_z", {}):
         z, c = db[key]["z_chunk"], db[key]["chunk_steps"]
         batch.schedule(z, c)
         batch.set_persistent(db[key]["persistent"])
