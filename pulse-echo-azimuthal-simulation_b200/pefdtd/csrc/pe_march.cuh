@@ -14,8 +14,7 @@ struct MarchModel {
 // 20 march lengths each. The stress kernel's blocks drift apart (interior tiles
 // are faster), so its last wave costs its fraction and half a wave; the
 // velocity kernel's waves run nearly in step. On those grids no choice is more
-// than 0.4 % slower than that of whole waves with at least four planes (the
-// rule of the one-block kernels), and the means over the grids are 2.4 %
+// than 0.4 % slower than that of whole waves with at least four planes, and the means over the grids are 2.4 %
 // (stress) and 2.0 % (velocity) above the best length's time, against 8.0 and
 // 8.8 % with whole waves. In us: velocity 96x160x160 53.2 -> 47.5 (20 -> 9
 // planes), 20x24x28 14.7 -> 10.3 (4 -> 1); stress 30x200x200 54.2 -> 48.4
@@ -25,17 +24,15 @@ constexpr MarchModel VELOCITY_PAIR_MARCH{0.5, 0.9, 1.1, 1.0, 0.1};
 
 // The split of nz into chunks that minimises the modelled time of a launch of
 // `tiles` columns. Without a model (kernels that run their waves in step, one
-// block per slot) a wave counts whole and the least cost wins; with one a
+// block per slot, and the untiled ones, which on 15 grids come within 3 % of
+// their best length so) a wave counts whole and the least cost wins; with one a
 // shorter march must be worth 2 %, since longer ones re-read less of the halo.
-// min_zc: the shortest march considered.
-inline int pick_zchunk(int nz, long long tiles, int slots, int nsm, double startup, const MarchModel *m = nullptr,
-                       int min_zc = 1)
+inline int pick_zchunk(int nz, long long tiles, int slots, int nsm, double startup, const MarchModel *m = nullptr)
 {
     int best_zc = nz;
     double best = 1e300;
     for (int nch = 1; nch <= nz; ++nch) {
         const int zc = (nz + nch - 1) / nch;
-        if (zc < min_zc && nch > 1) break;
         const long long blocks = tiles * ((nz + zc - 1) / zc);
         const double whole = (double)((blocks + slots - 1) / slots);
         double waves = whole;

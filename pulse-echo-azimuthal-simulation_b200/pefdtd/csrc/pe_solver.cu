@@ -533,8 +533,8 @@ int configure_kernels(PeSolver *S)
     if (S->variant == PE_KERNEL_SIMPLE || S->variant == PE_KERNEL_DENSE) {
         const long long tiles = (long long)((c.nx + S->tx - 1) / S->tx) * ((c.ny + S->ty - 1) / S->ty);
         const int slots = occupancy_slots(pe::k_stress<T, 32, 8>, 32 * S->ty, 0);
-        S->zc_s = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tiles, slots, device_sms(), 2, nullptr, 4);
-        S->zc_v = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tiles, slots, device_sms(), 2, nullptr, 4);
+        S->zc_s = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tiles, slots, device_sms(), 2);
+        S->zc_v = c.z_chunk > 0 ? c.z_chunk : pe::pick_zchunk(c.nz, tiles, slots, device_sms(), 2);
         return S->variant == PE_KERNEL_DENSE && std::is_same<T, float>::value ? configure_pair(S, optin) : PE_OK;
     }
     // allow every launch up to the device's opt-in shared memory per block

@@ -17,12 +17,12 @@ PROGRAM = r"""
 #include "pe_march.cuh"
 int main()
 {
-    int nz, slots, model, min_zc;
+    int nz, slots, model;
     long long tiles;
     double startup;
     const pe::MarchModel *m[] = {nullptr, &pe::STRESS_PAIR_MARCH, &pe::VELOCITY_PAIR_MARCH};
-    while (scanf("%d %lld %d %lf %d %d", &nz, &tiles, &slots, &startup, &model, &min_zc) == 6)
-        printf("%d\n", pe::pick_zchunk(nz, tiles, slots, 148, startup, m[model], min_zc));
+    while (scanf("%d %lld %d %lf %d", &nz, &tiles, &slots, &startup, &model) == 5)
+        printf("%d\n", pe::pick_zchunk(nz, tiles, slots, 148, startup, m[model]));
     return 0;
 }
 """
@@ -52,17 +52,22 @@ def pick(tmp_path_factory):
 
 
 def test_whole_waves_take_the_least_planes(pick):
-    rows = [(nz, t, 148, s, 0, 1) for nz in (1, 7, 20, 61, 84, 136, 170) for t in (1, 9, 72, 78, 150, 400) for s in (3, 4)]
-    for (nz, t, slots, s, _, _), zc in zip(rows, pick(rows)):
+    rows = [(nz, t, 148, s, 0) for nz in (1, 7, 20, 61, 84, 136, 170) for t in (1, 9, 72, 78, 150, 400) for s in (3, 4)]
+    for (nz, t, slots, s, _), zc in zip(rows, pick(rows)):
         cost = {z: -(-t * -(-nz // z) // slots) * (z + s) for z in range(1, nz + 1)}
         assert cost[zc] == min(cost.values()), (nz, t, zc)
+
+
+def whole_waves(nz, tiles, slots, startup, least):
+    """The march of at least `least` planes that takes the least whole waves x planes (the longest such)."""
+    lengths = [z for z in sorted({-(-nz // n) for n in range(1, nz + 1)}, reverse=True) if z >= least] or [nz]
+    return min(lengths, key=lambda z: -(-tiles * -(-nz // z) // slots) * (z + startup))
 
 
 def test_pair_choices_lose_nothing_against_whole_waves(pick):
     rows = []
     for (nz, ny, nx), model, _ in MEASURED:
         tiles = ((nx + 30) // 30) * ((ny + 13) // 14) if model == 1 else ((nx + 31) // 32) * ((ny + 15) // 16)
-        rows += [(nz, tiles, 296, 0, model, 1), (nz, tiles, 296, 4 - model, 0, 4)]   # the rule, whole waves
-    zc = pick(rows)
-    for k, (grid, model, us) in enumerate(MEASURED):
-        assert us[zc[2 * k]] <= 1.004 * us[zc[2 * k + 1]], (grid, model, zc[2 * k:2 * k + 2])
+        rows.append((nz, tiles, 296, 0, model))
+    for (nz, tiles, slots, _, model), (grid, _, us), zc in zip(rows, MEASURED, pick(rows)):
+        assert us[zc] <= 1.004 * us[whole_waves(nz, tiles, slots, 4 - model, 4)], (grid, model, zc)
