@@ -148,7 +148,8 @@ int pe_solver_set_wavelet(PeSolver *s, const void *wavelet, int64_t nt);
  * (cudaStream_t, NULL = legacy default stream) and write trace rows
  * traces_dev[n * n_groups + g] for those steps (traces_dev: device, dtype,
  * at least step_end * n_groups elements). Asynchronous with respect to the
- * host. Full chunks run as one captured CUDA graph each. */
+ * host. Full chunks run as one captured CUDA graph each, from the second on
+ * the same state and trace buffers; the first goes out as plain launches. */
 int pe_solver_run(PeSolver *s, const PeState *state, void *traces_dev, int64_t step_begin,
                   int64_t step_end, void *stream);
 
@@ -246,7 +247,9 @@ typedef struct PeBatch PeBatch;
 int pe_batch_create(int n, const PeConfig *cfgs, const PeMedium *media, const PeProbe *probes,
                     PeBatch **out);
 /* Work layout: planes per z-march (0 = FP32 pair batches cut into equal
- * shares per block, others 40 planes) and steps per captured graph (0 = keep). Chosen by pefdtd.autotune. */
+ * shares per block, others 40 planes) and steps per captured graph (0 = keep).
+ * Chosen by pefdtd.autotune. Waits for the batch's queued runs, and so does
+ * pe_batch_set_wavelet. */
 int pe_batch_schedule(PeBatch *b, int z_chunk, int chunk_steps);
 /* Persistent batch mode (on = 1): one cooperative launch per graph chunk
  * advances every batched solve by the chunk's steps, its blocks alternating

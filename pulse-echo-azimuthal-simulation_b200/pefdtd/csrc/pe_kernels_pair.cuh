@@ -879,8 +879,8 @@ __device__ __forceinline__ float div_face_rcp(float a, float b, bool own, float 
 // by TMA boxes or 64-bit pairs; a run of several steps therefore copies it
 // once into solver-owned fields whose rows are padded to four cells, steps
 // those with the pair kernels, and copies it back. Each copy moves 72 B per
-// cell, about one step's traffic. 100 steps of 136x338x338: 120.8 ms with the
-// cp.async kernels, 73.8 ms padded, both copies included.
+// cell, about one step's traffic. 100 steps of 136x338x338: 121 ms with the
+// cp.async kernels, 67 ms padded, both copies included.
 struct FieldSet {
     float *f[9];
 };

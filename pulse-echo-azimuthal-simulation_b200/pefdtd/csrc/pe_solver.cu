@@ -1556,7 +1556,7 @@ bool batched(const PeBatch *B, const PeSolver *S)
 // share is full, at marches of four planes and more. A launch has a block for
 // each share with marches in it and no more: idle blocks take SM halves, and
 // the busy ones then pair up on the other SMs (two solves of 64x96x96 at
-// 20 planes: 200 steps 20.9 ms with 296 blocks, 18.0 with as many as shares). Load in planes of an
+// 20 planes: 200 steps 20.9 ms with 296 blocks, 18.5 with as many as shares). Load in planes of an
 // interior tile: a guarded tile's plane costs 1.25, a march's start-up 2 planes
 // (stress) or 1 (velocity). Against 40-plane chunks dealt in equal counts, 12
 // solves of 64x96x96 (672 items on 296 blocks: three for some, none for
