@@ -10,17 +10,17 @@ namespace pe {
 struct MarchModel {
     double startup, lone, one, whole, tail;
 };
-// Fitted to the profiled times of 42 grids from 20x24x28 to 160x256x256 at 6 to
+// Fitted to the profiled times of 62 grids from 20x24x28 to 160x256x256 at 6 to
 // 20 march lengths each. The stress kernel's blocks drift apart (interior tiles
-// are faster), so its last wave costs its fraction and half a wave; the
-// velocity kernel's waves run nearly in step. On those grids no choice is more
-// than 0.4 % slower than that of whole waves with at least four planes, and the means over the grids are 2.4 %
-// (stress) and 2.0 % (velocity) above the best length's time, against 8.0 and
-// 8.8 % with whole waves. In us: velocity 96x160x160 53.2 -> 47.5 (20 -> 9
-// planes), 20x24x28 14.7 -> 10.3 (4 -> 1); stress 30x200x200 54.2 -> 48.4
-// (15 -> 6), 87x223x223 134 -> 127 (44 -> 11).
-constexpr MarchModel STRESS_PAIR_MARCH{2.0, 0.95, 1.2, 0.0, 0.5};
-constexpr MarchModel VELOCITY_PAIR_MARCH{0.5, 0.9, 1.1, 1.0, 0.1};
+// are faster), so much of its last wave counts by its fraction; the velocity
+// kernel's waves run nearly in step. Against whole waves with at least four
+// planes no choice on those grids is slower by more than 1.3 % (stress) and 0.4
+// % (velocity), and the means over the grids are 2.2 and 1.9 % above the best
+// length's time, where whole waves are 7.1 and 7.8 % above it. In us: velocity
+// 96x160x160 53.2 -> 47.5 (20 -> 9 planes), 20x24x28 14.7 -> 10.3 (4 -> 1);
+// stress 30x200x200 54.2 -> 48.4 (15 -> 6), 87x223x223 134 -> 129 (44 -> 22).
+constexpr MarchModel STRESS_PAIR_MARCH{2.0, 0.85, 1.2, 0.25, 0.4};
+constexpr MarchModel VELOCITY_PAIR_MARCH{1.0, 0.9, 1.1, 0.75, 0.05};
 
 // The split of nz into chunks that minimises the modelled time of a launch of
 // `tiles` columns. Without a model (kernels that run their waves in step, one
